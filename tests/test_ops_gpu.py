@@ -251,6 +251,68 @@ def test_qk_norm_rope_attention(do_norm):
         _close(wk.grad, wkr.grad, 5e-2, 0.05 * wkr.grad.abs().max().item(), "dwk")
 
 
+def _attention_float64(qkv, wq, wk, cos, sin, lens, Hq, Hkv, D, eps, causal):
+    """The block in float64 without any rounding inside."""
+    T = qkv.shape[0]
+    q, k, v = (t.reshape(T, -1, D) for t in qkv.split([Hq * D, Hkv * D, Hkv * D], dim=-1))
+    norm = lambda t, w: t if w is None else t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + eps) * w
+
+    def rope(t):
+        a, b, c, s = t[..., :D // 2], t[..., D // 2:], cos.double()[:, None], sin.double()[:, None]
+        return torch.cat([a * c - b * s, b * c + a * s], -1)
+
+    q, k = rope(norm(q, wq)), rope(norm(k, wk))
+    out, s = [], 0
+    for n in lens:
+        qb, kb, vb = (t[s:s + n].transpose(0, 1) for t in (q, k, v))
+        kb, vb = kb.repeat_interleave(Hq // Hkv, 0), vb.repeat_interleave(Hq // Hkv, 0)
+        sc = qb @ kb.transpose(1, 2) / math.sqrt(D)
+        if causal:
+            sc = sc.masked_fill(~torch.ones(n, n, dtype=torch.bool, device=sc.device).tril(), float("-inf"))
+        out.append((sc.softmax(-1) @ vb).transpose(0, 1).reshape(n, Hq * D))
+        s += n
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,causal,do_norm", [
+    ([1], 2, 1, True, True), ([63, 1, 65], 4, 4, True, False), ([128, 64, 129], 8, 2, False, False),
+    ([257, 700, 3], 16, 4, True, True), ([511], 6, 2, False, True)])
+def test_hd64_attention_loses_no_precision(lens, Hq, Hkv, causal, do_norm):
+    """64-wide heads: the kernels against float64, next to the reference path with its fp32
+    probabilities.  Without norm and rotation only the rounding of outputs and gradients to bf16 is left,
+    1.6e-3 of the norm; bf16 probabilities would add as much again (1.4x), the split ones add 1e-5."""
+    from xorl_b200.ops import attention as A
+    torch.manual_seed(0)
+    D, T, eps = 64, sum(lens), 1e-6
+    cu = _make_cu(lens)
+    base = torch.randn(T, (Hq + 2 * Hkv) * D, device=DEV, dtype=torch.bfloat16)
+    ws = [(1 + 0.1 * torch.randn(D, device=DEV)).bfloat16() if do_norm else None for _ in range(2)]
+    pos = torch.cat([torch.arange(l, device=DEV) for l in lens]).float()
+    ang = pos[:, None] / (1e4 ** (torch.arange(0, D, 2, device=DEV).float() / D))[None] * float(do_norm)
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    go = torch.randn(T, Hq * D, device=DEV, dtype=torch.bfloat16)
+
+    def grads(fn, dtype=None):
+        ins = [t if t is None else t.detach().to(dtype or t.dtype).requires_grad_() for t in (base, *ws)]
+        y = fn(*ins)
+        y.backward(go.to(y.dtype))
+        return [y.detach()] + [t.grad for t in ins if t is not None]
+
+    before = A.launch_count()
+    got = grads(lambda x, a, b: A.qk_norm_rope_attention(x, a, b, cos, sin, cu, Hq, Hkv, D, eps, causal))
+    assert A.launch_count() > before
+    ref = grads(lambda x, a, b: A.qk_norm_rope_attention_reference(x, a, b, cos, sin, cu, Hq, Hkv, D, eps, causal,
+                                                                  D ** -0.5))
+    exact = grads(lambda x, a, b: _attention_float64(x, a, b, cos, sin, lens, Hq, Hkv, D, eps, causal), torch.float64)
+    for name, g, r, e in zip(("out", "dqkv", "dwq", "dwk"), got, ref, exact):
+        # a gradient that cancels to zero (a document of one token) does so to the rounding of the fp32 sums
+        # dP and delta over 64 products: 64 * 2^-24 = 4e-6 of their terms
+        base_norm = max(e.norm().item(), 1e-4 * go.double().norm().item())
+        eg, er = ((t.double() - e).norm().item() / base_norm for t in (g, r))
+        # weight gradients: 64 values rounded once each to bf16, up to half an ulp (2^-9) off
+        assert eg <= 1.02 * er + (2 ** -9 if name in ("dwq", "dwk") else 2e-5), (name, eg, er)
+
+
 def test_status_words_clean():
     from xorl_b200.ops import _lib
     assert _lib.read_status()[0] == 0

@@ -430,6 +430,20 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo,
   if (lane == 0) delta[(size_t)h * T + t] = s;
 }
 
+// as above from the unrounded output, head dim 64 (out: [T, Hq, 64] fp32)
+__global__ void __launch_bounds__(256)
+attn_delta_hd64_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ dout, long long lddo,
+                       float* __restrict__ delta, int T, int Hq) {
+  const long long wid = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (wid >= (long long)T * Hq) return;
+  const int t = (int)(wid / Hq), h = (int)(wid % Hq);
+  const int lane = threadIdx.x & 31;
+  const float2 a = reinterpret_cast<const float2*>(o + (size_t)wid * 64)[lane];
+  const float2 b = unpack_bf16x2(reinterpret_cast<const uint32_t*>(dout + (size_t)t * lddo + (size_t)h * 64)[lane]);
+  const float s = warp_sum(a.x * b.x + a.y * b.y);
+  if (lane == 0) delta[(size_t)h * T + t] = s;
+}
+
 static int g_split = 1;
 
 }  // namespace xb_attn_bwd_ns
@@ -446,13 +460,13 @@ XB_API int xb_attn_bwd_set_split(int split) {
 XB_API int xb_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dout, const float* lse,
                           const float* delta, float* dq, const int* cu_seqlens, const int* k_starts,
                           long long ldq, long long ldk, long long ldv, long long lddo, int num_seqs, int T,
-                          int Tk, int Hq, int Hkv, int causal, float scale, int accumulate, int max_q_tiles,
-                          void* stream);
+                          int Tk, int Hq, int Hkv, int D, int causal, float scale, int accumulate,
+                          int max_q_tiles, void* stream);
 XB_API int xb_attn_bwd_dkv(const void* q, const void* k, const void* v, const void* dout, const float* lse,
                            const float* delta, float* dk, void* dv, const int* cu_seqlens, const int* k_starts,
                            long long ldq, long long ldk, long long ldv, long long lddo, long long lddv,
-                           int num_seqs, int T, int Tk, int Hq, int Hkv, int causal, float scale, int max_tiles,
-                           void* stream);
+                           int num_seqs, int T, int Tk, int Hq, int Hkv, int D, int causal, float scale,
+                           int max_tiles, void* stream);
 
 // Inputs as in xb_attn_fwd plus out / dout [T, Hq, 128] and lse [Hq, T].
 // Scratch: delta fp32 [Hq * T]; dq_accum fp32 [T * Hq * 128] (this call zeroes it).
@@ -514,11 +528,11 @@ XB_API int xb_attn_bwd_ex(const void* q, const void* k, const void* v, const voi
     // dq_accum is written with plain stores (added to when flags bit 0 is set); rows outside every
     // sequence keep the zeros of the memset above
     int rc = xb_attn_bwd_dkv(q, k, v, dout, lse, delta, dk, dv, cu_seqlens, k_starts, ldq, ldk, ldv, lddo, lddv,
-                             num_seqs, T, Tk, Hq, Hkv, causal, scale, max_tiles, stream);
+                             num_seqs, T, Tk, Hq, Hkv, D, causal, scale, max_tiles, stream);
     if (rc) return rc;
     const int q_tiles = max_tiles > 0 ? (max_tiles + 1) / 2 + num_seqs : 0;
     return xb_attn_bwd_dq(q, k, v, dout, lse, delta, dq_accum, cu_seqlens, k_starts, ldq, ldk, ldv, lddo,
-                          num_seqs, T, Tk, Hq, Hkv, causal, scale, (flags & 1) ? 1 : 0, q_tiles, stream);
+                          num_seqs, T, Tk, Hq, Hkv, D, causal, scale, (flags & 1) ? 1 : 0, q_tiles, stream);
   }
   Params p;
   p.lse = lse; p.delta = delta; p.dq_accum = dq_accum; p.dk = dk;
@@ -539,4 +553,26 @@ XB_API int xb_attn_bwd_ex(const void* q, const void* k, const void* v, const voi
   dim3 grid(tiles, Hkv);
   attn_bwd_kernel<<<grid, NUM_THREADS, SMEM_BYTES, st>>>(tq, tk, tv, tdo, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// Backward of xb_attn_fwd_hd64.  out_f32: the unrounded output of the forward.  dq, dk fp32
+// [T, H, 64], dv bf16 with token stride lddv; rows outside every sequence are zero.
+XB_API int xb_attn_bwd_hd64(const void* q, const void* k, const void* v, const float* out_f32, const void* dout,
+                            const float* lse, float* delta, float* dq, float* dk, void* dv, const int* cu_seqlens,
+                            long long ldq, long long ldk, long long ldv, long long lddo, long long lddv,
+                            int num_seqs, int T, int Hq, int Hkv, int causal, float scale, void* stream) {
+  using namespace xb_attn_bwd_ns;
+  if (T <= 0 || num_seqs <= 0) return 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (cudaMemsetAsync(dq, 0, (size_t)T * Hq * 64 * sizeof(float), st) != cudaSuccess ||
+      cudaMemsetAsync(dk, 0, (size_t)T * Hkv * 64 * sizeof(float), st) != cudaSuccess ||
+      cudaMemset2DAsync(dv, (size_t)lddv * 2, 0, (size_t)Hkv * 64 * 2, T, st) != cudaSuccess)
+    return -6;
+  const long long rows = (long long)T * Hq;
+  attn_delta_hd64_kernel<<<(int)((rows + 7) / 8), 256, 0, st>>>(out_f32, (const __nv_bfloat16*)dout, lddo, delta, T, Hq);
+  int rc = xb_attn_bwd_dkv(q, k, v, dout, lse, delta, dk, dv, cu_seqlens, nullptr, ldq, ldk, ldv, lddo, lddv,
+                           num_seqs, T, T, Hq, Hkv, 64, causal & 1, scale, 0, stream);
+  if (rc) return rc;
+  return xb_attn_bwd_dq(q, k, v, dout, lse, delta, dq, cu_seqlens, nullptr, ldq, ldk, ldv, lddo, num_seqs, T, T,
+                        Hq, Hkv, 64, causal & 1, scale, 0, 0, stream);
 }

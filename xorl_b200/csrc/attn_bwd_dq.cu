@@ -1,5 +1,5 @@
 // dQ of flash-attention backward without atomics (sm_100a; packed varlen, causal or full, GQA,
-// head_dim 128).
+// head_dim 128 or 64).
 //
 // One CTA owns a 128-row query tile of one query head and walks the 64-row key/value tiles it can
 // see.  Per step three tcgen05 GEMM groups:
@@ -18,7 +18,6 @@
 
 namespace xb_attn_dq_ns {
 
-constexpr int D = 128;
 constexpr int BQ = 128;
 constexpr int BKV = 64;
 constexpr int NS = 3;                          // K/V ring stages
@@ -28,17 +27,25 @@ constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0;                       // + 128 * buf
 constexpr int COL_DP = 64;                     // + 128 * buf
 constexpr int COL_DQ = 256;
-constexpr int KV_TILE_BYTES = BKV * D * 2;     // 16 KB : two d-chunks of [64 rows][128 B]
 constexpr int KV_CHUNK_BYTES = BKV * 128;
-constexpr int Q_TILE_BYTES = BQ * D * 2;       // 32 KB : two d-chunks of [128 rows][128 B]
 constexpr int Q_CHUNK_BYTES = BQ * 128;
 constexpr int DS_BYTES = BQ * BKV * 2;         // 16 KB : [128 q rows][64 kv = 128 B]
-constexpr int SMEM_Q = 0;
-constexpr int SMEM_DO = SMEM_Q + Q_TILE_BYTES;
-constexpr int SMEM_KV = SMEM_DO + Q_TILE_BYTES;                 // NS x (K tile, V tile)
-constexpr int SMEM_DS = SMEM_KV + NS * 2 * KV_TILE_BYTES;       // 2 buffers
-constexpr int SMEM_BAR = SMEM_DS + 2 * DS_BYTES;
-constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
+
+// Shared-memory layout by head dim; at 64, dS is the sum of two bf16 tiles (see attn_fwd.cu).
+template <int D>
+struct Cfg {
+  static constexpr bool SPLIT = D == 64;
+  static constexpr int CHUNKS = D / 64;
+  static constexpr int KV_TILE_BYTES = CHUNKS * KV_CHUNK_BYTES;
+  static constexpr int Q_TILE_BYTES = CHUNKS * Q_CHUNK_BYTES;
+  static constexpr int SMEM_Q = 0;
+  static constexpr int SMEM_DO = SMEM_Q + Q_TILE_BYTES;
+  static constexpr int SMEM_KV = SMEM_DO + Q_TILE_BYTES;                 // NS x (K tile, V tile)
+  static constexpr int SMEM_DS = SMEM_KV + NS * 2 * KV_TILE_BYTES;       // 2 buffers (high part, remainder)
+  static constexpr int DS_BUF = (SPLIT ? 2 : 1) * DS_BYTES;
+  static constexpr int SMEM_BAR = SMEM_DS + 2 * DS_BUF;
+  static constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
+};
 
 struct Params {
   const float* lse;     // [Hq, T]
@@ -65,10 +72,13 @@ struct __align__(8) Barriers {
   int abort_flag;
 };
 
+template <int D>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                    const Params p) {
+  using C = Cfg<D>;
+  constexpr int KV_TILE_BYTES = C::KV_TILE_BYTES, Q_TILE_BYTES = C::Q_TILE_BYTES;
   // tiles are numbered so that, inside a sequence, the last (most expensive under a causal mask)
   // query tile comes first
   const int tile_id = blockIdx.x;
@@ -99,7 +109,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~(uintptr_t)1023);
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + SMEM_BAR);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + C::SMEM_BAR);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -138,10 +148,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     if (lane == 0) {
       const int qtok = seq_start + q0;
       mbar_expect_tx(&bars->q_full, 2 * Q_TILE_BYTES);
-      tma_load_3d(smem + SMEM_Q, &tmap_q, &bars->q_full, 0, head, qtok);
-      tma_load_3d(smem + SMEM_Q + Q_CHUNK_BYTES, &tmap_q, &bars->q_full, 64, head, qtok);
-      tma_load_3d(smem + SMEM_DO, &tmap_do, &bars->q_full, 0, head, qtok);
-      tma_load_3d(smem + SMEM_DO + Q_CHUNK_BYTES, &tmap_do, &bars->q_full, 64, head, qtok);
+#pragma unroll
+      for (int c = 0; c < C::CHUNKS; ++c) {
+        tma_load_3d(smem + C::SMEM_Q + c * Q_CHUNK_BYTES, &tmap_q, &bars->q_full, c * 64, head, qtok);
+        tma_load_3d(smem + C::SMEM_DO + c * Q_CHUNK_BYTES, &tmap_do, &bars->q_full, c * 64, head, qtok);
+      }
       bool ok = true;
       int issued = 0;
       for (int j = 0; j < n_steps && ok; ++j) {
@@ -152,13 +163,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           break;
         }
         const int tok = k_start + (jt0 + j) * BKV;
-        uint8_t* sk = smem + SMEM_KV + s * 2 * KV_TILE_BYTES;
+        uint8_t* sk = smem + C::SMEM_KV + s * 2 * KV_TILE_BYTES;
         uint8_t* sv = sk + KV_TILE_BYTES;
         mbar_expect_tx(&bars->kv_full[s], 2 * KV_TILE_BYTES);
-        tma_load_3d(sk, &tmap_k, &bars->kv_full[s], 0, kv_head, tok);
-        tma_load_3d(sk + KV_CHUNK_BYTES, &tmap_k, &bars->kv_full[s], 64, kv_head, tok);
-        tma_load_3d(sv, &tmap_v, &bars->kv_full[s], 0, kv_head, tok);
-        tma_load_3d(sv + KV_CHUNK_BYTES, &tmap_v, &bars->kv_full[s], 64, kv_head, tok);
+#pragma unroll
+        for (int c = 0; c < C::CHUNKS; ++c) {
+          tma_load_3d(sk + c * KV_CHUNK_BYTES, &tmap_k, &bars->kv_full[s], c * 64, kv_head, tok);
+          tma_load_3d(sv + c * KV_CHUNK_BYTES, &tmap_v, &bars->kv_full[s], c * 64, kv_head, tok);
+        }
         issued = j + 1;
       }
       if (!ok) {
@@ -178,7 +190,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       constexpr uint32_t idesc_q = xb_idesc(1, 1, BQ, D, 0, 1);     // dS K (K tile MN-major)
       constexpr uint64_t kmaj = xb_smem_desc_base_sw128(16, 1024);
       constexpr uint64_t mn_kv = xb_smem_desc_base_sw128(KV_CHUNK_BYTES, 1024);
-      const uint32_t sq = xb_smem_u32(smem + SMEM_Q), sdo = xb_smem_u32(smem + SMEM_DO);
+      const uint32_t sq = xb_smem_u32(smem + C::SMEM_Q), sdo = xb_smem_u32(smem + C::SMEM_DO);
       bool ok = mbar_wait(&bars->q_full, 0, abort_flag, p.status, XB_K_ATTN_BWD, 600);
       auto issue_sdp = [&](int j) -> bool {
         const int s = j % NS, b = j & 1;
@@ -187,7 +199,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         if (!mbar_wait(&bars->sdp_empty[b], ((j >> 1) & 1) ^ 1, abort_flag, p.status, XB_K_ATTN_BWD, 620 + b))
           return false;
         tc_fence_after();
-        const uint32_t sk = xb_smem_u32(smem + SMEM_KV + s * 2 * KV_TILE_BYTES);
+        const uint32_t sk = xb_smem_u32(smem + C::SMEM_KV + s * 2 * KV_TILE_BYTES);
         const uint32_t sv = sk + KV_TILE_BYTES;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
@@ -217,12 +229,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           break;
         }
         tc_fence_after();
-        const uint32_t sk = xb_smem_u32(smem + SMEM_KV + s * 2 * KV_TILE_BYTES);
-        const uint32_t sds = xb_smem_u32(smem + SMEM_DS + b * DS_BYTES);
+        const uint32_t sk = xb_smem_u32(smem + C::SMEM_KV + s * 2 * KV_TILE_BYTES);
+        const uint32_t sds = xb_smem_u32(smem + C::SMEM_DS + b * C::DS_BUF);
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k) {
           tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + k * 32),
                         xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, (j > 0 || k > 0) ? 1u : 0u);
+          if constexpr (C::SPLIT)
+            tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + DS_BYTES + k * 32),
+                          xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, 1u);
         }
         tc_commit(&bars->kv_empty[s]);   // K_j (and V_j, read earlier) no longer needed
         tc_commit(&bars->ds_free[b]);
@@ -288,7 +303,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         ok = false;
         break;
       }
-      uint8_t* sd = smem + SMEM_DS + b * DS_BYTES + r * 128;
+      uint8_t* sd = smem + C::SMEM_DS + b * C::DS_BUF + r * 128;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int c16 = half * 4 + c;
@@ -298,6 +313,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         w.z = pack_bf16x2(ds[c * 8 + 4], ds[c * 8 + 5]);
         w.w = pack_bf16x2(ds[c * 8 + 6], ds[c * 8 + 7]);
         *reinterpret_cast<uint4*>(sd + ((c16 ^ (r & 7)) * 16)) = w;
+        if constexpr (C::SPLIT) {
+          uint4 w2;
+          w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
+          w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
+          w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
+          w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
+          *reinterpret_cast<uint4*>(sd + DS_BYTES + ((c16 ^ (r & 7)) * 16)) = w2;
+        }
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -309,12 +332,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
-      float* dst = p.dq + (tok * p.Hq + head) * D + half * 64;     // this thread: 64 of the 128 features
+      float* dst = p.dq + (tok * p.Hq + head) * D + half * (D / 2);     // this thread: half of the features
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < D / 64; ++c) {
         uint32_t a[32];
         if (n_steps > 0) {                                          // CTA-uniform
-          tmem_ld_32x32(tmem_base + lane_addr + COL_DQ + half * 64 + c * 32, a);
+          tmem_ld_32x32(tmem_base + lane_addr + COL_DQ + half * (D / 2) + c * 32, a);
           tc_wait_ld();
         } else {
 #pragma unroll
@@ -345,16 +368,33 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   }
 }
 
+template <int D>
+static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                  const Params& p, int tiles, cudaStream_t stream) {
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    if (cudaFuncSetAttribute(attn_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             Cfg<D>::SMEM_BYTES) != cudaSuccess)
+      return -10;
+    configured[dev & 63] = true;
+  }
+  attn_bwd_dq_kernel<D><<<dim3(tiles, p.Hq), NUM_THREADS, Cfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
 }  // namespace xb_attn_dq_ns
 
-// dq[T, Hq, 128] fp32 (= or +=) dS K for every query row; same tensor-map inputs as xb_attn_bwd_ex.
+// dq[T, Hq, D] fp32 (= or +=) dS K for every query row; same tensor-map inputs as xb_attn_bwd_ex.
 // max_q_tiles bounds the grid (>= sum over sequences of ceil(len / 128)); 0 = derive from T.
 XB_API int xb_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dout, const float* lse,
                           const float* delta, float* dq, const int* cu_seqlens, const int* k_starts,
                           long long ldq, long long ldk, long long ldv, long long lddo, int num_seqs, int T,
-                          int Tk, int Hq, int Hkv, int causal, float scale, int accumulate, int max_q_tiles,
-                          void* stream) {
+                          int Tk, int Hq, int Hkv, int D, int causal, float scale, int accumulate,
+                          int max_q_tiles, void* stream) {
   using namespace xb_attn_dq_ns;
+  if (D != 128 && D != 64) return -1;
   if (T <= 0 || num_seqs <= 0) return 0;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || Hq % Hkv) return -1;
   CUtensorMap tq, tk, tv, tdo;
@@ -375,17 +415,7 @@ XB_API int xb_attn_bwd_dq(const void* q, const void* k, const void* v, const voi
   p.num_seqs = num_seqs; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1; p.window = causal >> 1; p.accumulate = accumulate;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.status = xb_status_ptr();
-  static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!configured[dev & 63]) {
-    if (cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
-        cudaSuccess)
-      return -10;
-    configured[dev & 63] = true;
-  }
   const int tiles = max_q_tiles > 0 ? max_q_tiles : (T + BQ - 1) / BQ + num_seqs;
-  dim3 grid(tiles, Hq);
-  attn_bwd_dq_kernel<<<grid, NUM_THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(tq, tk, tv, tdo, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  return D == 128 ? launch<128>(tq, tk, tv, tdo, p, tiles, (cudaStream_t)stream)
+                  : launch<64>(tq, tk, tv, tdo, p, tiles, (cudaStream_t)stream);
 }

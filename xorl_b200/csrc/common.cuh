@@ -340,6 +340,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
+__device__ __forceinline__ float2 unpack_bf16x2(uint32_t u);
+// what rounding (lo, hi) to the packed pair `rounded` left over, as a bf16 pair
+__device__ __forceinline__ uint32_t pack_bf16x2_rest(float lo, float hi, uint32_t rounded) {
+  const float2 f = unpack_bf16x2(rounded);
+  return pack_bf16x2(lo - f.x, hi - f.y);
+}
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(v);
