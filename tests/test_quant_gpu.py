@@ -352,3 +352,44 @@ def test_mx_grouped_linear_gradients():
                 tol = 1e-6
             rel = (a - b).norm() / b.norm()
             assert rel <= tol, (mode, name, float(rel))
+
+
+@pytest.mark.parametrize("S,E", [(0, 4), (1, 1), (2, 8), (1000, 8), (1024, 16), (1025, 128), (32768, 16), (70000, 512),
+                                 (160000, 1024)])
+def test_moe_plan_matches_the_sorting_path(S, E):
+    from xorl_b200.ops import _lib, moe
+    torch.manual_seed(S)
+    ids = torch.randint(0, E, (S,), device="cuda")
+    ids[ids == E // 2] = 0                                   # an expert without rows, one with more than its share
+    rows = moe.buffer_rows(S, E)
+    dest, seg, slot = moe.sort_plan(ids, E, rows)
+    d0, s0, _ = moe.aligned_sort_indices(ids, E)
+    inv = torch.full((rows,), -1, device="cuda", dtype=torch.int32)
+    inv[d0] = torch.arange(S, device="cuda", dtype=torch.int32)
+    assert torch.equal(dest, d0) and torch.equal(seg, s0) and torch.equal(slot, inv)
+    assert _lib.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("T,E,k,renorm,scale", [(1, 1, 1, True, 1.0), (300, 8, 2, True, 1.0), (513, 128, 8, True, 2.5),
+                                                (77, 60, 3, False, 0.5), (64, 512, 32, True, 1.0)])
+def test_chosen_weights_and_balancing_loss_match_torch(T, E, k, renorm, scale):
+    from xorl_b200.ops import moe
+    torch.manual_seed(T)
+    logits = torch.randn(T, E, device="cuda")
+    idx = torch.randint(0, E, (T, k), device="cuda")         # with repeats: both slots contribute
+    counts = moe.expert_histogram(idx, E)
+    gw = torch.randn(T, k, device="cuda")
+
+    def run(kernels):
+        x = logits.clone().requires_grad_()
+        p = torch.softmax(x, -1)
+        if kernels:
+            w, aux = moe.chosen_weights(p, idx, renorm, scale), moe.load_balancing_loss(p, idx, E, counts=counts, scale=0.3)
+        else:
+            w = moe._renorm_reference(p, idx, renorm, scale)
+            aux = 0.3 * E * torch.dot(counts.float() / (T * k), p.mean(0))
+        ((w * gw).sum() + 7 * aux).backward()
+        return w.detach(), aux.detach(), x.grad
+
+    for got, ref in zip(run(True), run(False)):
+        torch.testing.assert_close(got, ref, rtol=2e-5, atol=2e-6)

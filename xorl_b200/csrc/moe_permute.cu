@@ -11,6 +11,9 @@
 //                        weighted combine of the k expert outputs of a token; backward of the
 //                        permutation (w = null)
 //   xb_moe_slot_dots     dw[t,j] = <dout[t], y[idx[t,j]]>        gradient of the routing weights
+//   xb_moe_gather_slots  as gather_rows over a map row -> slot (token = slot / k)
+//   xb_moe_combine_bwd   both gradients of the weighted combine in one pass over the buffer rows:
+//                        dy[r] = w[slot] * dout[token], dw[slot] = <dout[token], y[r]>
 #include "common.cuh"
 
 namespace {
@@ -29,7 +32,7 @@ __device__ __forceinline__ uint4 pack8(const float (&a)[8]) {
 
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(uint4* __restrict__ out, long long ld_out, const uint4* __restrict__ in, long long ld_in,
-                   const int* __restrict__ src, const float* __restrict__ scale, int rows, int vecs) {
+                   const int* __restrict__ src, const float* __restrict__ scale, int k, int rows, int vecs) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int r = warp; r < rows; r += nwarps) {
@@ -39,7 +42,7 @@ gather_rows_kernel(uint4* __restrict__ out, long long ld_out, const uint4* __res
       for (int v = lane; v < vecs; v += 32) o[v] = make_uint4(0, 0, 0, 0);
       continue;
     }
-    const uint4* i = in + (long long)s * ld_in;
+    const uint4* i = in + (long long)(s / k) * ld_in;
     if (scale == nullptr) {
       for (int v = lane; v < vecs; v += 32) o[v] = i[v];
     } else {
@@ -93,6 +96,40 @@ slot_dots_kernel(float* __restrict__ dw, const uint4* __restrict__ dout, long lo
   if (lane == 0) dw[warp] = s;
 }
 
+// dout rows are read k times out of L2; y and dy stream through once each
+__global__ void __launch_bounds__(256)
+combine_bwd_kernel(uint4* __restrict__ dy, long long ld_dy, float* __restrict__ dw, const uint4* __restrict__ dout,
+                   long long ld_do, const uint4* __restrict__ y, long long ld_y, const int* __restrict__ slot,
+                   const float* __restrict__ w, int k, int rows, int vecs) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (int r = warp; r < rows; r += nwarps) {
+    const int s = slot[r];
+    uint4* o = dy + (long long)r * ld_dy;
+    if (s < 0) {
+      for (int v = lane; v < vecs; v += 32) o[v] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    const uint4* a = dout + (long long)(s / k) * ld_do;
+    const uint4* b = y + (long long)r * ld_y;
+    const float ws = w[s];
+    float dot = 0.f;
+#pragma unroll 4
+    for (int v = lane; v < vecs; v += 32) {
+      const uint4 x = a[v], z = b[v];
+      float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      fma8(g, x, ws);
+      o[v] = pack8(g);
+      const float2 x0 = unpack_bf16x2(x.x), x1 = unpack_bf16x2(x.y), x2 = unpack_bf16x2(x.z), x3 = unpack_bf16x2(x.w);
+      const float2 z0 = unpack_bf16x2(z.x), z1 = unpack_bf16x2(z.y), z2 = unpack_bf16x2(z.z), z3 = unpack_bf16x2(z.w);
+      dot += x0.x * z0.x + x0.y * z0.y + x1.x * z1.x + x1.y * z1.y + x2.x * z2.x + x2.y * z2.y + x3.x * z3.x +
+             x3.y * z3.y;
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) dw[s] = dot;
+  }
+}
+
 inline int grid_for(long long warps) {
   long long blocks = (warps + 7) / 8;
   const long long cap = 148ll * 16;
@@ -107,7 +144,28 @@ XB_API int xb_moe_gather_rows(void* out, long long ld_out, const void* in, long 
   if (rows <= 0) return 0;
   if (width % 8 || ld_out % 8 || ld_in % 8) return -1;
   gather_rows_kernel<<<grid_for(rows), 256, 0, (cudaStream_t)stream>>>((uint4*)out, ld_out / 8, (const uint4*)in,
-                                                                        ld_in / 8, src, scale, rows, width / 8);
+                                                                        ld_in / 8, src, scale, 1, rows, width / 8);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// slot: the slot of every row, or -1 for a zero row; row r is in[slot / k]
+XB_API int xb_moe_gather_slots(void* out, long long ld_out, const void* in, long long ld_in, const int* slot,
+                               int k, int rows, int width, void* stream) {
+  if (rows <= 0) return 0;
+  if (width % 8 || ld_out % 8 || ld_in % 8 || k <= 0) return -1;
+  gather_rows_kernel<<<grid_for(rows), 256, 0, (cudaStream_t)stream>>>((uint4*)out, ld_out / 8, (const uint4*)in,
+                                                                        ld_in / 8, slot, nullptr, k, rows, width / 8);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// y, dy [rows, width]; dout [T, width]; w, dw fp32 [T * k]; slot int32 [rows] names every slot once
+XB_API int xb_moe_combine_bwd(void* dy, long long ld_dy, float* dw, const void* dout, long long ld_do, const void* y,
+                              long long ld_y, const int* slot, const float* w, int k, int rows, int width,
+                              void* stream) {
+  if (rows <= 0) return 0;
+  if (width % 8 || ld_dy % 8 || ld_do % 8 || ld_y % 8 || k <= 0) return -1;
+  combine_bwd_kernel<<<grid_for(rows), 256, 0, (cudaStream_t)stream>>>(
+      (uint4*)dy, ld_dy / 8, dw, (const uint4*)dout, ld_do / 8, (const uint4*)y, ld_y / 8, slot, w, k, rows, width / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -181,19 +181,16 @@ class MoEBlock(nn.Module):
             # replay recorded expert choices (recompute / pipeline backward / rollout routing);
             # the weights are re-derived from the current probabilities so gradients still flow
             indices = replay
-            weights = probs.gather(1, indices)
-            if self.cfg.norm_topk_prob:
-                weights = weights / weights.sum(-1, keepdim=True).clamp_min(1e-20)
-            if self.gate.scale != 1.0 and self.gate.scoring != "softmax_after_topk":
-                weights = weights * self.gate.scale
+            scale = self.gate.scale if self.gate.scoring != "softmax_after_topk" else 1.0
+            weights = moe_ops.chosen_weights(probs, indices, self.cfg.norm_topk_prob, scale)
         elif ctx.aux.get("record_routing", False):
             ctx.aux[("routing_record", self.layer_idx)] = indices.detach()
         counts = None
         if ctx.training and self.aux_coef > 0 and ctx.aux.get("aux_loss_scale") is not None:
             counts = moe_ops.expert_histogram(indices, self.cfg.num_experts)
-            aux = moe_ops.load_balancing_loss(probs, indices, self.cfg.num_experts,
-                                              ctx.aux.get("aux_global_group"), counts=counts)
-            ctx.aux[("aux_loss", self.layer_idx)] = aux * (self.aux_coef * ctx.aux["aux_loss_scale"])
+            ctx.aux[("aux_loss", self.layer_idx)] = moe_ops.load_balancing_loss(
+                probs, indices, self.cfg.num_experts, ctx.aux.get("aux_global_group"), counts=counts,
+                scale=self.aux_coef * ctx.aux["aux_loss_scale"])
         if ctx.aux.get("collect_expert_load", False):
             if counts is None:
                 counts = moe_ops.expert_histogram(indices, self.cfg.num_experts)

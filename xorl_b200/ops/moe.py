@@ -35,7 +35,7 @@ _SCORING_ID = {"softmax": 0, "sigmoid": 1, "softmax_after_topk": 2}
 
 class _RouteKernel(torch.autograd.Function):
     """Forward: one fused kernel (csrc/moe_route.cu).  Backward: closed forms on the saved
-    probabilities / choices (a few [T, E] elementwise ops)."""
+    probabilities / choices in one kernel (csrc/moe_plan.cu)."""
 
     @staticmethod
     def forward(ctx, logits, bias, k, renorm, scoring, scale):
@@ -52,12 +52,28 @@ class _RouteKernel(torch.autograd.Function):
         ctx.save_for_backward(probs, idx, w)
         ctx.cfg = (renorm, scoring, scale)
         ctx.mark_non_differentiable(idx)
+        ctx.set_materialize_grads(False)
         return w, idx, probs
 
     @staticmethod
     def backward(ctx, dw, _didx, dprobs):
+        global _launches
         probs, idx, w = ctx.saved_tensors
         renorm, scoring, scale = ctx.cfg
+        if dw is None and dprobs is None:
+            return (None,) * 6
+        if not torch.is_grad_enabled() and scale != 0:
+            T, E = probs.shape
+            dw = dw.contiguous() if dw is not None else None
+            if dprobs is not None and dprobs.stride(1) != 1:
+                dprobs = dprobs.contiguous()
+            dlogits = torch.empty_like(probs)
+            _lib.check(_lib.cuda_lib().xb_moe_route_bwd(
+                _lib.ptr(dw), _lib.ptr(dprobs), 0 if dprobs is None else dprobs.stride(0), probs.data_ptr(),
+                idx.data_ptr(), w.data_ptr(), dlogits.data_ptr(), T, E, idx.shape[1], _SCORING_ID[scoring],
+                int(renorm), float(scale), _lib.stream_ptr()), "xb_moe_route_bwd")
+            _launches += 1
+            return dlogits, None, None, None, None, None
         dp = dprobs.clone() if dprobs is not None else torch.zeros_like(probs)
         dlogits = None
         if dw is not None:
@@ -122,6 +138,62 @@ def topk_route(logits: torch.Tensor, k: int, renorm: bool = True, scoring: str =
     return weights, indices, probs
 
 
+class _RenormKernel(torch.autograd.Function):
+    """probs [T, E] -> scale * p / max(sum p, 1e-20) of the chosen ``indices`` [T, k] (``renorm`` False:
+    scale * p)."""
+
+    @staticmethod
+    def forward(ctx, probs, indices, renorm, scale):
+        global _launches
+        p = probs.gather(1, indices)
+        T, k = p.shape
+        w = torch.empty_like(p)
+        _lib.check(_lib.cuda_lib().xb_moe_renorm(p.data_ptr(), w.data_ptr(), T, k, int(renorm), float(scale),
+                                                 _lib.stream_ptr()), "xb_moe_renorm")
+        _launches += 1
+        ctx.save_for_backward(probs, indices, p)
+        ctx.cfg = (renorm, scale)
+        return w
+
+    @staticmethod
+    def backward(ctx, dw):
+        global _launches
+        probs, indices, p = ctx.saved_tensors
+        renorm, scale = ctx.cfg
+        if torch.is_grad_enabled():              # a graph of the gradient is wanted
+            return (*torch.autograd.grad(_renorm_reference(probs, indices, renorm, scale), probs, dw,
+                                         create_graph=True), None, None, None)
+        T, E = probs.shape
+        dw = dw.contiguous()
+        dprobs = torch.empty_like(probs)
+        _lib.check(_lib.cuda_lib().xb_moe_renorm_bwd(dw.data_ptr(), p.data_ptr(), indices.data_ptr(),
+                                                     dprobs.data_ptr(), T, E, p.shape[1], int(renorm), float(scale),
+                                                     _lib.stream_ptr()), "xb_moe_renorm_bwd")
+        _launches += 1
+        return dprobs, None, None, None
+
+
+def _renorm_reference(probs, indices, renorm: bool, scale: float):
+    weights = probs.gather(1, indices)
+    if renorm:
+        weights = weights / weights.sum(-1, keepdim=True).clamp_min(1e-20)
+    return weights * scale if scale != 1.0 else weights
+
+
+def _plain_autograd() -> bool:
+    """No function transform or forward-mode derivative is active (those go through torch operations)."""
+    return not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+
+
+def chosen_weights(probs: torch.Tensor, indices: torch.Tensor, renorm: bool, scale: float = 1.0) -> torch.Tensor:
+    """Routing weights [T, k] of given expert choices, re-derived from the router's probabilities [T, E]."""
+    if (probs.is_cuda and probs.dtype == torch.float32 and probs.is_contiguous() and indices.dtype == torch.int64
+            and indices.is_cuda and 0 < indices.shape[1] <= 32 and probs.shape[0] == indices.shape[0]
+            and _lib.have_cuda_lib() and _plain_autograd()):
+        return _RenormKernel.apply(probs, indices.contiguous(), bool(renorm), float(scale))
+    return _renorm_reference(probs, indices, renorm, scale)
+
+
 def expert_histogram(indices: torch.Tensor, num_experts: int) -> torch.Tensor:
     """int32 [E]: number of (token, slot) pairs routed to every expert (one kernel on CUDA)."""
     global _launches
@@ -136,14 +208,51 @@ def expert_histogram(indices: torch.Tensor, num_experts: int) -> torch.Tensor:
     return torch.bincount(flat, minlength=num_experts).to(torch.int32)
 
 
+class _AuxKernel(torch.autograd.Function):
+    """factor * sum_t sum_e counts[e] probs[t, e].  The gradient is the same for every token, so it is
+    formed once per expert and handed on as a broadcast view."""
+
+    @staticmethod
+    def forward(ctx, probs, counts, factor):
+        global _launches
+        T, E = probs.shape
+        lib = _lib.cuda_lib()
+        ws = torch.empty(lib.xb_moe_aux_workspace(), device=probs.device, dtype=torch.float32)
+        out = torch.empty((), device=probs.device, dtype=torch.float32)
+        _lib.check(lib.xb_moe_aux(probs.data_ptr(), counts.data_ptr(), ws.data_ptr(), out.data_ptr(), T, E, factor,
+                                  _lib.stream_ptr()), "xb_moe_aux")
+        _launches += 1
+        ctx.save_for_backward(counts)
+        ctx.cfg = (T, E, factor)
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        global _launches
+        (counts,) = ctx.saved_tensors
+        T, E, factor = ctx.cfg
+        if torch.is_grad_enabled():
+            return (g * (counts.float() * factor)).expand(T, E), None, None
+        out = torch.empty(E, device=counts.device, dtype=torch.float32)
+        _lib.check(_lib.cuda_lib().xb_moe_aux_grad(g.data_ptr(), counts.data_ptr(), out.data_ptr(), E, factor,
+                                                   _lib.stream_ptr()), "xb_moe_aux_grad")
+        _launches += 1
+        return out.expand(T, E), None, None
+
+
 def load_balancing_loss(probs: torch.Tensor, indices: torch.Tensor, num_experts: int,
-                        global_group=None, counts: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``E * sum_e f_e * P_e`` with f_e the fraction of routed slots sent to expert e and P_e the
+                        global_group=None, counts: Optional[torch.Tensor] = None,
+                        scale: float = 1.0) -> torch.Tensor:
+    """``scale * E * sum_e f_e * P_e`` with f_e the fraction of routed slots sent to expert e and P_e the
     mean router probability.  With ``global_group`` the counts are summed over that group.
     ``counts``: the per-expert histogram of ``indices`` when the caller already has it."""
     T, k = indices.shape
     if counts is None:
         counts = expert_histogram(indices, num_experts)
+    if (global_group is None and T > 0 and probs.is_cuda and probs.dtype == torch.float32 and probs.is_contiguous()
+            and probs.shape == (T, num_experts) and counts.dtype == torch.int32 and counts.numel() == num_experts
+            and counts.is_contiguous() and _lib.have_cuda_lib() and _plain_autograd()):
+        return _AuxKernel.apply(probs, counts, float(scale) * num_experts / (float(T) * k * T))
     counts = counts.float()
     if global_group is not None:
         total = torch.tensor(float(T), device=probs.device)
@@ -152,7 +261,8 @@ def load_balancing_loss(probs: torch.Tensor, indices: torch.Tensor, num_experts:
         f = counts / (total * k)
     else:
         f = counts * (1.0 / (T * k))
-    return num_experts * torch.dot(f, probs.mean(0))
+    loss = num_experts * torch.dot(f, probs.mean(0))
+    return loss * scale if scale != 1.0 else loss
 
 
 # --------------------------------------------------------------------------------------------
@@ -178,6 +288,26 @@ def aligned_sort_indices(expert_ids: torch.Tensor, num_experts: int, align: int 
     dest = torch.empty_like(dest_sorted)
     dest[order] = dest_sorted
     return dest, seg.to(torch.int32), counts
+
+
+PLAN_MAX_EXPERTS = 1024
+
+
+def sort_plan(expert_ids: torch.Tensor, num_experts: int, rows: int):
+    """``aligned_sort_indices`` for int64 ids on the GPU in two launches, without the host waiting for the
+    counts: (dest int64 [S], seg int32 [E+1], slot_of_row int32 [rows], -1 for padding rows).  An id
+    outside the experts is placed nowhere (``dest`` 0) and raises the status word."""
+    global _launches
+    S, dev = expert_ids.numel(), expert_ids.device
+    lib = _lib.cuda_lib()
+    ws = torch.empty(lib.xb_moe_plan_workspace(S, num_experts), device=dev, dtype=torch.int32)
+    dest = torch.empty(S, device=dev, dtype=torch.int64)
+    seg = torch.empty(num_experts + 1, device=dev, dtype=torch.int32)
+    slot_of_row = torch.empty(rows, device=dev, dtype=torch.int32)
+    _lib.check(lib.xb_moe_plan(expert_ids.data_ptr(), S, num_experts, SEG_ALIGN, rows, ws.data_ptr(), dest.data_ptr(),
+                               seg.data_ptr(), slot_of_row.data_ptr(), _lib.stream_ptr()), "xb_moe_plan")
+    _launches += 2
+    return dest, seg, slot_of_row
 
 
 def buffer_rows(num_slots: int, num_experts: int, align: int = SEG_ALIGN) -> int:
@@ -412,9 +542,17 @@ class _Permute(torch.autograd.Function):
     """x [T,H] -> buffer [rows,H]: row dest[t,j] holds x[t]; rows nobody owns are zero."""
 
     @staticmethod
-    def forward(ctx, x, dest, tok_of_row):
+    def forward(ctx, x, dest, slot_of_row):
+        global _launches
         ctx.save_for_backward(dest)
-        return _gather_rows(x, tok_of_row, tok_of_row.numel())
+        x = x.contiguous()
+        rows, H = slot_of_row.numel(), x.shape[1]
+        out = torch.empty((rows, H), device=x.device, dtype=x.dtype)
+        _lib.check(_lib.cuda_lib().xb_moe_gather_slots(out.data_ptr(), H, x.data_ptr(), H, slot_of_row.data_ptr(),
+                                                       dest.shape[1], rows, H, _lib.stream_ptr()),
+                   "xb_moe_gather_slots")
+        _launches += 1
+        return out
 
     @staticmethod
     def backward(ctx, dbuf):
@@ -426,25 +564,24 @@ class _Combine(torch.autograd.Function):
     """out[t] = sum_j w[t,j] * y[dest[t,j]] (fp32 accumulation, bf16 result)."""
 
     @staticmethod
-    def forward(ctx, y, w, dest, tok_of_row):
+    def forward(ctx, y, w, dest, slot_of_row):
         w = w.float().contiguous()
-        ctx.save_for_backward(y, w, dest, tok_of_row)
+        y = y.contiguous()
+        ctx.save_for_backward(y, w, dest, slot_of_row)
         return _gather_sum(y, dest, w)
 
     @staticmethod
     def backward(ctx, dout):
         global _launches
-        y, w, dest, tok_of_row = ctx.saved_tensors
+        y, w, dest, slot_of_row = ctx.saved_tensors
         dout = dout.contiguous()
-        rows = y.shape[0]
-        T, k = dest.shape
-        scale_row = torch.zeros(rows, device=y.device, dtype=torch.float32)
-        scale_row[dest.reshape(-1)] = w.reshape(-1)
-        dy = _gather_rows(dout, tok_of_row, rows, scale_row)
-        dw = torch.empty((T, k), device=y.device, dtype=torch.float32)
-        _lib.check(_lib.cuda_lib().xb_moe_slot_dots(dw.data_ptr(), dout.data_ptr(), dout.stride(0), y.data_ptr(),
-                                                    y.stride(0), dest.data_ptr(), T, k, y.shape[1],
-                                                    _lib.stream_ptr()), "xb_moe_slot_dots")
+        rows, H = y.shape
+        dy = torch.empty_like(y)
+        dw = torch.empty_like(w)
+        _lib.check(_lib.cuda_lib().xb_moe_combine_bwd(dy.data_ptr(), H, dw.data_ptr(), dout.data_ptr(), H,
+                                                      y.data_ptr(), H, slot_of_row.data_ptr(), w.data_ptr(),
+                                                      dest.shape[1], rows, H, _lib.stream_ptr()),
+                   "xb_moe_combine_bwd")
         _launches += 1
         return dy, dw, None, None
 
@@ -479,14 +616,16 @@ def local_moe_forward(x: torch.Tensor, weights: torch.Tensor, indices: torch.Ten
     combine the k expert outputs of every token with its routing weights (fp32 accumulation)."""
     T, H = x.shape
     k = indices.shape[1]
-    dest, seg, _ = aligned_sort_indices(indices.reshape(-1), num_experts)
     rows = buffer_rows(T * k, num_experts)
-    if _permute_kernels_ok(x) and not canonical:
-        tok = token_of_row(dest, rows, k)
+    flat = indices.reshape(-1)
+    if (_permute_kernels_ok(x) and not canonical and flat.dtype == torch.int64 and num_experts <= PLAN_MAX_EXPERTS
+            and rows < 2 ** 31):
+        dest, seg, slot_of_row = sort_plan(flat.contiguous(), num_experts, rows)
         dest2 = dest.view(T, k)
-        buf = _Permute.apply(x, dest2, tok)
+        buf = _Permute.apply(x, dest2, slot_of_row)
         y = expert_mlp_aligned(buf, seg, experts.gate_up_proj, experts.down_proj, **experts_mlp_kwargs(experts))
-        return _Combine.apply(y, weights, dest2, tok)
+        return _Combine.apply(y, weights, dest2, slot_of_row)
+    dest, seg, _ = aligned_sort_indices(flat, num_experts)
     token_of_slot = torch.arange(T, device=x.device).repeat_interleave(k)
     buf = x.new_zeros((rows, H)).index_copy(0, dest, x.index_select(0, token_of_slot))
     y = expert_mlp_aligned(buf, seg, experts.gate_up_proj, experts.down_proj, **experts_mlp_kwargs(experts))

@@ -540,7 +540,6 @@ def fused_ep_forward(x, weights, indices, experts, num_experts, ctx):
     if moe_ops._permute_kernels_ok(x):
         # weighted sum over the k slots of a token in one gather kernel (slot rows are contiguous)
         slots = torch.arange(T * k, device=x.device).view(T, k)
-        tok = (torch.arange(T * k, device=x.device) // k).to(torch.int32)
-        return moe_ops._Combine.apply(y_slots, weights, slots, tok)
+        return moe_ops._Combine.apply(y_slots, weights, slots, slots.view(-1).to(torch.int32))
     out = (y_slots.view(T, k, H).float() * weights.unsqueeze(-1).float()).sum(1)
     return out.to(x.dtype)
