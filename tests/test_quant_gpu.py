@@ -393,3 +393,35 @@ def test_chosen_weights_and_balancing_loss_match_torch(T, E, k, renorm, scale):
 
     for got, ref in zip(run(True), run(False)):
         torch.testing.assert_close(got, ref, rtol=2e-5, atol=2e-6)
+
+
+@pytest.mark.parametrize("counts,K,N", [([0, 130, 1, 0], 256, 264), ([3], 128, 128), ([0, 0], 64, 512), ([100] * 130, 64, 72)])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.float32, False), (torch.float32, True), (torch.bfloat16, False),
+                                              (torch.bfloat16, True)])
+def test_grouped_gemm_writes_all_rows_and_experts(counts, K, N, dtype, accumulate):
+    """Rows behind the last segment are zero without a fill; weight gradients of every output form, experts
+    without rows and row counts of an expert that are no multiple of a tile included."""
+    from xorl_b200.ops import _lib, moe
+    torch.manual_seed(K)
+    E = len(counts)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).cuda()
+    dest, seg, _ = moe.aligned_sort_indices(ids, E)
+    rows = moe.buffer_rows(ids.numel(), E)
+    x = torch.zeros(rows, K, device="cuda", dtype=torch.bfloat16)
+    x[dest] = torch.randn(ids.numel(), K, device="cuda").bfloat16()
+    w = torch.randn(E, K, N, device="cuda", dtype=torch.bfloat16)
+    y = torch.full((rows, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    moe._grouped_rows_cuda(x, w, seg, y, b_kmajor=False, zero_tail=True)
+    s = seg.tolist()
+    assert (y[s[E]:] == 0).all()
+    out0 = torch.randn(E, K, N, device="cuda").to(dtype)
+    out = out0.clone() if accumulate else torch.full_like(out0, float("nan"))
+    dy = torch.randn(rows, N, device="cuda", dtype=torch.bfloat16)
+    moe._grouped_wgrad_cuda(x, dy, seg, out, accumulate)
+    for e in range(E):
+        a = x[s[e]:s[e + 1]].double()
+        # fp32 sums of up to 256 products, one bf16 rounding where the output has it
+        torch.testing.assert_close(y[s[e]:s[e + 1]].double(), a @ w[e].double(), rtol=2 ** -8, atol=1e-3)
+        ref = a.t() @ dy[s[e]:s[e + 1]].double() + (out0[e].double() if accumulate else 0)
+        torch.testing.assert_close(out[e].double(), ref, rtol=2 ** -8 if dtype == torch.bfloat16 else 1e-4, atol=1e-3)
+    assert _lib.read_status()[0] == 0

@@ -171,6 +171,29 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const vo
                "r"(xb_smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(xb_smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* m, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)),
+               "r"(xb_smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+// Expert that row m0 belongs to (-1: behind the last segment), from the segment starts in shared memory.
+// A scan over the experts costs a load each; with 128 of them that is as long as a short tile's math.
+__device__ __forceinline__ int xb_expert_of_row(const int* seg, int E, int m0) {
+  if (m0 >= seg[E]) return -1;
+  int lo = 0, hi = E;                 // seg[lo] <= m0 < seg[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (seg[mid] <= m0) lo = mid; else hi = mid;
+  }
+  return lo;
+}
 __device__ __forceinline__ void tma_store_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }

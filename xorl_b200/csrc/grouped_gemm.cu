@@ -33,6 +33,8 @@ struct Params {
   long long ldc;       // rows mode: row stride of C; wgrad: N (row stride inside one expert)
   int out_fp32, accumulate;
   int b_mn;            // rows mode: B stored [E,K,N] (1) or [E,N,K] (0)
+  int zero_tail;       // rows mode: rows behind the last segment are zeroed
+  int tma_out;         // the output goes through shared memory and TMA (wgrad: see below)
   int num_m_blocks, num_n_blocks;
   int* status;
 };
@@ -65,11 +67,8 @@ __device__ __forceinline__ Tile get_tile(const Params& p, const int* sseg, int t
     r.n0 = nb * BN;
     r.k0 = 0;
     r.num_kb = (p.K + BK - 1) / BK;
-    int e = -1;
-    for (int i = 0; i < p.E; ++i)
-      if (r.m0 >= sseg[i] && r.m0 < sseg[i + 1]) { e = i; break; }
-    r.e = e;
-    r.valid = e >= 0;
+    r.e = xb_expert_of_row(sseg, p.E, r.m0);
+    r.valid = r.e >= 0;
   } else {
     const int per_e = p.num_m_blocks * p.num_n_blocks;
     r.e = t / per_e;
@@ -103,7 +102,7 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    if (p.mode == 0) tma_prefetch_desc(&tmap_c);
+    if (p.tma_out) tma_prefetch_desc(&tmap_c);
   }
   if (warp == 1) { tmem_alloc(&bars->tmem_base, TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
@@ -199,7 +198,15 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const Tile tl = get_tile(p, sseg, t);
-      if (!tl.valid) continue;
+      if (!tl.valid) {
+        if (p.zero_tail) {               // a warp writes 32 rows, 512 bytes of one row at a time
+          const int col = tl.n0 + lane * 8;
+          for (int i = 0; i < 32 && col < p.N; ++i)
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) +
+                                      (long long)(tl.m0 + q * 32 + i) * p.ldc + col) = make_uint4(0, 0, 0, 0);
+        }
+        continue;
+      }
       const bool has_acc = tl.num_kb > 0;
       const int acc = tcount & 1;
       if (has_acc) {
@@ -209,50 +216,69 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       } else if (p.accumulate) {
         continue;  // nothing to add for an expert without tokens
       }
-      if (p.mode == 0) {
-        // rows mode (bf16 out, no accumulation): stage 64-column slabs in 128B-swizzled shared memory
-        // and let TMA write them, so that global memory sees whole 128-byte row segments
+      if (p.tma_out) {
+        // Stage 128-byte wide slabs (64 bf16 or 32 fp32 columns) in 128B-swizzled shared memory and let
+        // TMA write them, or add them, so that global memory sees whole 128-byte row segments.  A thread
+        // holds one row: its own stores would touch 32 rows at once, 16 bytes of each.
         const int r = q * 32 + lane;
         const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
         uint8_t* slab = smem + OFF_SLAB;
         uint8_t* srow = slab + r * 128;
+        const int slab_cols = p.out_fp32 ? SLAB_COLS / 2 : SLAB_COLS;
 #pragma unroll 1
-        for (int sl = 0; sl < BN / SLAB_COLS; ++sl) {
-          const int col0 = tl.n0 + sl * SLAB_COLS;
+        for (int c0 = 0; c0 < BN; c0 += slab_cols) {
+          const int col0 = tl.n0 + c0;
           if (col0 >= p.N) break;
           uint32_t v[2][32];
-          tmem_ld_32x32(taddr + sl * SLAB_COLS, v[0]);
-          tmem_ld_32x32(taddr + sl * SLAB_COLS + 32, v[1]);
-          tc_wait_ld();
+          if (has_acc) {
+            tmem_ld_32x32(taddr + c0, v[0]);
+            if (!p.out_fp32) tmem_ld_32x32(taddr + c0 + 32, v[1]);
+            tc_wait_ld();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[0][i] = v[1][i] = 0;
+          }
           if (warp == 2 && lane == 0) tma_store_wait_read<0>();
           asm volatile("bar.sync 2, 128;" ::: "memory");
+          if (p.out_fp32) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(srow + ((j ^ (r & 7)) * 16)) =
+                  make_uint4(v[0][4 * j], v[0][4 * j + 1], v[0][4 * j + 2], v[0][4 * j + 3]);
+          } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 o;
-              o.x = pack_bf16x2(__uint_as_float(v[h][8 * j]), __uint_as_float(v[h][8 * j + 1]));
-              o.y = pack_bf16x2(__uint_as_float(v[h][8 * j + 2]), __uint_as_float(v[h][8 * j + 3]));
-              o.z = pack_bf16x2(__uint_as_float(v[h][8 * j + 4]), __uint_as_float(v[h][8 * j + 5]));
-              o.w = pack_bf16x2(__uint_as_float(v[h][8 * j + 6]), __uint_as_float(v[h][8 * j + 7]));
-              *reinterpret_cast<uint4*>(srow + (((h * 4 + j) ^ (r & 7)) * 16)) = o;
-            }
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                uint4 o;
+                o.x = pack_bf16x2(__uint_as_float(v[h][8 * j]), __uint_as_float(v[h][8 * j + 1]));
+                o.y = pack_bf16x2(__uint_as_float(v[h][8 * j + 2]), __uint_as_float(v[h][8 * j + 3]));
+                o.z = pack_bf16x2(__uint_as_float(v[h][8 * j + 4]), __uint_as_float(v[h][8 * j + 5]));
+                o.w = pack_bf16x2(__uint_as_float(v[h][8 * j + 6]), __uint_as_float(v[h][8 * j + 7]));
+                *reinterpret_cast<uint4*>(srow + (((h * 4 + j) ^ (r & 7)) * 16)) = o;
+              }
+          }
           fence_proxy_async_smem();
           asm volatile("bar.sync 2, 128;" ::: "memory");
           if (warp == 2 && lane == 0) {
-            tma_store_2d(&tmap_c, slab, col0, tl.m0);
+            if (p.mode == 0) tma_store_2d(&tmap_c, slab, col0, tl.m0);
+            else if (p.accumulate) tma_reduce_add_3d(&tmap_c, slab, col0, tl.m0, tl.e);
+            else tma_store_3d(&tmap_c, slab, col0, tl.m0, tl.e);
             tma_store_commit();
           }
         }
-        tc_fence_before();
-        mbar_arrive(&bars->tmem_empty[acc]);
-        ++tcount;
+        if (has_acc) {
+          tc_fence_before();
+          mbar_arrive(&bars->tmem_empty[acc]);
+          ++tcount;
+        }
         continue;
       }
+      // wgrad added to a bf16 buffer, or an output that TMA cannot address
       const int row = tl.m0 + q * 32 + lane;
-      const int row_limit = p.mode == 0 ? p.R : p.M;
+      const int row_limit = p.M;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
-      const long long base = p.mode == 0 ? 0 : (long long)tl.e * p.M * p.N;
+      const long long base = (long long)tl.e * p.M * p.N;
       const int es = p.out_fp32 ? 4 : 2;
       const bool vec_ok = (p.ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(p.C) % 16) == 0;
 #pragma unroll 1
@@ -320,7 +346,7 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         ++tcount;
       }
     }
-    if (p.mode == 0 && warp == 2 && lane == 0) tma_store_wait<0>();
+    if (p.tma_out && warp == 2 && lane == 0) tma_store_wait<0>();
   }
   tc_fence_before();
   __syncthreads();
@@ -347,7 +373,8 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
 }  // namespace xb_ggemm
 
 // A [R, K] (row stride lda), B [E, K, N] (b_mn = 1) or [E, N, K] (b_mn = 0), C [R, N] (stride ldc),
-// seg int32 [E+1] with 128-aligned entries and seg[E] <= R.  Rows >= seg[E] are not written.
+// seg int32 [E+1] with 128-aligned entries and seg[E] <= R.  b_mn bit 1: rows >= seg[E] are zeroed
+// (else they are not written).
 XB_API int xb_grouped_gemm_rows(const void* A, const void* B, void* C, const int* seg, int E,
                                 long long R, int N, int K, long long lda, long long ldc, int b_mn,
                                 void* stream) {
@@ -355,6 +382,8 @@ XB_API int xb_grouped_gemm_rows(const void* A, const void* B, void* C, const int
   if (E <= 0 || R <= 0) return 0;
   if (E > MAX_E || (R % BM) || (lda % 8) || (K % 8) || (N % 8) || (ldc % 8) ||
       (reinterpret_cast<uintptr_t>(C) % 16)) return -1;
+  const int zero_tail = (b_mn >> 1) & 1;
+  b_mn &= 1;
   CUtensorMap ta, tb, tc;
   if (xb_make_tmap_2d(&ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, R, K, lda, BM, BK,
                       CU_TENSOR_MAP_SWIZZLE_128B)) return -2;
@@ -370,7 +399,7 @@ XB_API int xb_grouped_gemm_rows(const void* A, const void* B, void* C, const int
   if (rc) return -3;
   Params p{};
   p.mode = 0; p.E = E; p.R = (int)R; p.M = (int)R; p.N = N; p.K = K; p.seg = seg; p.C = C; p.ldc = ldc;
-  p.out_fp32 = 0; p.accumulate = 0; p.b_mn = b_mn;
+  p.out_fp32 = 0; p.accumulate = 0; p.b_mn = b_mn; p.zero_tail = zero_tail; p.tma_out = 1;
   p.num_m_blocks = (int)(R / BM); p.num_n_blocks = (N + BN - 1) / BN;
   p.status = xb_status_ptr();
   return launch(ta, tb, tc, p, (cudaStream_t)stream);
@@ -388,10 +417,19 @@ XB_API int xb_grouped_gemm_wgrad(const void* A, const void* B, void* C, const in
                       CU_TENSOR_MAP_SWIZZLE_128B)) return -2;
   if (xb_make_tmap_2d(&tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, R, N, ldb, BK, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
+  // the output map has the experts as its outermost dimension: rows of a tile behind the last of an
+  // expert are clipped instead of landing in the next one
+  const bool tma_out = (reinterpret_cast<uintptr_t>(C) % 16) == 0 && (out_fp32 || !accumulate);
+  CUtensorMap tc = ta;
+  if (tma_out && xb_make_tmap_3d(&tc, C, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                                 out_fp32 ? 4 : 2, E, M, N, (uint64_t)M * N, N, 1, BM,
+                                 out_fp32 ? SLAB_COLS / 2 : SLAB_COLS, CU_TENSOR_MAP_SWIZZLE_128B))
+    return -4;
   Params p{};
+  p.tma_out = tma_out;
   p.mode = 1; p.E = E; p.R = (int)R; p.M = M; p.N = N; p.K = 0; p.seg = seg; p.C = C; p.ldc = N;
   p.out_fp32 = out_fp32; p.accumulate = accumulate; p.b_mn = 1;
   p.num_m_blocks = (M + BM - 1) / BM; p.num_n_blocks = (N + BN - 1) / BN;
   p.status = xb_status_ptr();
-  return launch(ta, tb, ta, p, (cudaStream_t)stream);   // no output tensor map in wgrad mode
+  return launch(ta, tb, tc, p, (cudaStream_t)stream);
 }

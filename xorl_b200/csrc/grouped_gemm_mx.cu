@@ -56,6 +56,7 @@ struct Params {
   __nv_bfloat16* C;
   long long ldc;
   int num_m_blocks, num_n_blocks;
+  int zero_tail;           // rows behind the last segment are zeroed
   int* status;
 };
 
@@ -85,11 +86,8 @@ __device__ __forceinline__ Tile get_tile(const Params& p, const int* sseg, int t
   const int mb = first_m + u % gsz, nb = u / gsz;
   r.m0 = mb * BM;
   r.n0 = nb * BN;
-  int e = -1;
-  for (int i = 0; i < p.E; ++i)
-    if (r.m0 >= sseg[i] && r.m0 < sseg[i + 1]) { e = i; break; }
-  r.e = e;
-  r.valid = e >= 0;
+  r.e = xb_expert_of_row(sseg, p.E, r.m0);
+  r.valid = r.e >= 0;
   return r;
 }
 
@@ -224,7 +222,14 @@ ggemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const Tile tl = get_tile(p, sseg, t);
-      if (!tl.valid) continue;
+      if (!tl.valid) {
+        if (p.zero_tail) {                                  // a warp writes 32 rows, one at a time
+          const int col = tl.n0 + lane * 8;
+          for (int i = 0; i < 32 && lane * 8 < BN && col < p.N; ++i)
+            *reinterpret_cast<uint4*>(p.C + (long long)(tl.m0 + q * 32 + i) * p.ldc + col) = make_uint4(0, 0, 0, 0);
+        }
+        continue;
+      }
       const int acc = tcount & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[acc], (tcount >> 1) & 1, abort_flag, p.status,
                                              XB_K_GROUPED_GEMM, 400 + acc))) { ok = false; break; }
@@ -436,10 +441,11 @@ quant_mx_weight_kernel(const __nv_bfloat16* __restrict__ w, uint8_t* __restrict_
 // A e4m3 [R, K] (row stride lda bytes), sfa UE8M0 [R, sfa_ld]; B e4m3 [E, N, K] contiguous, sfb UE8M0
 // [E, ceil(N/128), sfb_ld]; the scale row strides are multiples of 16 >= K/128 (arrays 16-byte aligned);
 // C bf16 [R, N] (row stride ldc elements); seg int32 [E+1] with 128-aligned entries and seg[E] <= R.
+// zero_tail: rows >= seg[E] are zeroed (else they are not written).
 // K a multiple of 128, N a multiple of 16.
 XB_API int xb_grouped_gemm_mx_rows(const void* A, const void* sfa, const void* B, const void* sfb, void* C,
                                    const int* seg, int E, long long R, int N, int K, long long lda,
-                                   long long ldc, int sfa_ld, int sfb_ld, void* stream) {
+                                   long long ldc, int sfa_ld, int sfb_ld, int zero_tail, void* stream) {
   using namespace xb_ggemm_mx;
   if (E <= 0 || R <= 0) return 0;
   if (E > MAX_E || (R % BM) || (lda % 16) || (K % BK) || (N % 16) || (sfa_ld % 16) || sfa_ld < K / BK ||
@@ -458,7 +464,7 @@ XB_API int xb_grouped_gemm_mx_rows(const void* A, const void* sfa, const void* B
   Params p{};
   p.E = E; p.R = (int)R; p.N = N; p.K = K; p.seg = seg;
   p.sfa = (const uint8_t*)sfa; p.sfb = (const uint8_t*)sfb; p.sfa_ld = sfa_ld; p.sfb_ld = sfb_ld;
-  p.C = (__nv_bfloat16*)C; p.ldc = ldc;
+  p.C = (__nv_bfloat16*)C; p.ldc = ldc; p.zero_tail = zero_tail;
   p.num_m_blocks = (int)(R / BM); p.num_n_blocks = (N + BN - 1) / BN;
   p.status = xb_status_ptr();
   static bool configured[64] = {false};

@@ -95,7 +95,7 @@ _SIGNATURES = {
     "xb_dequant_fp8_blocks": [P, L, P, L, P, L, I, I, P],
     "xb_grouped_gemm_rows": [P, P, P, P, I, L, I, I, L, L, I, P],
     "xb_grouped_gemm_wgrad": [P, P, P, P, I, L, I, I, L, L, I, I, P],
-    "xb_grouped_gemm_mx_rows": [P, P, P, P, P, P, I, L, I, I, L, L, I, I, P],
+    "xb_grouped_gemm_mx_rows": [P, P, P, P, P, P, I, L, I, I, L, L, I, I, I, P],
     "xb_quant_mx_rows": [P, L, P, L, P, I, L, I, P],
     "xb_quant_mx_weight": [P, P, P, I, P, P, I, I, I, I, P],
     "xb_attn_fwd_sink": [P, P, P, P, P, P, P, P, L, L, L, L, I, I, I, I, I, I, I, F, I, P],

@@ -167,16 +167,18 @@ def cached_quantized_experts(w: torch.Tensor) -> QuantizedExperts:
 
 def grouped_rows_mx(xq: torch.Tensor, sfx: torch.Tensor, wq: torch.Tensor, sfw: torch.Tensor,
                     seg: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out[rows of e] = dequant(xq)[rows of e] @ dequant(wq[e])^T with wq [E, N, K] (K contiguous)."""
+    """out[rows of e] = dequant(xq)[rows of e] @ dequant(wq[e])^T with wq [E, N, K] (K contiguous).  Without
+    ``out`` a new tensor is returned, whose rows behind the last segment are zero."""
     global _launches
     R, K = xq.shape
     E, N, K2 = wq.shape
     assert K == K2
-    if out is None:
-        out = torch.zeros((R, N), device=xq.device, dtype=torch.bfloat16)
+    own = out is None
+    if own:
+        out = torch.empty((R, N), device=xq.device, dtype=torch.bfloat16)
     _lib.check(_lib.cuda_lib().xb_grouped_gemm_mx_rows(
         xq.data_ptr(), sfx.data_ptr(), wq.data_ptr(), sfw.data_ptr(), out.data_ptr(), seg.data_ptr(), E, R, N, K,
-        xq.stride(0), out.stride(0), sfx.stride(0), sfw.stride(1), _lib.stream_ptr()), "xb_grouped_gemm_mx_rows")
+        xq.stride(0), out.stride(0), sfx.stride(0), sfw.stride(1), int(own), _lib.stream_ptr()), "xb_grouped_gemm_mx_rows")
     _launches += 1
     return out
 
@@ -206,8 +208,8 @@ class _GroupedLinearFP8(torch.autograd.Function):
                 dq, sfd = quantize_rows(dy)
                 dx = grouped_rows_mx(dq, sfd, qe.q_kn, qe.sf_kn, seg)      # dy @ w[e]^T
             else:
-                dx = torch.zeros_like(x)
-                _grouped_rows_cuda(dy, w, seg, dx, b_kmajor=True)
+                dx = torch.empty_like(x)
+                _grouped_rows_cuda(dy, w, seg, dx, b_kmajor=True, zero_tail=True)
         dw = None
         if ctx.needs_input_grad[1]:
             tgt, fresh = grad_target(w)

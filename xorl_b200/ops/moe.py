@@ -317,8 +317,9 @@ def buffer_rows(num_slots: int, num_experts: int, align: int = SEG_ALIGN) -> int
 # --------------------------------------------------------------------------------------------
 # grouped GEMM
 # --------------------------------------------------------------------------------------------
-def _grouped_rows_cuda(a, b, seg, out, b_kmajor: bool):
-    """out[rows of e] = a[rows of e] @ op(b[e]); b [E, K, N] (b_kmajor False) or [E, N, K]."""
+def _grouped_rows_cuda(a, b, seg, out, b_kmajor: bool, zero_tail: bool = False):
+    """out[rows of e] = a[rows of e] @ op(b[e]); b [E, K, N] (b_kmajor False) or [E, N, K].
+    ``zero_tail``: the kernel zeroes the rows of ``out`` behind the last segment."""
     global _launches
     E = b.shape[0]
     if b_kmajor:
@@ -327,7 +328,7 @@ def _grouped_rows_cuda(a, b, seg, out, b_kmajor: bool):
         K, N = b.shape[1], b.shape[2]
     rc = _lib.cuda_lib().xb_grouped_gemm_rows(a.data_ptr(), b.data_ptr(), out.data_ptr(),
                                               seg.data_ptr(), E, a.shape[0], N, K, a.stride(0),
-                                              out.stride(0), int(not b_kmajor), _lib.stream_ptr())
+                                              out.stride(0), int(not b_kmajor) | (2 if zero_tail else 0), _lib.stream_ptr())
     _lib.check(rc, "xb_grouped_gemm_rows")
     _launches += 1
     return out
@@ -365,8 +366,8 @@ class _GroupedLinear(torch.autograd.Function):
     def forward(ctx, x, w, seg):
         ctx.save_for_backward(x, seg)
         ctx.w = w
-        out = torch.zeros((x.shape[0], w.shape[2]), device=x.device, dtype=x.dtype)
-        return _grouped_rows_cuda(x, w, seg, out, b_kmajor=False)
+        out = torch.empty((x.shape[0], w.shape[2]), device=x.device, dtype=x.dtype)
+        return _grouped_rows_cuda(x, w, seg, out, b_kmajor=False, zero_tail=True)
 
     @staticmethod
     def backward(ctx, dy):
@@ -375,8 +376,8 @@ class _GroupedLinear(torch.autograd.Function):
         dy = dy.contiguous()
         dx = None
         if ctx.needs_input_grad[0]:
-            dx = torch.zeros_like(x)
-            _grouped_rows_cuda(dy, w, seg, dx, b_kmajor=True)   # dx = dy @ w[e]^T
+            dx = torch.empty_like(x)
+            _grouped_rows_cuda(dy, w, seg, dx, b_kmajor=True, zero_tail=True)   # dx = dy @ w[e]^T
         dw = None
         if ctx.needs_input_grad[1]:
             tgt, fresh = grad_target(w)

@@ -337,7 +337,7 @@ def _rows_gemm(ws, sc, a, a_cols, w, out, n_out, b_mn: int, fp8, qe_w, qe_sf, st
                    "xb_quant_mx_rows_lim")
         _lib.check(lib.xb_grouped_gemm_mx_rows(sc.q.data_ptr(), sc.sf.data_ptr(), qe_w.data_ptr(), qe_sf.data_ptr(),
                                                out.data_ptr(), sc.seg.data_ptr(), ws.El, ws.cap, n_out, a_cols,
-                                               sc.q.stride(0), out.stride(0), sc.sf.stride(0), qe_sf.stride(1), st),
+                                               sc.q.stride(0), out.stride(0), sc.sf.stride(0), qe_sf.stride(1), 0, st),
                    "xb_grouped_gemm_mx_rows")
     else:
         _lib.check(lib.xb_grouped_gemm_rows(a.data_ptr(), w.data_ptr(), out.data_ptr(), sc.seg.data_ptr(), ws.El,
@@ -414,7 +414,7 @@ class _FusedEPMoE(torch.autograd.Function):
         if pre_q:
             _lib.check(lib.xb_grouped_gemm_mx_rows(recv.data_ptr(), recv.data_ptr() + H, qg.q_nk.data_ptr(),
                                                    qg.sf_nk.data_ptr(), sc.h.data_ptr(), sc.seg.data_ptr(), ws.El, ws.cap,
-                                                   I2, H, rb, sc.h.stride(0), rb, qg.sf_nk.stride(1), st),
+                                                   I2, H, rb, sc.h.stride(0), rb, qg.sf_nk.stride(1), 0, st),
                        "xb_grouped_gemm_mx_rows")
         else:
             _rows_gemm(ws, sc, recv, H, gate_up, sc.h, I2, 1, fp8, None if qg is None else qg.q_nk,
