@@ -97,70 +97,106 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
+// Sum over the block with one barrier: every warp leaves its sum in ``red`` and every thread adds the
+// eight of them in the same order.  Callers alternate between two arrays, so the next call's writes
+// cannot meet this call's reads.
+__device__ __forceinline__ float block_sum_once(float v, float* red) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.f;
+#pragma unroll
+  for (int i = 0; i < NORM_THREADS / 32; ++i) t += red[i];
+  return t;
+}
+
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres) ; dw partial[blockIdx][H] += dy * xhat
+//
+// Bound by memory: dy, x and dres in, dx out.  A CTA walks its rows and needs the whole row's sum before
+// it can write, so a row at a time leaves the memory idle for three latencies per row (loads, sum, dres).
+// For rows up to 4096 wide the next row's three vectors are therefore loaded before this row's sum is
+// taken: 2 CTAs x 256 threads x 96 bytes are then in flight per SM all the time.  Wider rows have no
+// registers left for that.
 template <int NV>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, int T, int H, int zero_centered) {
-  __shared__ float red[32];
+  constexpr bool AHEAD = NV <= 2;
+  __shared__ float red[2][NORM_THREADS / 32];
   const int nvec = H >> 3;
   float dwacc[NV][8];
+  uint4 wv[NV], dyn[NV], xn[NV], rn[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * NORM_THREADS;
+    wv[i] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : make_uint4(0, 0, 0, 0);
+    dyn[i] = xn[i] = rn[i] = make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    const float rstd = rstd_in[row];
-    float g[NV][8];   // dy * w
-    float xh[NV][8];  // x * rstd
-    float dot = 0.f;
+  }
+  float rstd_n = 0.f;
+  auto load = [&](int row) {
+    rstd_n = rstd_in[row];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * NORM_THREADS;
       if (v < nvec) {
-        uint4 a = reinterpret_cast<const uint4*>(dy + (size_t)row * H)[v];
-        uint4 b = reinterpret_cast<const uint4*>(x + (size_t)row * H)[v];
-        uint4 c = reinterpret_cast<const uint4*>(w)[v];
-        const uint32_t au[4] = {a.x, a.y, a.z, a.w};
-        const uint32_t bu[4] = {b.x, b.y, b.z, b.w};
-        const uint32_t cu[4] = {c.x, c.y, c.z, c.w};
+        dyn[i] = reinterpret_cast<const uint4*>(dy + (size_t)row * H)[v];
+        xn[i] = reinterpret_cast<const uint4*>(x + (size_t)row * H)[v];
+        if (dres) rn[i] = reinterpret_cast<const uint4*>(dres + (size_t)row * H)[v];
+      }
+    }
+  };
+  int buf = 0;
+  if (AHEAD && blockIdx.x < T) load(blockIdx.x);
+  for (int row = blockIdx.x; row < T; row += gridDim.x, buf ^= 1) {
+    if (!AHEAD) load(row);
+    const float rstd = rstd_n;
+    uint4 a[NV], b[NV], r[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) { a[i] = dyn[i]; b[i] = xn[i]; r[i] = rn[i]; }
+    if (AHEAD && row + (int)gridDim.x < T) load(row + gridDim.x);
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const uint32_t au[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+      const uint32_t bu[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+      const uint32_t cu[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 d = unpack_bf16x2(au[j]);
+        const float2 xx = unpack_bf16x2(bu[j]);
+        float2 ww = unpack_bf16x2(cu[j]);
+        if (zero_centered) { ww.x += 1.f; ww.y += 1.f; }
+        const float x0 = xx.x * rstd, x1 = xx.y * rstd;
+        dwacc[i][2 * j] += d.x * x0;
+        dwacc[i][2 * j + 1] += d.y * x1;
+        dot += d.x * ww.x * x0 + d.y * ww.y * x1;
+      }
+    }
+    const float mean = block_sum_once(dot, red[buf]) / (float)H;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * NORM_THREADS;
+      if (v < nvec) {
+        const uint32_t au[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+        const uint32_t bu[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+        const uint32_t cu[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+        const uint32_t ru[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+        uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 d = unpack_bf16x2(au[j]);
           const float2 xx = unpack_bf16x2(bu[j]);
           float2 ww = unpack_bf16x2(cu[j]);
           if (zero_centered) { ww.x += 1.f; ww.y += 1.f; }
-          xh[i][2 * j] = xx.x * rstd;
-          xh[i][2 * j + 1] = xx.y * rstd;
-          g[i][2 * j] = d.x * ww.x;
-          g[i][2 * j + 1] = d.y * ww.y;
-          dwacc[i][2 * j] += d.x * xh[i][2 * j];
-          dwacc[i][2 * j + 1] += d.y * xh[i][2 * j + 1];
-          dot += g[i][2 * j] * xh[i][2 * j] + g[i][2 * j + 1] * xh[i][2 * j + 1];
-        }
-      }
-    }
-    const float mean = block_sum(dot, red) / (float)H;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = threadIdx.x + i * NORM_THREADS;
-      if (v < nvec) {
-        uint32_t ru[4] = {0, 0, 0, 0};
-        if (dres) {
-          uint4 r = reinterpret_cast<const uint4*>(dres + (size_t)row * H)[v];
-          ru[0] = r.x; ru[1] = r.y; ru[2] = r.z; ru[3] = r.w;
-        }
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float a0 = rstd * (g[i][2 * j] - xh[i][2 * j] * mean);
-          float a1 = rstd * (g[i][2 * j + 1] - xh[i][2 * j + 1] * mean);
+          float a0 = rstd * (d.x * ww.x - xx.x * rstd * mean);
+          float a1 = rstd * (d.y * ww.y - xx.y * rstd * mean);
           if (dres) {
-            const float2 r = unpack_bf16x2(ru[j]);
-            a0 += r.x; a1 += r.y;
+            const float2 rr = unpack_bf16x2(ru[j]);
+            a0 += rr.x; a1 += rr.y;
           }
           o[j] = pack_bf16x2(a0, a1);
         }
@@ -180,17 +216,33 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// out[h] (+)= sum_p partial[p][h], fixed summation order.
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, int P, int H,
-                                       __nv_bfloat16* __restrict__ out_bf16,
-                                       float* __restrict__ out_f32, int accumulate) {
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= H) return;
+// out[h] (+)= sum_p partial[p][h], fixed summation order.  A block owns 32 columns and splits the
+// partial rows over 16 warps: one thread per column reads several hundred rows one after the other,
+// which takes longer than the kernel that made them.  Columns from ``split`` on go to out2_bf16 (two
+// weights reduced in one launch).
+constexpr int REDUCE_ROWS = 16;
+__global__ void __launch_bounds__(32 * REDUCE_ROWS)
+reduce_partials_kernel(const float* __restrict__ partial, int P, int H, __nv_bfloat16* __restrict__ out_bf16,
+                       float* __restrict__ out_f32, int accumulate, __nv_bfloat16* __restrict__ out2_bf16,
+                       int split) {
+  __shared__ float sh[REDUCE_ROWS][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int h = blockIdx.x * 32 + tx;
   float s = 0.f;
-  for (int p = 0; p < P; ++p) s += partial[(size_t)p * H + h];
+  if (h < H) {
+#pragma unroll 4
+    for (int p = ty; p < P; p += REDUCE_ROWS) s += partial[(size_t)p * H + h];
+  }
+  sh[ty][tx] = s;
+  __syncthreads();
+  if (ty != 0 || h >= H) return;
+  s = 0.f;
+#pragma unroll
+  for (int i = 0; i < REDUCE_ROWS; ++i) s += sh[i][tx];
   if (out_f32) out_f32[h] = accumulate ? out_f32[h] + s : s;
-  if (out_bf16)
-    out_bf16[h] = __float2bfloat16(accumulate ? __bfloat162float(out_bf16[h]) + s : s);
+  __nv_bfloat16* o = h < split ? out_bf16 : out2_bf16;
+  const int c = h < split ? h : h - split;
+  if (o) o[c] = __float2bfloat16(accumulate ? __bfloat162float(o[c]) + s : s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -299,8 +351,12 @@ qk_norm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, long long ld_in,
 }
 
 // Backward of the above.  dout: [T, (Hq+Hkv)*D] (bf16, or fp32 when dout_f32 != nullptr, which is
-// how the attention backward hands over its atomically accumulated dq).  Writes the q and k
-// slices of dqkv and accumulates dw partials [gridDim.x][2][D].
+// how the attention backward hands over dq and dk).  Writes the q and k slices of dqkv and
+// accumulates dw partials [gridDim.x][2][D].
+//
+// Bound by memory (12 bytes per element with fp32 gradients).  As in the forward, a warp takes QKR_HPW
+// heads of one token: their loads are all issued before the first is used, and the token's cos / sin
+// are read once.
 template <int D>
 __global__ void __launch_bounds__(256)
 qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout_bf16,
@@ -314,72 +370,117 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout_bf16,
   constexpr int HALF = D / 2;
   constexpr int PER = HALF / 32;
   const int heads = Hq + Hkv;
+  const int groups = (heads + QKR_HPW - 1) / QKR_HPW;
   const int lane = threadIdx.x & 31;
   const int warps_per_block = blockDim.x >> 5;
   float dwq_a[PER], dwq_b[PER], dwk_a[PER], dwk_b[PER];
+  float wqv[2][PER], wkv[2][PER];
 #pragma unroll
-  for (int i = 0; i < PER; ++i) dwq_a[i] = dwq_b[i] = dwk_a[i] = dwk_b[i] = 0.f;
+  for (int i = 0; i < PER; ++i) {
+    dwq_a[i] = dwq_b[i] = dwk_a[i] = dwk_b[i] = 0.f;
+    const int e = lane * PER + i;
+    wqv[0][i] = do_norm ? __bfloat162float(wq[e]) : 1.f;
+    wqv[1][i] = do_norm ? __bfloat162float(wq[HALF + e]) : 1.f;
+    wkv[0][i] = do_norm ? __bfloat162float(wk[e]) : 1.f;
+    wkv[1][i] = do_norm ? __bfloat162float(wk[HALF + e]) : 1.f;
+  }
 
-  const long long total = (long long)T * heads;
+  const long long total = (long long)T * groups;
   for (long long wid = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); wid < total;
        wid += (long long)gridDim.x * warps_per_block) {
-    const int t = (int)(wid / heads);
-    const int h = (int)(wid % heads);
-    float g1[PER], g2[PER];
+    const int t = (int)(wid / groups);
+    const int h0 = (int)(wid - (long long)t * groups) * QKR_HPW;
+    float d1[QKR_HPW][PER], d2[QKR_HPW][PER], x1[QKR_HPW][PER], x2[QKR_HPW][PER], rs[QKR_HPW];
+#pragma unroll
+    for (int g = 0; g < QKR_HPW; ++g) {
+      const int h = h0 + g;
+      rs[g] = 0.f;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) d1[g][i] = d2[g][i] = x1[g][i] = x2[g][i] = 0.f;
+      if (h < heads) {                                    // warp-uniform
+        if (dout_f32_q != nullptr) {
+          const float* s = (h < Hq) ? dout_f32_q + ((size_t)t * Hq + h) * D
+                                    : dout_f32_k + ((size_t)t * Hkv + (h - Hq)) * D;
+#pragma unroll
+          for (int i = 0; i < PER; ++i) {
+            d1[g][i] = s[lane * PER + i];
+            d2[g][i] = s[HALF + lane * PER + i];
+          }
+        } else {
+          const __nv_bfloat16* s = dout_bf16 + (size_t)t * ld_dout + (size_t)h * D;
+#pragma unroll
+          for (int i = 0; i < PER; ++i) {
+            d1[g][i] = __bfloat162float(s[lane * PER + i]);
+            d2[g][i] = __bfloat162float(s[HALF + lane * PER + i]);
+          }
+        }
+        if (do_norm) {
+          const __nv_bfloat16* src = qkv + (size_t)t * ld_in + (size_t)h * D;
+#pragma unroll
+          for (int i = 0; i < PER; ++i) {
+            x1[g][i] = __bfloat162float(src[lane * PER + i]);
+            x2[g][i] = __bfloat162float(src[HALF + lane * PER + i]);
+          }
+          rs[g] = rstd_in[(size_t)t * heads + h];
+        }
+      }
+    }
+    float c[PER], sn[PER];
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-      const int e = lane * PER + i;
-      float d1, d2;
-      if (dout_f32_q != nullptr) {
-        const float* s = (h < Hq) ? dout_f32_q + ((size_t)t * Hq + h) * D
-                                  : dout_f32_k + ((size_t)t * Hkv + (h - Hq)) * D;
-        d1 = s[e];
-        d2 = s[HALF + e];
-      } else {
-        const __nv_bfloat16* s = dout_bf16 + (size_t)t * ld_dout + (size_t)h * D;
-        d1 = __bfloat162float(s[e]);
-        d2 = __bfloat162float(s[HALF + e]);
-      }
-      const float c = cosb[(size_t)t * HALF + e], sn = sinb[(size_t)t * HALF + e];
-      // transpose of the rotation
-      g1[i] = d1 * c + d2 * sn;
-      g2[i] = d2 * c - d1 * sn;
+      c[i] = __ldg(cosb + (size_t)t * HALF + lane * PER + i);
+      sn[i] = __ldg(sinb + (size_t)t * HALF + lane * PER + i);
     }
-    __nv_bfloat16* dst = dqkv + (size_t)t * ld_dqkv + (size_t)h * D;
-    if (!do_norm) {
+#pragma unroll
+    for (int g = 0; g < QKR_HPW; ++g) {
+      const int h = h0 + g;
+      if (h >= heads) break;                              // warp-uniform
+      const bool is_q = h < Hq;
+      float o1[PER], o2[PER];
+      float gw1[PER], gw2[PER];
+      float dot = 0.f;
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        dst[lane * PER + i] = __float2bfloat16(g1[i]);
-        dst[HALF + lane * PER + i] = __float2bfloat16(g2[i]);
+        // transpose of the rotation
+        o1[i] = d1[g][i] * c[i] + d2[g][i] * sn[i];
+        o2[i] = d2[g][i] * c[i] - d1[g][i] * sn[i];
+        if (do_norm) {
+          x1[g][i] *= rs[g];
+          x2[g][i] *= rs[g];
+          gw1[i] = o1[i] * (is_q ? wqv[0][i] : wkv[0][i]);
+          gw2[i] = o2[i] * (is_q ? wqv[1][i] : wkv[1][i]);
+          dot += gw1[i] * x1[g][i] + gw2[i] * x2[g][i];
+          if (is_q) {
+            dwq_a[i] += o1[i] * x1[g][i];
+            dwq_b[i] += o2[i] * x2[g][i];
+          } else {
+            dwk_a[i] += o1[i] * x1[g][i];
+            dwk_b[i] += o2[i] * x2[g][i];
+          }
+        }
       }
-      continue;
-    }
-    const __nv_bfloat16* src = qkv + (size_t)t * ld_in + (size_t)h * D;
-    const __nv_bfloat16* w = (h < Hq) ? wq : wk;
-    const float rstd = rstd_in[(size_t)t * heads + h];
-    float xh1[PER], xh2[PER], gw1[PER], gw2[PER];
-    float dot = 0.f;
+      if (do_norm) {
+        const float mean = warp_sum(dot) / (float)D;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int e = lane * PER + i;
-      xh1[i] = __bfloat162float(src[e]) * rstd;
-      xh2[i] = __bfloat162float(src[HALF + e]) * rstd;
-      gw1[i] = g1[i] * __bfloat162float(w[e]);
-      gw2[i] = g2[i] * __bfloat162float(w[HALF + e]);
-      dot += gw1[i] * xh1[i] + gw2[i] * xh2[i];
-      if (h < Hq) {
-        dwq_a[i] += g1[i] * xh1[i];
-        dwq_b[i] += g2[i] * xh2[i];
+        for (int i = 0; i < PER; ++i) {
+          o1[i] = rs[g] * (gw1[i] - x1[g][i] * mean);
+          o2[i] = rs[g] * (gw2[i] - x2[g][i] * mean);
+        }
+      }
+      __nv_bfloat16* dst = dqkv + (size_t)t * ld_dqkv + (size_t)h * D;
+      if constexpr (PER % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < PER; i += 2) {
+          *reinterpret_cast<__nv_bfloat162*>(dst + lane * PER + i) = __floats2bfloat162_rn(o1[i], o1[i + 1]);
+          *reinterpret_cast<__nv_bfloat162*>(dst + HALF + lane * PER + i) = __floats2bfloat162_rn(o2[i], o2[i + 1]);
+        }
       } else {
-        dwk_a[i] += g1[i] * xh1[i];
-        dwk_b[i] += g2[i] * xh2[i];
-      }
-    }
-    const float mean = warp_sum(dot) / (float)D;
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      dst[lane * PER + i] = __float2bfloat16(rstd * (gw1[i] - xh1[i] * mean));
-      dst[HALF + lane * PER + i] = __float2bfloat16(rstd * (gw2[i] - xh2[i] * mean));
+        for (int i = 0; i < PER; ++i) {
+          dst[lane * PER + i] = __float2bfloat16(o1[i]);
+          dst[HALF + lane * PER + i] = __float2bfloat16(o2[i]);
+        }
+      }
     }
   }
   if (!do_norm || dw_partial == nullptr) return;
@@ -437,13 +538,13 @@ XB_API int xb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const fl
 #define XB_ARGS (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, \
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, partial, T, H, zero_centered
   const int nv = (H / 8 + NORM_THREADS - 1) / NORM_THREADS;
-  if (nv <= 2) rmsnorm_bwd_kernel<2><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
+  if (nv <= 1) rmsnorm_bwd_kernel<1><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
+  else if (nv <= 2) rmsnorm_bwd_kernel<2><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
   else if (nv <= 4) rmsnorm_bwd_kernel<4><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
   else rmsnorm_bwd_kernel<8><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
 #undef XB_ARGS
-  reduce_partials_kernel<<<(H + 255) / 256, 256, 0, st>>>(partial, rows, H,
-                                                          (__nv_bfloat16*)dw_bf16, dw_f32,
-                                                          accumulate);
+  reduce_partials_kernel<<<(H + 31) / 32, 32 * REDUCE_ROWS, 0, st>>>(partial, rows, H, (__nv_bfloat16*)dw_bf16, dw_f32,
+                                                                     accumulate, nullptr, H);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -491,14 +592,9 @@ XB_API int xb_qk_norm_rope_bwd(const void* dout_bf16, const float* dq_f32, const
   else return -1;
 #undef XB_LAUNCH
   if (do_norm && partial) {
-    // partial rows are [2][D]: reduce q weights then k weights
-    reduce_partials_kernel<<<(2 * D + 255) / 256, 256, 0, st>>>(partial, grid, 2 * D, nullptr,
-                                                                partial, 0);
-    // partial[0 .. 2D) now holds the totals; add them into the bf16 weight grads
-    reduce_partials_kernel<<<1, 256, 0, st>>>(partial, 1, D, (__nv_bfloat16*)dwq, nullptr,
-                                              accumulate);
-    reduce_partials_kernel<<<1, 256, 0, st>>>(partial + D, 1, D, (__nv_bfloat16*)dwk, nullptr,
-                                              accumulate);
+    // partial rows are [2][D]: q weights, then k weights
+    reduce_partials_kernel<<<(2 * D + 31) / 32, 32 * REDUCE_ROWS, 0, st>>>(
+        partial, grid, 2 * D, (__nv_bfloat16*)dwq, nullptr, accumulate, (__nv_bfloat16*)dwk, D);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -570,12 +666,12 @@ XB_API int xb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* w, 
 #define XB_ARGS (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, \
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, partial, T, H, zero_centered
   const int nv = (H / 8 + NORM_THREADS - 1) / NORM_THREADS;
-  if (nv <= 2) rmsnorm_bwd_kernel<2><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
+  if (nv <= 1) rmsnorm_bwd_kernel<1><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
+  else if (nv <= 2) rmsnorm_bwd_kernel<2><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
   else rmsnorm_bwd_kernel<4><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
 #undef XB_ARGS
   // every one of the `rows` partial rows was just written by the kernel above
-  reduce_partials_kernel<<<(H + 255) / 256, 256, 0, st>>>(partial, rows, H,
-                                                          (__nv_bfloat16*)dw_bf16, dw_f32,
-                                                          accumulate);
+  reduce_partials_kernel<<<(H + 31) / 32, 32 * REDUCE_ROWS, 0, st>>>(partial, rows, H, (__nv_bfloat16*)dw_bf16, dw_f32,
+                                                                     accumulate, nullptr, H);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
