@@ -11,95 +11,60 @@ __device__ __forceinline__ float round_bf16(float x) {
   return __bfloat162float(__float2bfloat16(x));
 }
 
-// Both SwiGLU kernels are bound by memory.  A thread loads two vectors of every operand before it uses
-// the first, and row and column come from a 32-bit division wherever the element count allows: the
-// 64-bit one costs more instructions than the activation.
-constexpr int SWIGLU_UNROLL = 2;
-
-__device__ __forceinline__ uint4 swiglu_vec(const uint4 g, const uint4 u, int two_round) {
-  const uint32_t gg[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w};
-  uint32_t o[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 a = unpack_bf16x2(gg[j]), b = unpack_bf16x2(uu[j]);
-    float s0 = silu_f(a.x), s1 = silu_f(a.y);
-    if (two_round) { s0 = round_bf16(s0); s1 = round_bf16(s1); }
-    o[j] = pack_bf16x2(s0 * b.x, s1 * b.y);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
-}
-
-// gu: [T, 2I] (gate = [:, :I], up = [:, I:]) -> out [T, I].  Index: unsigned or unsigned long long.
-template <typename Index>
+// gu: [T, 2I] (gate = [:, :I], up = [:, I:]) -> out [T, I]
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                   long long T, int I, int two_round, const int* __restrict__ row_limit) {
-  const Index vec_per_row = I >> 3;
+  const int vec_per_row = I >> 3;
   // row_limit (optional, device memory): only the first *row_limit rows hold data
   if (row_limit != nullptr) T = min(T, (long long)*row_limit);
-  const Index total = (Index)T * vec_per_row, stride = (Index)gridDim.x * 256;
-  const uint4* in = reinterpret_cast<const uint4*>(gu);
-  uint4* o = reinterpret_cast<uint4*>(out);
-  for (Index i0 = (Index)blockIdx.x * 256 + threadIdx.x; i0 < total; i0 += SWIGLU_UNROLL * stride) {
-    uint4 g[SWIGLU_UNROLL], u[SWIGLU_UNROLL];
+  const long long total = T * vec_per_row;
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const long long t = idx / vec_per_row;
+    const int v = (int)(idx % vec_per_row);
+    const uint4 g = reinterpret_cast<const uint4*>(gu + t * 2 * I)[v];
+    const uint4 u = reinterpret_cast<const uint4*>(gu + t * 2 * I + I)[v];
+    const uint32_t gg[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w};
+    uint32_t o[4];
 #pragma unroll
-    for (int k = 0; k < SWIGLU_UNROLL; ++k) {
-      const Index i = i0 + k * stride;
-      if (i < total) {
-        const size_t at = (size_t)i + (size_t)(i / vec_per_row) * vec_per_row;   // 2 * row * vecs + column
-        g[k] = in[at];
-        u[k] = in[at + vec_per_row];
-      }
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = unpack_bf16x2(gg[j]), b = unpack_bf16x2(uu[j]);
+      float s0 = silu_f(a.x), s1 = silu_f(a.y);
+      if (two_round) { s0 = round_bf16(s0); s1 = round_bf16(s1); }
+      o[j] = pack_bf16x2(s0 * b.x, s1 * b.y);
     }
-#pragma unroll
-    for (int k = 0; k < SWIGLU_UNROLL; ++k) {
-      const Index i = i0 + k * stride;
-      if (i < total) o[i] = swiglu_vec(g[k], u[k], two_round);
-    }
+    reinterpret_cast<uint4*>(out + t * I)[v] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
 // dgu[:, :I] = dout * up * dsilu(gate);  dgu[:, I:] = dout * silu(gate)
-template <typename Index>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ gu,
                   __nv_bfloat16* __restrict__ dgu, long long T, int I, const int* __restrict__ row_limit) {
-  const Index vec_per_row = I >> 3;
+  const int vec_per_row = I >> 3;
   if (row_limit != nullptr) T = min(T, (long long)*row_limit);
-  const Index total = (Index)T * vec_per_row, stride = (Index)gridDim.x * 256;
-  const uint4* in = reinterpret_cast<const uint4*>(gu);
-  const uint4* din = reinterpret_cast<const uint4*>(dout);
-  uint4* o = reinterpret_cast<uint4*>(dgu);
-  for (Index i0 = (Index)blockIdx.x * 256 + threadIdx.x; i0 < total; i0 += SWIGLU_UNROLL * stride) {
-    uint4 g[SWIGLU_UNROLL], u[SWIGLU_UNROLL], d[SWIGLU_UNROLL];
-    size_t at[SWIGLU_UNROLL];
+  const long long total = T * vec_per_row;
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const long long t = idx / vec_per_row;
+    const int v = (int)(idx % vec_per_row);
+    const uint4 g = reinterpret_cast<const uint4*>(gu + t * 2 * I)[v];
+    const uint4 u = reinterpret_cast<const uint4*>(gu + t * 2 * I + I)[v];
+    const uint4 d = reinterpret_cast<const uint4*>(dout + t * I)[v];
+    const uint32_t gg[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w},
+                   dd[4] = {d.x, d.y, d.z, d.w};
+    uint32_t og[4], ou[4];
 #pragma unroll
-    for (int k = 0; k < SWIGLU_UNROLL; ++k) {
-      const Index i = i0 + k * stride;
-      if (i < total) {
-        at[k] = (size_t)i + (size_t)(i / vec_per_row) * vec_per_row;
-        g[k] = in[at[k]];
-        u[k] = in[at[k] + vec_per_row];
-        d[k] = din[i];
-      }
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = unpack_bf16x2(gg[j]), b = unpack_bf16x2(uu[j]), c = unpack_bf16x2(dd[j]);
+      const float sg0 = sigmoid_f(a.x), sg1 = sigmoid_f(a.y);
+      const float ds0 = sg0 * (1.f + a.x * (1.f - sg0)), ds1 = sg1 * (1.f + a.y * (1.f - sg1));
+      og[j] = pack_bf16x2(c.x * b.x * ds0, c.y * b.y * ds1);
+      ou[j] = pack_bf16x2(c.x * a.x * sg0, c.y * a.y * sg1);
     }
-#pragma unroll
-    for (int k = 0; k < SWIGLU_UNROLL; ++k) {
-      if (i0 + k * stride >= total) break;
-      const uint32_t gg[4] = {g[k].x, g[k].y, g[k].z, g[k].w}, uu[4] = {u[k].x, u[k].y, u[k].z, u[k].w},
-                     dd[4] = {d[k].x, d[k].y, d[k].z, d[k].w};
-      uint32_t og[4], ou[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 a = unpack_bf16x2(gg[j]), b = unpack_bf16x2(uu[j]), c = unpack_bf16x2(dd[j]);
-        const float sg0 = sigmoid_f(a.x), sg1 = sigmoid_f(a.y);
-        const float ds0 = sg0 * (1.f + a.x * (1.f - sg0)), ds1 = sg1 * (1.f + a.y * (1.f - sg1));
-        og[j] = pack_bf16x2(c.x * b.x * ds0, c.y * b.y * ds1);
-        ou[j] = pack_bf16x2(c.x * a.x * sg0, c.y * a.y * sg1);
-      }
-      o[at[k]] = make_uint4(og[0], og[1], og[2], og[3]);
-      o[at[k] + vec_per_row] = make_uint4(ou[0], ou[1], ou[2], ou[3]);
-    }
+    reinterpret_cast<uint4*>(dgu + t * 2 * I)[v] = make_uint4(og[0], og[1], og[2], og[3]);
+    reinterpret_cast<uint4*>(dgu + t * 2 * I + I)[v] = make_uint4(ou[0], ou[1], ou[2], ou[3]);
   }
 }
 
@@ -176,66 +141,42 @@ static inline int grid_for(long long work_items, int threads) {
   return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-// An index counts vectors of eight of one operand.  No cap on the grid: a block that is done makes room for
-// the next, where a fixed number of blocks walking the rows leaves its last pass partly filled.
-static int swiglu_grid(long long items) {
-  const long long g = (items + 256 * SWIGLU_UNROLL - 1) / (256 * SWIGLU_UNROLL);
-  return (int)(g < (1 << 24) ? g : (1 << 24));
-}
-
-static int swiglu_fwd(const void* gu, void* out, long long T, int I, int two_round, const int* row_limit,
-                      void* stream) {
-  if (I % 8) return -1;
-  if (T <= 0) return 0;
-  const long long items = T * (I / 8);
-  const int grid = swiglu_grid(items);
-  cudaStream_t st = (cudaStream_t)stream;
-  // the last index that is formed lies up to SWIGLU_UNROLL strides behind the last item
-  if (items < (1ll << 31))
-    swiglu_fwd_kernel<unsigned><<<grid, 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I, two_round,
-                                                      row_limit);
-  else
-    swiglu_fwd_kernel<unsigned long long><<<grid, 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I,
-                                                                two_round, row_limit);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
-
-static int swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int I, const int* row_limit,
-                      void* stream) {
-  if (I % 8) return -1;
-  if (T <= 0) return 0;
-  const long long items = T * (I / 8);
-  const int grid = swiglu_grid(items);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (items < (1ll << 31))
-    swiglu_bwd_kernel<unsigned><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu,
-                                                      (__nv_bfloat16*)dgu, T, I, row_limit);
-  else
-    swiglu_bwd_kernel<unsigned long long><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu,
-                                                                (__nv_bfloat16*)dgu, T, I, row_limit);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
-
 XB_API int xb_swiglu_fwd(const void* gu, void* out, long long T, int I, int two_round,
                          void* stream) {
-  return swiglu_fwd(gu, out, T, I, two_round, nullptr, stream);
+  if (I % 8) return -1;
+  if (T <= 0) return 0;
+  swiglu_fwd_kernel<<<grid_for(T * (I / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I, two_round, nullptr);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 // Variants for buffers sized for the worst case: only the first *row_limit rows (an int in device
 // memory, e.g. the end of the last expert segment) are processed; the grid is sized for T rows.
 XB_API int xb_swiglu_fwd_rows(const void* gu, void* out, long long T, int I, int two_round, const int* row_limit,
                               void* stream) {
-  return swiglu_fwd(gu, out, T, I, two_round, row_limit, stream);
+  if (I % 8) return -1;
+  if (T <= 0) return 0;
+  swiglu_fwd_kernel<<<grid_for(T * (I / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I, two_round, row_limit);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 XB_API int xb_swiglu_bwd_rows(const void* dout, const void* gu, void* dgu, long long T, int I, const int* row_limit,
                               void* stream) {
-  return swiglu_bwd(dout, gu, dgu, T, I, row_limit, stream);
+  if (I % 8) return -1;
+  if (T <= 0) return 0;
+  swiglu_bwd_kernel<<<grid_for(T * (I / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, T, I, row_limit);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 XB_API int xb_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int I,
                          void* stream) {
-  return swiglu_bwd(dout, gu, dgu, T, I, nullptr, stream);
+  if (I % 8) return -1;
+  if (T <= 0) return 0;
+  swiglu_bwd_kernel<<<grid_for(T * (I / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, T, I, nullptr);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 XB_API int xb_embedding_fwd(const long long* ids, const void* table, void* out, int T, int H,
