@@ -425,3 +425,16 @@ def test_grouped_gemm_writes_all_rows_and_experts(counts, K, N, dtype, accumulat
         ref = a.t() @ dy[s[e]:s[e + 1]].double() + (out0[e].double() if accumulate else 0)
         torch.testing.assert_close(out[e].double(), ref, rtol=2 ** -8 if dtype == torch.bfloat16 else 1e-4, atol=1e-3)
     assert _lib.read_status()[0] == 0
+
+
+def test_mx_scale_of_every_bf16_magnitude():
+    """The power-of-two scale from the bits of the maximum, for every finite bf16 value of a block."""
+    from xorl_b200.ops import fp8_grouped as fg
+    vals = torch.arange(0, 0x7f80, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = torch.zeros(vals.numel(), 128, dtype=torch.bfloat16)
+    x[:, 5] = -vals
+    x[:, 9] = vals * 0.5
+    q, sf = fg.quantize_rows(x.cuda())
+    rq, re = fg.quantize_rows_ref(x)
+    assert torch.equal(sf[:, 0].cpu().int(), re[:, 0] + 127)
+    assert torch.equal(q.cpu().view(torch.float8_e4m3fn).float(), rq.float())

@@ -329,11 +329,18 @@ ggemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 // ------------------------------------------------------------------------------------------------
 constexpr float FP8_MAX = 448.f;
 
-__device__ __forceinline__ uint8_t to_e4m3(float v) {
-  return (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
+__device__ __forceinline__ uint32_t to_e4m3x2(float lo, float hi) {
+  return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
 }
-// Smallest power of two s with amax / s <= 448, as a UE8M0 byte (127 -> 1.0); inv = 1 / s.
+// Smallest power of two s with amax / s <= 448, as a UE8M0 byte (127 -> 1.0); inv = 1 / s.  448 is
+// 1.75 * 2^8 and amax a bf16 value m * 2^x, 1 <= m < 2: the exponent is x - 8, or x - 7 where m > 1.75.
 __device__ __forceinline__ uint8_t pow2_scale(float amax, float& inv) {
+  const uint32_t bits = __float_as_uint(amax);
+  if (amax > 0.f && bits < 0x7f800000u) {
+    const int e = max(-126, min(126, (int)(bits >> 23) - 127 - 8 + ((bits & 0x7fffffu) > 0x600000u ? 1 : 0)));
+    inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    return (uint8_t)(e + 127);
+  }
   int e = -127;
   if (amax > 0.f) {
     int ex;
@@ -348,7 +355,9 @@ __device__ __forceinline__ uint8_t pow2_scale(float amax, float& inv) {
 }
 
 // One warp per row; a pass covers 256 elements (two scale blocks): lane owns 8 consecutive elements
-// (one 16-byte load, one 8-byte store), the block maximum is taken over 16 lanes.
+// (one 16-byte load, one 8-byte store), the block maximum is taken over 16 lanes.  Bound by memory: the loads
+// of QUANT_AHEAD passes are issued before the first maximum, whose shuffles they would otherwise wait behind.
+constexpr int QUANT_AHEAD = 4;
 __global__ void __launch_bounds__(256)
 quant_mx_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ q, long long ldq,
                      uint8_t* __restrict__ sf, int sf_ld, long long M, int KB, const int* __restrict__ row_limit) {
@@ -359,25 +368,33 @@ quant_mx_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t
   const __nv_bfloat16* xr = x + row * ldx;
   uint8_t* qr = q + row * ldq;
   const int K = KB * 128;
-#pragma unroll 4
-  for (int k0 = 0; k0 < K; k0 += 256) {
-    const int k = k0 + lane * 8;
-    const bool in = k < K;
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (in) raw = *reinterpret_cast<const uint4*>(xr + k);
-    const float2 a = unpack_bf16x2(raw.x), b = unpack_bf16x2(raw.y), c = unpack_bf16x2(raw.z), d = unpack_bf16x2(raw.w);
-    float amax = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))),
-                       fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
+  for (int k00 = 0; k00 < K; k00 += 256 * QUANT_AHEAD) {
+    uint4 raw[QUANT_AHEAD];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    float inv;
-    const uint8_t byte = pow2_scale(amax, inv);
-    if (in) {
-      uint2 out;
-      out.x = to_e4m3(a.x * inv) | (to_e4m3(a.y * inv) << 8) | (to_e4m3(b.x * inv) << 16) | ((uint32_t)to_e4m3(b.y * inv) << 24);
-      out.y = to_e4m3(c.x * inv) | (to_e4m3(c.y * inv) << 8) | (to_e4m3(d.x * inv) << 16) | ((uint32_t)to_e4m3(d.y * inv) << 24);
-      *reinterpret_cast<uint2*>(qr + k) = out;
-      if ((lane & 15) == 0) sf[row * sf_ld + (k >> 7)] = byte;
+    for (int u = 0; u < QUANT_AHEAD; ++u) {
+      const int k = k00 + u * 256 + lane * 8;
+      raw[u] = make_uint4(0, 0, 0, 0);
+      if (k < K) raw[u] = *reinterpret_cast<const uint4*>(xr + k);
+    }
+#pragma unroll
+    for (int u = 0; u < QUANT_AHEAD; ++u) {
+      if (k00 + u * 256 >= K) break;                       // warp-uniform
+      const int k = k00 + u * 256 + lane * 8;
+      const float2 a = unpack_bf16x2(raw[u].x), b = unpack_bf16x2(raw[u].y), c = unpack_bf16x2(raw[u].z),
+                   d = unpack_bf16x2(raw[u].w);
+      float amax = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))),
+                         fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      float inv;
+      const uint8_t byte = pow2_scale(amax, inv);
+      if (k < K) {
+        uint2 out;
+        out.x = to_e4m3x2(a.x * inv, a.y * inv) | (to_e4m3x2(b.x * inv, b.y * inv) << 16);
+        out.y = to_e4m3x2(c.x * inv, c.y * inv) | (to_e4m3x2(d.x * inv, d.y * inv) << 16);
+        *reinterpret_cast<uint2*>(qr + k) = out;
+        if ((lane & 15) == 0) sf[row * sf_ld + (k >> 7)] = byte;
+      }
     }
   }
 }
@@ -388,7 +405,7 @@ quant_mx_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t
 __global__ void __launch_bounds__(256)
 quant_mx_weight_kernel(const __nv_bfloat16* __restrict__ w, uint8_t* __restrict__ q_kn, uint8_t* __restrict__ sf_kn,
                        int ld_kn, uint8_t* __restrict__ q_nk, uint8_t* __restrict__ sf_nk, int ld_nk, int K, int N) {
-  __shared__ uint8_t tile[128][132];
+  __shared__ __align__(16) uint8_t tile[128][132];
   __shared__ float red[8];
   const int nb = blockIdx.x, kb = blockIdx.y, e = blockIdx.z;
   const int KB = K / 128, NB = N / 128;
@@ -420,10 +437,9 @@ quant_mx_weight_kernel(const __nv_bfloat16* __restrict__ w, uint8_t* __restrict_
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const int r = r0 + 8 * i;
-    const uint8_t q0 = to_e4m3(v[i][0] * inv), q1 = to_e4m3(v[i][1] * inv), q2 = to_e4m3(v[i][2] * inv),
-                  q3 = to_e4m3(v[i][3] * inv);
-    *reinterpret_cast<uint32_t*>(dkn + (long long)r * N + c4) = q0 | (q1 << 8) | (q2 << 16) | ((uint32_t)q3 << 24);
-    tile[r][c4] = q0; tile[r][c4 + 1] = q1; tile[r][c4 + 2] = q2; tile[r][c4 + 3] = q3;
+    const uint32_t q = to_e4m3x2(v[i][0] * inv, v[i][1] * inv) | (to_e4m3x2(v[i][2] * inv, v[i][3] * inv) << 16);
+    *reinterpret_cast<uint32_t*>(dkn + (long long)r * N + c4) = q;
+    *reinterpret_cast<uint32_t*>(&tile[r][c4]) = q;
   }
   __syncthreads();
   // transposed write: output row n (of this block), 128 contiguous k bytes
