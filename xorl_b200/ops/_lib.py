@@ -166,7 +166,36 @@ def host_lib():
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def current_stream() -> torch.cuda.Stream:
+    """``torch.cuda.current_stream()`` with the device named: left to find it, torch spends 10 us on
+    environment lookups, on every call."""
+    return torch.cuda.current_stream(torch._C._cuda_getDevice())
+
+
+class _NoGrad:
+    """Stands in for an autograd context when nothing will be differentiated."""
+    needs_input_grad = ()
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    mark_non_differentiable = save_for_backward
+
+    def set_materialize_grads(self, value):
+        pass
+
+
+def apply(fn, *args):
+    """``fn.apply(*args)``; with gradients off, and no function transform or forward-mode derivative active,
+    its forward alone: an autograd node that is thrown away costs as much host time as the launch."""
+    if torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0 \
+            or torch._C._are_functorch_transforms_active():
+        return fn.apply(*args)
+    return fn.forward(_NoGrad(), *args)
 
 
 def ptr(t) -> int | None:

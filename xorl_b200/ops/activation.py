@@ -58,5 +58,5 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(gu: torch.Tensor, two_round: bool = True) -> torch.Tensor:
     if gu.is_cuda and gu.dtype == torch.bfloat16 and (gu.shape[-1] // 2) % 8 == 0:
-        return _SwiGLU.apply(gu, two_round)
+        return _lib.apply(_SwiGLU, gu, two_round)
     return swiglu_reference(gu, two_round)

@@ -402,7 +402,7 @@ def qk_norm_rope_attention(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps=1e
     """
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if _kernel_ok(qkv, D) or (D == 64 and _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv)):
-        return _QKNormRopeAttn.apply(qkv.contiguous(), wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps, causal,
+        return _lib.apply(_QKNormRopeAttn, qkv.contiguous(), wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps, causal,
                                      scale)
     return qk_norm_rope_attention_reference(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps,
                                             causal, scale)

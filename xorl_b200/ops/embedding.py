@@ -60,5 +60,5 @@ class _Embedding(torch.autograd.Function):
 
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     if table.is_cuda and table.dtype == torch.bfloat16 and table.shape[1] % 8 == 0:
-        return _Embedding.apply(ids, table)
+        return _lib.apply(_Embedding, ids, table)
     return torch.nn.functional.embedding(ids, table)

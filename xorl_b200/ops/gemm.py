@@ -138,7 +138,7 @@ def gemm_symmetric(a: torch.Tensor, b: torch.Tensor | None = None, *, out_dtype:
     out = torch.empty((M, M), device=a.device, dtype=out_dtype or torch.bfloat16)
     # A panel alone has too few tiles to fill 148 SMs, so the panels run side by side on a few
     # streams (largest first); the launching stream waits for all of them before the mirror.
-    main = torch.cuda.current_stream()
+    main = _lib.current_stream()
     ready = torch.cuda.Event()
     ready.record(main)
     panels = [(r0, min(M, r0 + block)) for r0 in range(0, M, block)][::-1]
@@ -160,6 +160,12 @@ def gemm_symmetric(a: torch.Tensor, b: torch.Tensor | None = None, *, out_dtype:
     return out
 
 
+# A weight gradient below this many multiply-adds runs for a few microseconds on the tensor cores: the
+# stream switch, its events and the lifetime records (about 25 us of host time) cost more than the tail of
+# the input gradient that it could fill.
+SIDE_STREAM_MIN_MACS = 2 ** 31
+
+
 def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
     """dW = dy2^T @ x2 for weight ``w``: written straight into the flat gradient buffer of the ZeRO
     unit (returns None), deferred to a W slot of a zero-bubble schedule, or returned as a tensor."""
@@ -172,10 +178,11 @@ def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
                      gemm(a, b, a_mn=True, b_mn=True, out=o, accumulate=acc))
         return None
     if tgt is not None:
-        side = wgrad_stream(dy2.device) if dy2.is_cuda else None
+        macs = dy2.shape[0] * dy2.shape[1] * x2.shape[1]
+        side = wgrad_stream(dy2.device) if dy2.is_cuda and macs >= SIDE_STREAM_MIN_MACS else None
         if side is not None:
             # overlap with the input-gradient GEMM that follows on the main stream
-            side.wait_stream(torch.cuda.current_stream())
+            side.wait_stream(_lib.current_stream())
             with torch.cuda.stream(side):
                 gemm(dy2, x2, a_mn=True, b_mn=True, out=tgt, accumulate=not fresh)
             dy2.record_stream(side)
@@ -239,7 +246,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -
                 "ops.gemm.linear: %s x %s with K=%d, N=%d runs in the library GEMM, not the tcgen05 kernel "
                 "(bf16 operands, K %% 8 == 0 and N %% 8 == 0 are required)", x.dtype, w.dtype, x.shape[-1], w.shape[0])
         return torch.nn.functional.linear(x, w, bias)
-    y = _Linear.apply(x, w)
+    y = _lib.apply(_Linear, x, w)
     if bias is not None:
         y = y + bias
     return y

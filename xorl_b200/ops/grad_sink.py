@@ -10,6 +10,8 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib
+
 
 def grad_target(p: torch.Tensor):
     """(buffer view or None, fresh) — ``fresh`` means nothing has been written yet in this
@@ -97,5 +99,5 @@ def join_wgrad_stream() -> None:
     global _wgrad_pending
     if _wgrad_pending:
         for st in _wgrad_stream.values():
-            torch.cuda.current_stream().wait_stream(st)
+            _lib.current_stream().wait_stream(st)
         _wgrad_pending = False

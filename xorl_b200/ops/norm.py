@@ -101,7 +101,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6,
             h = x + residual
             return _rmsnorm_ref(h, w, eps, zero_centered), h
         return _rmsnorm_ref(x, w, eps, zero_centered)
-    y, h = _RMSNorm.apply(x, residual, w, eps, zero_centered)
+    y, h = _lib.apply(_RMSNorm, x, residual, w, eps, zero_centered)
     if residual is not None:
         return y, h
     return y

@@ -29,6 +29,7 @@ import torch
 import torch.distributed as dist
 from torch import nn
 
+from ..ops import _lib
 from ..ops import optim as optim_ops
 from .state import ParallelState, get_parallel_state
 
@@ -83,6 +84,7 @@ class FlatParamGroup:
         self.sq: Optional[torch.Tensor] = None  # ||grad shard||^2 of this step, when computed early
         self.sq_valid = False
         self.weight_decay_mask: Optional[List[float]] = None
+        self._kept_views: Dict[str, Tuple[torch.Tensor, List[torch.Tensor]]] = {}
 
     # ---- layout helpers ---------------------------------------------------------------------
     def shard_range(self) -> Tuple[int, int]:
@@ -91,10 +93,25 @@ class FlatParamGroup:
     def param_views(self, flat: torch.Tensor) -> List[torch.Tensor]:
         return [flat[o:o + math.prod(s)].view(s) for o, s in zip(self.offsets, self.shapes)]
 
+    def _own_views(self, flat: torch.Tensor) -> List[torch.Tensor]:
+        """``param_views`` of a buffer that this group keeps for good (its weights or gradients where it is
+        the only owner), made once; buffers that come from the pool are viewed anew each time."""
+        if flat is self.grad_shard:
+            role = "gradients"
+        elif self.full_persistent and flat is self.full:
+            role = "weights"
+        else:
+            return self.param_views(flat)
+        kept = self._kept_views.get(role)
+        if kept is None or kept[0] is not flat:
+            kept = self._kept_views[role] = (flat, self.param_views(flat))
+        return kept[1]
+
     def attach_params(self) -> None:
         """Point every parameter at its view of the gathered buffer."""
-        for (_, p), v in zip(self.named_params, self.param_views(self.full)):
-            p.data = v
+        for (_, p), v in zip(self.named_params, self._own_views(self.full)):
+            if p.data_ptr() != v.data_ptr() or p.shape != v.shape or not p.numel():
+                p.data = v
 
     def detach_params(self) -> None:
         empty = torch.empty(0, device=self.device, dtype=self.compute_dtype)
@@ -109,7 +126,7 @@ class FlatParamGroup:
             self.grad_full[a:b].zero_()
 
     def attach_grad_views(self, fresh: bool = True) -> None:
-        for (_, p), v in zip(self.named_params, self.param_views(self.grad_full)):
+        for (_, p), v in zip(self.named_params, self._own_views(self.grad_full)):
             p._xb_grad_buf = v
             p._xb_grad_fresh = fresh
             p.grad = None
@@ -178,7 +195,7 @@ class ActivationOffloader:
             host = tuple(None if a is None else self._host_buffer(a).copy_(a) for a in acts)
             self.bytes_offloaded += sum(h.numel() * h.element_size() for h in host if h is not None)
             return _Offloaded(host, None)
-        self.stream.wait_stream(torch.cuda.current_stream())
+        self.stream.wait_stream(_lib.current_stream())
         host = []
         with torch.cuda.stream(self.stream):
             for a in acts:
@@ -212,10 +229,10 @@ class ActivationOffloader:
             return item
         self.prefetch(item)
         if item.back is not None:
-            torch.cuda.current_stream().wait_event(item.back)
+            _lib.current_stream().wait_event(item.back)
             for d in item.device:
                 if d is not None:
-                    d.record_stream(torch.cuda.current_stream())
+                    d.record_stream(_lib.current_stream())
         for h in item.host:
             if h is not None:
                 self.pool.setdefault((tuple(h.shape), h.dtype), []).append(h)
@@ -473,7 +490,7 @@ class Zero3Engine:
         side stream first waits for everything issued so far (gradients, clip coefficient)."""
         if not (self.overlap_optimizer and self.symm is None):
             return None
-        cur = torch.cuda.current_stream()
+        cur = _lib.current_stream()
         self.opt_stream.wait_stream(cur)
         for t in tensors:
             if t is not None and t.is_cuda:
@@ -490,13 +507,13 @@ class Zero3Engine:
     def _wait_update(self, g: FlatParamGroup, stream=None) -> None:
         ev = g.update_event
         if ev is not None:
-            (stream or torch.cuda.current_stream()).wait_event(ev)
+            (stream or _lib.current_stream()).wait_event(ev)
 
     def sync_optimizer(self) -> None:
         """Makes the current stream wait for every pending optimizer kernel (anything that reads or
         writes shards outside the forward / backward path calls this first)."""
         if self._opt_pending:
-            torch.cuda.current_stream().wait_stream(self.opt_stream)
+            _lib.current_stream().wait_stream(self.opt_stream)
             for g in self.all_groups():
                 g.update_event = None
             self._opt_pending = False
@@ -512,7 +529,7 @@ class Zero3Engine:
         if pool:
             t, ev = pool.pop()
             if ev is not None and not on_comm_stream:
-                torch.cuda.current_stream().wait_event(ev)
+                _lib.current_stream().wait_event(ev)
             return t
         return torch.empty(numel, device=self.device, dtype=dtype)
 
@@ -530,7 +547,7 @@ class Zero3Engine:
             if self.symm is not None and self.symm.can_gather(g):
                 self.symm.all_gather(g, self.comm_stream)
             elif self.is_cuda:
-                self.comm_stream.wait_stream(torch.cuda.current_stream())
+                self.comm_stream.wait_stream(_lib.current_stream())
                 with torch.cuda.stream(self.comm_stream):
                     dist.all_gather_into_tensor(g.full, g.shard_lp, group=g.pg)
                     g.gather_event = torch.cuda.Event()
@@ -543,7 +560,7 @@ class Zero3Engine:
             if g.full_persistent:
                 self._wait_update(g)          # single owner: the optimizer wrote these weights in place
             if g.gather_event is not None:
-                torch.cuda.current_stream().wait_event(g.gather_event)
+                _lib.current_stream().wait_event(g.gather_event)
                 g.gather_event = None
             g.attach_params()
 
@@ -555,7 +572,7 @@ class Zero3Engine:
             if self.is_cuda:
                 # the buffer may be re-filled by the side stream only after compute is done with it
                 ev = torch.cuda.Event()
-                ev.record(torch.cuda.current_stream())
+                ev.record(_lib.current_stream())
                 self.comm_stream.wait_event(ev)
             self._give_full(g.full)
             g.full = None
@@ -607,7 +624,7 @@ class Zero3Engine:
                 # gradients were produced in place in g.grad_shard
                 if early:
                     ev = torch.cuda.Event()
-                    ev.record(torch.cuda.current_stream())
+                    ev.record(_lib.current_stream())
                     self.norm_stream.wait_event(ev)
                     with torch.cuda.stream(self.norm_stream):
                         self._group_sumsq(g)
@@ -619,7 +636,7 @@ class Zero3Engine:
                         self._group_sumsq(g)
             elif self.is_cuda:
                 ev = torch.cuda.Event()
-                ev.record(torch.cuda.current_stream())
+                ev.record(_lib.current_stream())
                 self.comm_stream.wait_event(ev)
                 with torch.cuda.stream(self.comm_stream):
                     self._rs_collective(g, gf, accumulate)
@@ -675,7 +692,7 @@ class Zero3Engine:
         """Wait for outstanding reductions; all-reduce over replicas (HSDP / DDP) and over
         sequence-parallel ranks that are not part of the shard group."""
         if self.is_cuda:
-            torch.cuda.current_stream().wait_stream(self.comm_stream)
+            _lib.current_stream().wait_stream(self.comm_stream)
         for unit in self.units:
             for g in unit.groups:
                 g.reduce_event = None
@@ -700,7 +717,7 @@ class Zero3Engine:
         if self.symm is not None:
             self.sync_optimizer()
             # parameter shards were rewritten by the optimizer: no peer may read them earlier
-            self.symm.step_barrier(torch.cuda.current_stream())
+            self.symm.step_barrier(_lib.current_stream())
         for unit in self.units:
             for g in unit.groups:
                 g.grad_ready = False
@@ -806,7 +823,8 @@ class Zero3Engine:
             if aux is not None:
                 tensors.append(aux)
                 grads.append(torch.ones_like(aux))
-            torch.autograd.backward(tensors, grads)
+            with torch.autograd.set_multithreading_enabled(False):     # no hand-over to a worker thread per unit
+                torch.autograd.backward(tensors, grads)
             if self.is_cuda:
                 from ..ops.grad_sink import join_wgrad_stream
                 join_wgrad_stream()          # weight-gradient GEMMs issued on their side stream
@@ -855,18 +873,23 @@ class Zero3Engine:
                 extra = extra_loss_fn(ctx)
                 if extra is not None:
                     total = total + extra
-            total.backward()
+            with torch.autograd.set_multithreading_enabled(False):
+                total.backward()
         if self.is_cuda:
             from ..ops.grad_sink import join_wgrad_stream
             join_wgrad_stream()
         return loss.detach(), tuple(a.grad if a is not None else None for a in head_in)
 
-    def embed_backward(self, input_ids, ctx, dacts) -> None:
-        with torch.enable_grad():
-            emb = self.model.forward_embed(input_ids, ctx)
+    def embed_backward(self, input_ids, ctx, dacts, emb=None) -> None:
+        """``emb``: the embedding's outputs with their graph; looked up again where the caller has not kept
+        them."""
+        if emb is None:
+            with torch.enable_grad():
+                emb = self.model.forward_embed(input_ids, ctx)
         pairs = [(o, d) for o, d in zip(emb, dacts) if o is not None and d is not None]
         if pairs and pairs[0][0].requires_grad:
-            torch.autograd.backward([o for o, _ in pairs], [d for _, d in pairs])
+            with torch.autograd.set_multithreading_enabled(False):
+                torch.autograd.backward([o for o, _ in pairs], [d for _, d in pairs])
         if self.is_cuda:
             from ..ops.grad_sink import join_wgrad_stream
             join_wgrad_stream()
@@ -882,13 +905,14 @@ class Zero3Engine:
         self.gather(root)
         self.wait_gather(root)
         ctx = self.make_step_context(input_ids, position_ids, cu_seqlens, grad_scale, extra)
-        with torch.no_grad():
-            acts = model.forward_embed(input_ids, ctx)
+        with torch.enable_grad():
+            emb = model.forward_embed(input_ids, ctx)
+        acts = tuple(e.detach() if e is not None else None for e in emb)
         acts, saved = self.chunk_forward(layers, acts, ctx, keep_last_gathered=True)
         self._prepare_grad_buffers(root)
         loss_value, dacts = self.head_forward_backward(acts, labels, ctx, grad_scale, extra_loss_fn)
         dacts, _ = self.chunk_backward(layers, saved, dacts, ctx)
-        self.embed_backward(input_ids, ctx, dacts)
+        self.embed_backward(input_ids, ctx, dacts, emb)
         self._reduce_unit_grads(root)
         if self.reshard:
             self.release(root)
@@ -947,8 +971,7 @@ class Zero3Engine:
         1-element device tensors (no host sync).  Dense shards are summed over the shard group,
         expert shards over ep_fsdp x ep (src/xorl/distributed/fsdp2/clip_grad_norm.py:60-257)."""
         dev = self.device
-        dense_sq = torch.zeros(1, device=dev, dtype=torch.float32)
-        expert_sq = torch.zeros(1, device=dev, dtype=torch.float32)
+        dense_sq = expert_sq = None
         first_d = first_e = True
 
         def counts_as_expert(g) -> bool:
@@ -956,7 +979,7 @@ class Zero3Engine:
 
         # lm-head rows under lm-head-only tensor parallelism: distinct rows on the ranks of an lm_head_tp group,
         # each sharded over its lm_head_replica group
-        head_sq = torch.zeros(1, device=dev, dtype=torch.float32)
+        head_sq = torch.zeros(1, device=dev, dtype=torch.float32) if getattr(self.ps, "lm_head_tp_size", 1) > 1 else 0
         head_groups = [g for g in self.all_groups() if getattr(g, "is_head", False) and g.grad_ready]
         for g in head_groups:
             head_sq += g.grad_shard.float().pow(2).sum()
@@ -964,8 +987,8 @@ class Zero3Engine:
 
         if self.is_cuda:
             # per-unit partial sums taken early live on the side streams
-            torch.cuda.current_stream().wait_stream(self.norm_stream)
-            torch.cuda.current_stream().wait_stream(self.comm_stream)
+            _lib.current_stream().wait_stream(self.norm_stream)
+            _lib.current_stream().wait_stream(self.comm_stream)
         early_d, early_e = [], []
         for g in self.all_groups():
             if not g.grad_ready or getattr(g, "is_head", False):
@@ -974,16 +997,26 @@ class Zero3Engine:
                 (early_e if counts_as_expert(g) else early_d).append(g.sq)
                 g.sq_valid = False
             elif counts_as_expert(g):
+                if first_e:
+                    expert_sq = torch.zeros(1, device=dev, dtype=torch.float32)
                 optim_ops.sumsq_(g.grad_shard, expert_sq, not first_e)
                 first_e = False
             else:
+                if first_d:
+                    dense_sq = torch.zeros(1, device=dev, dtype=torch.float32)
                 optim_ops.sumsq_(g.grad_shard, dense_sq, not first_d)
                 first_d = False
         # fixed order (unit order), one reduction: the same bits every run
         if early_d:
-            dense_sq = dense_sq + torch.cat(early_d).sum()
+            early = torch.cat(early_d).sum(0, keepdim=True)
+            dense_sq = early if first_d else dense_sq + early
         if early_e:
-            expert_sq = expert_sq + torch.cat(early_e).sum()
+            early = torch.cat(early_e).sum(0, keepdim=True)
+            expert_sq = early if first_e else expert_sq + early
+        if dense_sq is None:
+            dense_sq = torch.zeros(1, device=dev, dtype=torch.float32)
+        if expert_sq is None and self.ps.ep_size > 1:
+            expert_sq = torch.zeros(1, device=dev, dtype=torch.float32)
         tp_pg = self.ps.group("tp") if self.ps.tp_size > 1 else None
         if tp_pg is not None:
             # replicated parameters (norm weights, embeddings) hold identical gradients on every
@@ -1007,7 +1040,7 @@ class Zero3Engine:
                 dist.all_reduce(expert_sq, group=self.ep_shard_pg)
             if self.ps.group("ep") is not None:
                 dist.all_reduce(expert_sq, group=self.ps.group("ep"))
-        total = dense_sq + expert_sq
+        total = dense_sq if expert_sq is None else dense_sq + expert_sq
         if getattr(self.ps, "lm_head_tp_size", 1) > 1:
             if head_groups and head_groups[0].pg is not None:
                 dist.all_reduce(head_sq, group=head_groups[0].pg)
@@ -1016,8 +1049,8 @@ class Zero3Engine:
             total = total + head_sq
         if self.ps.pp_size > 1 and self.ps.group("pp") is not None:
             dist.all_reduce(total, group=self.ps.group("pp"))
-        norm = torch.zeros(1, device=dev, dtype=torch.float32)
-        coef = torch.ones(1, device=dev, dtype=torch.float32)
+        norm = torch.empty(1, device=dev, dtype=torch.float32)      # both are written, nothing is added to them
+        coef = torch.empty(1, device=dev, dtype=torch.float32)
         optim_ops.clip_coef_(total, max_norm, norm, coef)
         return norm, coef
 
