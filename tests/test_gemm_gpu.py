@@ -52,3 +52,29 @@ def test_gemm_fp32_out_and_accumulate(variant):
     cb = gemm.gemm(a, b)
     cb2 = gemm.gemm(a, b, out=cb.clone(), accumulate=True)
     assert torch.allclose(cb2.float(), 2 * ref, rtol=2e-2, atol=0.5)
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 1024), (61, 4096, 4096), (16, 2048, 8192), (4096, 48, 4096), (136, 264, 1032),
+                                   (128, 256, 4160), (520, 16, 12288), (8, 1000, 520)])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_gemm_with_few_tiles_splits_the_reduction(M, N, K, a_mn, b_mn, out, accumulate):
+    """Cluster split-K: ragged tiles, remainders of K over the CTAs, every output form.  fp32 sums of K
+    products differ by at most K * 2^-24 of the sum of their magnitudes; a bf16 result adds 2^-8."""
+    from xorl_b200.ops import _lib, gemm
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("row pitch of an MN-major operand")
+    torch.manual_seed(M + N)
+    a = torch.randn((K, M) if a_mn else (M, K), device="cuda", dtype=torch.bfloat16)
+    b = torch.randn((K, N) if b_mn else (N, K), device="cuda", dtype=torch.bfloat16)
+    c0 = torch.randn(M, N, device="cuda").to(out)
+    c = gemm.gemm(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn), out=c0.clone(), accumulate=accumulate)
+    again = gemm.gemm(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn), out=c0.clone(), accumulate=accumulate)
+    assert torch.equal(c, again)
+    A, B = (a.t() if a_mn else a).double(), (b.t() if b_mn else b).double()
+    ref = A @ B.t() + (c0.double() if accumulate else 0)
+    bound = (A.abs() @ B.abs().t() + c0.double().abs()) * (K * 2.0 ** -24)
+    if out == torch.bfloat16:
+        bound = bound + ref.abs() * 2.0 ** -8
+    assert ((c.double() - ref).abs() <= bound + 1e-6).all()
+    assert all(v == 0 for v in _lib.read_status()[:4])

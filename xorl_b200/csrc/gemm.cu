@@ -315,6 +315,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
 
 }  // namespace xb_gemm
 
+int xb_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, long long ldc,
+                   int a_mn, int b_mn, int out_fp32, int accumulate, cudaStream_t st);
+
 // C[M,N] (+)= op(A) * op(B)^T.  See the header comment for a_mn / b_mn.  Leading dimensions are in
 // elements and must be multiples of 8; A and B must be 16-byte aligned.  Returns 0 on success.
 XB_API int xb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
@@ -341,6 +344,9 @@ XB_API int xb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int
     rc = xb_make_tmap_2d(&tb, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, ldb, BK, 64,
                          CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return -3;
+  // few tiles: the reduction is split over the CTAs of a cluster where that fits (gemm_splitk.cu)
+  rc = xb_gemm_splitk(ta, tb, C, M, N, K, ldc, a_mn, b_mn, out_fp32, accumulate, reinterpret_cast<cudaStream_t>(stream));
+  if (rc != 1) return rc;
   Params p;
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc;

@@ -52,6 +52,13 @@ def set_batch_invariant(on: bool) -> bool:
     return prev
 
 
+def _splits_k(M: int, N: int, K: int) -> bool:
+    """Outputs of at most 37 tiles of 128 x 256 with a long reduction (low-rank factors, router, few rows):
+    four or more CTAs share a tile (csrc/gemm_splitk.cu); the pair kernel would keep as many SMs busy as there are
+    half tiles."""
+    return K >= 2048 and -(-M // 128) * -(-N // 256) <= 37
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None,
          accumulate: bool = False) -> torch.Tensor:
@@ -95,7 +102,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     lib = _lib.cuda_lib()
     args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
             out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate))
-    if _BATCH_INVARIANT or (_VARIANT == "pair" and M >= 384):
+    if _BATCH_INVARIANT or (_VARIANT == "pair" and M >= 384 and not _splits_k(M, N, K)):
         rc = lib.xb_gemm_bf16_pair(*args, _lib.stream_ptr())
     else:
         rc = lib.xb_gemm_bf16(*args, _lib.stream_ptr())
