@@ -78,3 +78,20 @@ def test_gemm_with_few_tiles_splits_the_reduction(M, N, K, a_mn, b_mn, out, accu
         bound = bound + ref.abs() * 2.0 ** -8
     assert ((c.double() - ref).abs() <= bound + 1e-6).all()
     assert all(v == 0 for v in _lib.read_status()[:4])
+
+
+@pytest.mark.parametrize("M,N,K,K2", [(384, 256, 64, 8), (1000, 520, 520, 48), (4096, 6144, 1024, 72), (200, 512, 256, 16)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_sum_of_two_products(M, N, K, K2, b_mn):
+    from xorl_b200.ops import _lib
+    from xorl_b200.ops.lora import gemm_sum
+    torch.manual_seed(K2)
+    x, x2 = (torch.randn(M, k, device="cuda", dtype=torch.bfloat16) for k in (K, K2))
+    w, w2 = (torch.randn((k, N) if b_mn else (N, k), device="cuda", dtype=torch.bfloat16) for k in (K, K2))
+    op = (lambda t: t.double()) if b_mn else (lambda t: t.double().t())
+    ref = x.double() @ op(w) + x2.double() @ op(w2)
+    mag = x.double().abs() @ op(w).abs() + x2.double().abs() @ op(w2).abs()
+    # one bf16 rounding (2^-8 of the result), two where the second product is added to the first
+    bound = mag * ((K + K2) * 2.0 ** -24) + (ref.abs() + (x.double() @ op(w)).abs()) * 2.0 ** -8
+    assert ((gemm_sum(x, w, x2, w2, b_mn).double() - ref).abs() <= bound + 1e-6).all()
+    assert all(v == 0 for v in _lib.read_status()[:4])

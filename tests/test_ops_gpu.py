@@ -385,3 +385,50 @@ def test_moe_block_gpu_matches_reference():
     _close(out, ref, 3e-2, 0.03 * ref.abs().max().item(), "moe out")
     assert x.grad is not None and torch.isfinite(x.grad.float()).all()
     assert torch.isfinite(blk.experts.gate_up_proj.grad.float()).all()
+
+
+@pytest.mark.parametrize("T,slices,out,rank,scaling", [(512, ((0, 256),), 256, 16, 2.0), (100, ((0, 256),), 256, 8, 1.0),
+                                                       (700, ((0, 256), (256, 320), (320, 384)), 384, 16, 0.3),
+                                                       (385, ((64, 128),), 384, 24, 2.0), (1, ((0, 64), (128, 192)), 256, 8, 0.5)])
+def test_lora_linear_against_float64(T, slices, out, rank, scaling):
+    """Adapters on whole and on partial outputs, with rows that have no adapter, against float64 and next to
+    one product per factor: no error may be larger (that path rounds each delta twice more)."""
+    from xorl_b200.adapters.lora import LoraLinear
+    from xorl_b200.models.layers import Linear
+    from xorl_b200.ops import lora as L
+    torch.manual_seed(T)
+    fin = 320
+    mod = LoraLinear(Linear(fin, out, dtype=torch.bfloat16, device=DEV), rank, scaling * rank,
+                     [(str(i), s, e) for i, (s, e) in enumerate(slices)])
+    for p in mod.parameters():
+        torch.nn.init.normal_(p, 0, 0.05)
+    x0 = torch.randn(T, fin, device=DEV, dtype=torch.bfloat16)
+    go = torch.randn(T, out, device=DEV, dtype=torch.bfloat16)
+
+    def run(fn, dtype):
+        x = x0.detach().clone().to(dtype).requires_grad_()
+        ps = [p.detach().to(dtype).requires_grad_() for d in (mod.lora_A, mod.lora_B) for p in d.values()]
+        y = fn(x, ps)
+        y.backward(go.to(dtype))
+        return [y.detach(), x.grad] + [p.grad for p in ps]
+
+    def plain(x, ps, lin):
+        w, n = mod.weight.to(x.dtype), len(slices)
+        y = lin(x, w)
+        cols = [y[:, :0]]
+        cur = 0
+        for i, (s, e) in enumerate(slices):
+            cols += [y[:, cur:s], y[:, s:e] + lin(lin(x, ps[i]), ps[n + i]) * scaling]
+            cur = e
+        return torch.cat(cols + [y[:, cur:]], -1)
+
+    from xorl_b200.ops.gemm import linear
+    before = L.launch_count()
+    got = run(lambda x, ps: L.lora_linear(x, mod.weight, scaling, slices, ps[:len(slices)], ps[len(slices):]), torch.bfloat16)
+    assert T < 384 or L.launch_count() > before
+    old = run(lambda x, ps: plain(x, ps, linear), torch.bfloat16)
+    exact = run(lambda x, ps: plain(x, ps, torch.nn.functional.linear), torch.float64)
+    assert L.lora_linear_ok(x0, mod.weight, slices, list(mod.lora_A.values()), list(mod.lora_B.values()))
+    for g, o, e in zip(got, old, exact):
+        eg, eo = ((t.double() - e).norm().item() / e.norm().item() for t in (g, o))
+        assert eg <= 1.05 * eo + 2 ** -12, (eg, eo)

@@ -21,6 +21,7 @@ from torch import nn
 
 from ..models.layers import Linear
 from ..ops import gemm as gemm_ops
+from ..ops import lora as lora_ops
 
 FUSED_PARTS = {"qkv_proj": ("q_proj", "k_proj", "v_proj"), "gate_up_proj": ("gate_proj", "up_proj")}
 DEFAULT_TARGETS = ("q_proj", "k_proj", "v_proj", "o_proj", "gate_proj", "up_proj", "down_proj")
@@ -53,6 +54,13 @@ class LoraLinear(nn.Module):
         self.b_init_std = b_init_std
 
     def forward(self, x):
+        if getattr(self, "enabled", True):
+            spans = tuple((s, e) for _, s, e in self.slices)
+            a = [self.lora_A[n] for n, _, _ in self.slices]
+            b = [self.lora_B[n] for n, _, _ in self.slices]
+            if lora_ops.lora_linear_ok(x, self.weight, spans, a, b):
+                y = lora_ops.lora_linear(x, self.weight, self.scaling, spans, a, b)
+                return y if self.bias is None else y + self.bias
         y = gemm_ops.linear(x, self.weight, self.bias)
         if not getattr(self, "enabled", True):
             return y                              # reference pass: the frozen base model alone

@@ -25,11 +25,22 @@
 
 namespace xb_gemm2 {
 
-template <bool A_MN, bool B_MN>
+// The second pair of operands.
+template <bool EXT>
+struct Ext {
+  CUtensorMap a, b, b64;
+  int num_kb;
+};
+template <>
+struct Ext<false> {};
+
+// EXT: the reduction goes on over a second pair of operands, C = A B^T + A2 B2^T in one accumulator
+// (a low-rank adapter beside its base weight: one more K block per tile instead of a pass over C).
+template <bool A_MN, bool B_MN, bool EXT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_b64, const __grid_constant__ CUtensorMap tmap_c,
-             const Params p) {
+             const __grid_constant__ Ext<EXT> ext, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~(uintptr_t)1023);
@@ -41,7 +52,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const uint32_t cta = cluster_ctarank();          // 0 = leader
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
-  const int num_kb = (p.K + BK - 1) / BK;
+  const int num_kb1 = (p.K + BK - 1) / BK;
+  int num_kb = num_kb1;
+  if constexpr (EXT) num_kb += ext.num_kb;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -90,24 +103,31 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           uint8_t* sb = sa + 2 * A_BYTES;
           const uint32_t full_leader = mapa_u32(xb_smem_u32(&bars->full[s]), 0);
           if (cta == 0) mbar_expect_tx(&bars->full[s], stage_tx);
-          const int k0 = kb * BK;
+          int k0 = kb * BK;
+          const CUtensorMap *map_a = &tmap_a, *map_b = &tmap_b, *map_b64 = &tmap_b64;
+          if constexpr (EXT) {
+            if (kb >= num_kb1) {
+              k0 = (kb - num_kb1) * BK;
+              map_a = &ext.a; map_b = &ext.b; map_b64 = &ext.b64;
+            }
+          }
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             if (u >= item.nsub) break;
             if (!A_MN) {
-              tma_load_2d_pair(sa + u * A_BYTES, &tmap_a, full_leader, k0, m0 + 256 * u);
+              tma_load_2d_pair(sa + u * A_BYTES, map_a, full_leader, k0, m0 + 256 * u);
             } else {
 #pragma unroll
               for (int j = 0; j < BM / 64; ++j)
-                tma_load_2d_pair(sa + u * A_BYTES + j * (BK * 128), &tmap_a, full_leader,
+                tma_load_2d_pair(sa + u * A_BYTES + j * (BK * 128), map_a, full_leader,
                                  m0 + 256 * u + 64 * j, k0);
             }
           }
           if (!B_MN) {
-            tma_load_2d_pair(sb, bcols == BNH ? &tmap_b : &tmap_b64, full_leader, k0, n0);
+            tma_load_2d_pair(sb, bcols == BNH ? map_b : map_b64, full_leader, k0, n0);
           } else {
             for (int j = 0; j < bcols / 64; ++j)
-              tma_load_2d_pair(sb + j * (BK * 128), &tmap_b, full_leader, n0 + 64 * j, k0);
+              tma_load_2d_pair(sb + j * (BK * 128), map_b, full_leader, n0 + 64 * j, k0);
           }
         }
       }
@@ -348,12 +368,12 @@ static int g_batch_invariant = 0;
 
 static int resident_pairs_cache[64] = {0};
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool EXT>
 static int resident_pairs() {
   int dev = 0;
   cudaGetDevice(&dev);
   static bool configured[64] = {false};
-  auto kern = gemm2_kernel<A_MN, B_MN>;
+  auto kern = gemm2_kernel<A_MN, B_MN, EXT>;
   if (!configured[dev & 63]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
       return -1;
@@ -375,10 +395,10 @@ static int resident_pairs() {
   return resident_pairs_cache[dev & 63];
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool EXT = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb64, const CUtensorMap& tc,
-                  Params& p, cudaStream_t stream) {
-  const int pairs_max = resident_pairs<A_MN, B_MN>();
+                  Params& p, cudaStream_t stream, const Ext<EXT>& ext = Ext<EXT>()) {
+  const int pairs_max = resident_pairs<A_MN, B_MN, EXT>();
   if (pairs_max <= 0) return -10;
   plan_items(p, pairs_max, true);
   if (g_batch_invariant) {
@@ -387,7 +407,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     p.num_items = p.full_items;
   }
   const int pairs = p.num_items < pairs_max ? p.num_items : pairs_max;
-  gemm2_kernel<A_MN, B_MN><<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, tb64, tc, p);
+  gemm2_kernel<A_MN, B_MN, EXT><<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, tb64, tc, ext, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -399,16 +419,12 @@ XB_API int xb_gemm_set_batch_invariant(int on) {
   return prev;
 }
 
-// Same contract as xb_gemm_bf16.
-XB_API int xb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
-                             long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32,
-                             int accumulate, void* stream) {
-  using namespace xb_gemm2;
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) % 16) ||
-      (reinterpret_cast<uintptr_t>(B) % 16))
+namespace xb_gemm2 {
+// Tensor maps of one operand pair; 0 or a negative code.
+static int operand_maps(CUtensorMap& ta, CUtensorMap& tb, CUtensorMap& tb64, const void* A, const void* B, int M,
+                        int N, int K, long long lda, long long ldb, int a_mn, int b_mn) {
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) % 16) || (reinterpret_cast<uintptr_t>(B) % 16))
     return -1;
-  CUtensorMap ta, tb, tb64;
   int rc;
   if (!a_mn)
     rc = xb_make_tmap_2d(&ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda, BM, BK,
@@ -428,8 +444,11 @@ XB_API int xb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N
                          CU_TENSOR_MAP_SWIZZLE_128B);
     tb64 = tb;
   }
-  if (rc) return -3;
-  Params p;
+  return rc ? -3 : 0;
+}
+
+static void fill_params(Params& p, CUtensorMap& tc, void* C, int M, int N, int K, long long ldc, int out_fp32,
+                        int accumulate) {
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc;
   p.out_fp32 = out_fp32; p.accumulate = accumulate;
@@ -439,7 +458,6 @@ XB_API int xb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N
   p.status = xb_status_ptr();
   // Output through shared memory + TMA when C can be described by a tensor map (16-byte aligned base
   // and row pitch) and the mode has a TMA form: plain store, or fp32 add for accumulation.
-  CUtensorMap tc = ta;
   const int es = out_fp32 ? 4 : 2;
   p.tma_epilogue = 0;
   static const bool tma_epi_enabled = []() {
@@ -451,9 +469,47 @@ XB_API int xb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N
                         ldc, BM, 128 / es, CU_TENSOR_MAP_SWIZZLE_128B) == 0)
       p.tma_epilogue = 1;
   }
+}
+}  // namespace xb_gemm2
+
+// Same contract as xb_gemm_bf16.
+XB_API int xb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                             long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32,
+                             int accumulate, void* stream) {
+  using namespace xb_gemm2;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  CUtensorMap ta, tb, tb64;
+  const int rc = operand_maps(ta, tb, tb64, A, B, M, N, K, lda, ldb, a_mn, b_mn);
+  if (rc) return rc;
+  Params p;
+  CUtensorMap tc = ta;
+  fill_params(p, tc, C, M, N, K, ldc, out_fp32, accumulate);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (!a_mn && !b_mn) return launch<false, false>(ta, tb, tb64, tc, p, st);
   if (!a_mn && b_mn) return launch<false, true>(ta, tb, tb64, tc, p, st);
   if (a_mn && !b_mn) return launch<true, false>(ta, tb, tb64, tc, p, st);
   return launch<true, true>(ta, tb, tb64, tc, p, st);
+}
+
+// C[M,N] (bf16) = A[M,K] op(B)[N,K]^T + A2[M,K2] op(B2)[N,K2]^T, both products in one fp32 accumulator;
+// b_mn holds for B and B2.
+XB_API int xb_gemm_bf16_pair_ext(const void* A, const void* B, const void* A2, const void* B2, void* C, int M, int N,
+                                 int K, int K2, long long lda, long long ldb, long long lda2, long long ldb2,
+                                 long long ldc, int b_mn, void* stream) {
+  using namespace xb_gemm2;
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || K2 <= 0) return -1;
+  CUtensorMap ta, tb, tb64;
+  int rc = operand_maps(ta, tb, tb64, A, B, M, N, K, lda, ldb, 0, b_mn);
+  if (rc) return rc;
+  Ext<true> ext;
+  rc = operand_maps(ext.a, ext.b, ext.b64, A2, B2, M, N, K2, lda2, ldb2, 0, b_mn);
+  if (rc) return rc;
+  ext.num_kb = (K2 + BK - 1) / BK;
+  Params p;
+  CUtensorMap tc = ta;
+  fill_params(p, tc, C, M, N, K, ldc, 0, 0);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!b_mn) return launch<false, false, true>(ta, tb, tb64, tc, p, st, ext);
+  return launch<false, true, true>(ta, tb, tb64, tc, p, st, ext);
 }

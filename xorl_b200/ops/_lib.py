@@ -32,6 +32,8 @@ _SIGNATURES = {
     "xb_gemm_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, P],
     "xb_gemm_set_batch_invariant": [I],
     "xb_gemm_bf16_pair": [P, P, P, I, I, I, L, L, L, I, I, I, I, P],
+    "xb_gemm_bf16_pair_ext": [P, P, P, P, P, I, I, I, I, L, L, L, L, L, I, P],
+    "xb_lora_pack": [P, P, P, P, P, I, P, P, I, I, P],
     "xb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, I, P],
     "xb_rmsnorm_bwd_partial_rows": [I],
     "xb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, P],
