@@ -251,6 +251,44 @@ def test_qk_norm_rope_attention(do_norm):
         _close(wk.grad, wkr.grad, 5e-2, 0.05 * wkr.grad.abs().max().item(), "dwk")
 
 
+@pytest.mark.parametrize("lens,Hq,Hkv,causal,window", [
+    ([1], 1, 1, True, 0), ([127, 129, 256, 257], 8, 1, True, 0), ([2000, 40], 16, 2, True, 0), ([8192], 8, 8, True, 0),
+    ([513], 12, 4, False, 0), ([900], 8, 1, True, 300), ([128, 640], 4, 1, False, 130), ([3000, 3000, 2192], 32, 8, True, 0)])
+def test_attention_128_against_the_single_backward_kernel(lens, Hq, Hkv, causal, window):
+    """Two query tiles per forward CTA, 128-row key tiles and heads dealt over clusters of 1, 2 and 4 in the
+    backward, on long and ragged documents: against float32 sums of the same bf16 values (short calls) and
+    against the kernel with 64-row tiles and P in shared memory (long ones).  Both round P and dS to bf16, so
+    results agree to about two of its roundings, 2^-8 of their norm."""
+    from xorl_b200.ops import _lib, attention as A
+    torch.manual_seed(1)
+    T, D = sum(lens), 128
+    cu = _make_cu(lens)
+    q, k, v = (torch.randn(T, h, D, device=DEV, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    go = torch.randn(T, Hq, D, device=DEV, dtype=torch.bfloat16)
+    out, lse = A._attn_fwd(q, k, v, cu, causal, D ** -0.5, window)
+    dv = torch.empty_like(v)
+    dq, dk = A._attn_bwd(q, k, v, out, go, lse, cu, causal, D ** -0.5, dv, window)
+    again = A._attn_bwd(q, k, v, out, go, lse, cu, causal, D ** -0.5, torch.empty_like(v), window)
+    assert torch.equal(dq, again[0]) and torch.equal(dk, again[1])      # sums in a fixed order
+    got = [out, dq, dk, dv]
+    if T <= 2048 or window:
+        ins = [t.float().requires_grad_() for t in (q, k, v)]
+        ref = A.attention_reference(*ins, cu, causal=causal, window=window or None)
+        ref.backward(go.float())
+        refs = [ref.detach()] + [t.grad for t in ins]
+    else:
+        prev = A.set_backward_mode("fused")
+        dv2 = torch.empty_like(v)
+        dq2, dk2 = A._attn_bwd(q, k, v, out, go, lse, cu, causal, D ** -0.5, dv2, window)
+        A.set_backward_mode(prev)
+        refs = [None, dq2, dk2, dv2]
+    for name, g, r in zip(("out", "dq", "dk", "dv"), got, refs):
+        if r is not None:
+            err = (g.float() - r.float()).norm().item() / max(r.float().norm().item(), 1e-3 * go.float().norm().item())
+            assert err < 2 ** -7, (name, err)
+    assert _lib.read_status()[0] == 0
+
+
 def _attention_float64(qkv, wq, wk, cos, sin, lens, Hq, Hkv, D, eps, causal):
     """The block in float64 without any rounding inside."""
     T = qkv.shape[0]

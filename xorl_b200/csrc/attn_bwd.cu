@@ -448,8 +448,8 @@ static int g_split = 1;
 
 }  // namespace xb_attn_bwd_ns
 
-// 1 (default): dK / dV from the key-stationary kernel in attn_bwd_dkv.cu and dQ from the
-// query-stationary kernel in attn_bwd_dq.cu (no atomics); 0: the single kernel of this file, which
+// 1 (default): dK / dV from a key-stationary and dQ from a query-stationary kernel (attn_bwd_hd128.cu, no
+// atomics); 0: the single kernel of this file, which
 // adds dQ partials to global memory with fp32 vector reductions.  Returns the previous setting.
 XB_API int xb_attn_bwd_set_split(int split) {
   const int prev = xb_attn_bwd_ns::g_split;
@@ -457,16 +457,19 @@ XB_API int xb_attn_bwd_set_split(int split) {
   return prev;
 }
 
-XB_API int xb_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dout, const float* lse,
-                          const float* delta, float* dq, const int* cu_seqlens, const int* k_starts,
-                          long long ldq, long long ldk, long long ldv, long long lddo, int num_seqs, int T,
-                          int Tk, int Hq, int Hkv, int D, int causal, float scale, int accumulate,
-                          int max_q_tiles, void* stream);
-XB_API int xb_attn_bwd_dkv(const void* q, const void* k, const void* v, const void* dout, const float* lse,
-                           const float* delta, float* dk, void* dv, const int* cu_seqlens, const int* k_starts,
-                           long long ldq, long long ldk, long long ldv, long long lddo, long long lddv,
-                           int num_seqs, int T, int Tk, int Hq, int Hkv, int D, int causal, float scale,
-                           int max_tiles, void* stream);
+int xb_attn_bwd_hd128(const void* q, const void* k, const void* v, const void* dout, const float* lse,
+                      const float* delta, float* dq, float* dk, void* dv, const int* cu_seqlens, const int* k_starts,
+                      long long ldq, long long ldk, long long ldv, long long lddo, long long lddv, int num_seqs, int T,
+                      int Tk, int Hq, int Hkv, int causal, float scale, int accumulate, int max_tiles,
+                      cudaStream_t stream);
+int xb_attn_dkv_hd64(const void* q, const void* k, const void* v, const void* dout, const float* lse,
+                     const float* delta, float* dk, void* dv, const int* cu_seqlens, long long ldq, long long ldk,
+                     long long ldv, long long lddo, long long lddv, int num_seqs, int T, int Hq, int Hkv, int causal,
+                     float scale, cudaStream_t stream);
+int xb_attn_dq_hd64(const void* q, const void* k, const void* v, const void* dout, const float* lse,
+                    const float* delta, float* dq, const int* cu_seqlens, long long ldq, long long ldk, long long ldv,
+                    long long lddo, int num_seqs, int T, int Hq, int Hkv, int causal, float scale,
+                    cudaStream_t stream);
 
 // Inputs as in xb_attn_fwd plus out / dout [T, Hq, 128] and lse [Hq, T].
 // Scratch: delta fp32 [Hq * T]; dq_accum fp32 [T * Hq * 128] (this call zeroes it).
@@ -527,12 +530,9 @@ XB_API int xb_attn_bwd_ex(const void* q, const void* k, const void* v, const voi
   if (g_split || (causal >> 1)) {     // sliding windows are implemented by the split kernels only
     // dq_accum is written with plain stores (added to when flags bit 0 is set); rows outside every
     // sequence keep the zeros of the memset above
-    int rc = xb_attn_bwd_dkv(q, k, v, dout, lse, delta, dk, dv, cu_seqlens, k_starts, ldq, ldk, ldv, lddo, lddv,
-                             num_seqs, T, Tk, Hq, Hkv, D, causal, scale, max_tiles, stream);
-    if (rc) return rc;
-    const int q_tiles = max_tiles > 0 ? (max_tiles + 1) / 2 + num_seqs : 0;
-    return xb_attn_bwd_dq(q, k, v, dout, lse, delta, dq_accum, cu_seqlens, k_starts, ldq, ldk, ldv, lddo,
-                          num_seqs, T, Tk, Hq, Hkv, D, causal, scale, (flags & 1) ? 1 : 0, q_tiles, stream);
+    const int tiles = max_tiles > 0 ? (max_tiles + 1) / 2 + num_seqs : 0;     // 128-row tiles
+    return xb_attn_bwd_hd128(q, k, v, dout, lse, delta, dq_accum, dk, dv, cu_seqlens, k_starts, ldq, ldk, ldv, lddo,
+                             lddv, num_seqs, T, Tk, Hq, Hkv, causal, scale, (flags & 1) ? 1 : 0, tiles, st);
   }
   Params p;
   p.lse = lse; p.delta = delta; p.dq_accum = dq_accum; p.dk = dk;
@@ -570,9 +570,9 @@ XB_API int xb_attn_bwd_hd64(const void* q, const void* k, const void* v, const f
     return -6;
   const long long rows = (long long)T * Hq;
   attn_delta_hd64_kernel<<<(int)((rows + 7) / 8), 256, 0, st>>>(out_f32, (const __nv_bfloat16*)dout, lddo, delta, T, Hq);
-  int rc = xb_attn_bwd_dkv(q, k, v, dout, lse, delta, dk, dv, cu_seqlens, nullptr, ldq, ldk, ldv, lddo, lddv,
-                           num_seqs, T, T, Hq, Hkv, 64, causal & 1, scale, 0, stream);
+  const int rc = xb_attn_dkv_hd64(q, k, v, dout, lse, delta, dk, dv, cu_seqlens, ldq, ldk, ldv, lddo, lddv, num_seqs,
+                                  T, Hq, Hkv, causal, scale, st);
   if (rc) return rc;
-  return xb_attn_bwd_dq(q, k, v, dout, lse, delta, dq, cu_seqlens, nullptr, ldq, ldk, ldv, lddo, num_seqs, T, T,
-                        Hq, Hkv, 64, causal & 1, scale, 0, 0, stream);
+  return xb_attn_dq_hd64(q, k, v, dout, lse, delta, dq, cu_seqlens, ldq, ldk, ldv, lddo, num_seqs, T, Hq, Hkv, causal,
+                         scale, st);
 }

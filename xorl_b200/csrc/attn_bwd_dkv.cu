@@ -1,9 +1,10 @@
-// dK / dV of flash-attention backward (sm_100a; packed varlen, causal or full, GQA, head_dim 128 or 64).
+// dK / dV of flash-attention backward (sm_100a; packed varlen, causal or full, GQA, head_dim 64;
+// head_dim 128: attn_bwd_hd128.cu).
 //
 // One CTA owns a 64-row key/value tile of one KV head and walks every query tile (128 rows) of
 // every query head of the group that can see it.  Per step four tcgen05 GEMM groups:
 //     S   = Q K^T            (128 x 64,  K = d)        dP  = dO V^T        (128 x 64,  K = d)
-//     dV^T += dO^T P         (128 x 64,  K = q rows)   dK^T += Q^T dS      (128 x 64,  K = q rows)
+//     dV^T += dO^T P         (64 x 64,  K = q rows)    dK^T += Q^T dS      (64 x 64,  K = q rows)
 // dV^T / dK^T stay in TMEM for the CTA's lifetime (d on the lanes); transposed operands are MN-major
 // descriptors over the TMA-written tiles.  dQ is produced by attn_bwd_dq.cu.
 //
@@ -26,36 +27,28 @@ constexpr int ROW_THREADS = 256;
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0;        // + 128 * buf
 constexpr int COL_DP = 64;      // + 128 * buf
-constexpr int COL_DV = 256, COL_DK = 320;
+constexpr int COL_DV = 256;     // dV^T, and 64 lanes and columns on dK^T
 constexpr int KV_CHUNK_BYTES = BKV * 128;
 constexpr int Q_CHUNK_BYTES = BQ * 128;
 constexpr int PS_BYTES = BQ * BKV * 2;        // 16 KB : [128 q rows][64 kv = 128 B]
 
-// Shared-memory layout by head dim.
-//   128: Q ring, dO ring, P buffers, dS buffers.
-//    64: P and dS are sums of two bf16 tiles (see attn_fwd.cu), and dO^T P and Q^T dS come from one
-//        product [dO | Q]^T [P | dS] of 128 x 128: its diagonal blocks are dV^T and dK^T.  A product of
-//        M = 64 would run the tensor core at half rate anyway, so the off-diagonal blocks are free and
-//        one MMA of N = 128 (65 cycles) replaces two of N = 64 (50 cycles each).  dO and Q of a stage,
-//        and P and dS of a buffer, lie next to each other as the two 64-wide chunks of one operand.
-template <int D>
-struct Cfg {
-  static constexpr bool SPLIT = D == 64;
-  static constexpr int CHUNKS = D / 64;
-  static constexpr int KV_TILE_BYTES = CHUNKS * KV_CHUNK_BYTES;
-  static constexpr int Q_TILE_BYTES = CHUNKS * Q_CHUNK_BYTES;
-  static constexpr int SMEM_K = 0;
-  static constexpr int SMEM_V = SMEM_K + KV_TILE_BYTES;
-  static constexpr int SMEM_RING = SMEM_V + KV_TILE_BYTES;              // 2 stages of Q and dO
-  static constexpr int SMEM_PS = SMEM_RING + 4 * Q_TILE_BYTES;          // 2 buffers of P and dS
-  static constexpr int SMEM_BAR = SMEM_PS + (SPLIT ? 8 : 4) * PS_BYTES;
-  static constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
-  __device__ static constexpr int q(int s) { return SPLIT ? SMEM_RING + (2 * s + 1) * Q_TILE_BYTES : SMEM_RING + s * Q_TILE_BYTES; }
-  __device__ static constexpr int dout(int s) { return SPLIT ? SMEM_RING + 2 * s * Q_TILE_BYTES : SMEM_RING + (2 + s) * Q_TILE_BYTES; }
-  __device__ static constexpr int pr(int s) { return SPLIT ? SMEM_PS + 4 * s * PS_BYTES : SMEM_PS + s * PS_BYTES; }
-  __device__ static constexpr int ds(int s) { return SPLIT ? SMEM_PS + (4 * s + 1) * PS_BYTES : SMEM_PS + (2 + s) * PS_BYTES; }
-  static constexpr int REST = 2 * PS_BYTES;   // from a high part to its remainder
-};
+constexpr int D = 64;
+// P and dS are sums of two bf16 tiles (see attn_fwd.cu), and dO^T P and Q^T dS come from one product
+// [dO | Q]^T [P | dS] of 128 x 128: its diagonal blocks are dV^T and dK^T.  A product of M = 64 would run the
+// tensor core at half rate anyway, so the off-diagonal blocks are free and one MMA of N = 128 (65 cycles)
+// replaces two of N = 64 (50 cycles each).  dO and Q of a stage, and P and dS of a buffer, lie next to each
+// other as the two 64-wide chunks of one operand.
+constexpr int SMEM_K = 0;
+constexpr int SMEM_V = SMEM_K + KV_CHUNK_BYTES;
+constexpr int SMEM_RING = SMEM_V + KV_CHUNK_BYTES;                    // 2 stages of dO and Q
+constexpr int SMEM_PS = SMEM_RING + 4 * Q_CHUNK_BYTES;                // 2 buffers of P, dS and their remainders
+constexpr int SMEM_BAR = SMEM_PS + 8 * PS_BYTES;
+constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
+constexpr int REST = 2 * PS_BYTES;                                    // from a high part to its remainder
+__device__ constexpr int at_do(int s) { return SMEM_RING + 2 * s * Q_CHUNK_BYTES; }
+__device__ constexpr int at_q(int s) { return at_do(s) + Q_CHUNK_BYTES; }
+__device__ constexpr int at_p(int b) { return SMEM_PS + 4 * b * PS_BYTES; }
+__device__ constexpr int at_ds(int b) { return at_p(b) + PS_BYTES; }
 
 struct Params {
   const float* lse;     // [Hq, T]
@@ -64,11 +57,9 @@ struct Params {
   __nv_bfloat16* dv;    // [Tk, Hkv, D] with token stride lddv
   long long lddv;
   const int* cu_seqlens;
-  const int* k_starts;
   int num_seqs;
   int T, Hq, Hkv;
   int causal;
-  int window;
   float scale, scale_log2;
   int* status;
 };
@@ -83,13 +74,10 @@ struct __align__(8) Barriers {
   int abort_flag;
 };
 
-template <int D>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                     const Params p) {
-  using C = Cfg<D>;
-  constexpr int KV_TILE_BYTES = C::KV_TILE_BYTES, Q_TILE_BYTES = C::Q_TILE_BYTES;
   const int tile_id = blockIdx.x;
   int seq = -1, kt = 0, seq_start = 0, seq_len = 0;
   {
@@ -105,22 +93,18 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     }
   }
   if (seq < 0) return;
-  const int k_start = p.k_starts ? p.k_starts[seq] : seq_start;
-  if (k_start < 0) return;  // this query block takes no part in the call
   const int kv_head = blockIdx.y;
   const int G = p.Hq / p.Hkv;
   const int kv0 = kt * BKV;                         // position inside the sequence
   const int n_q_tiles = (seq_len + BQ - 1) / BQ;
   const int qt0 = p.causal ? kv0 / BQ : 0;           // first query tile that sees this KV tile
-  // last query that sees key k under a window is k + window - 1
-  const int qt_end = p.window > 0 ? min(n_q_tiles, (kv0 + BKV + p.window - 2) / BQ + 1) : n_q_tiles;
-  const int per_head = max(0, qt_end - qt0);
+  const int per_head = n_q_tiles - qt0;
   const int n_steps = per_head * G;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~(uintptr_t)1023);
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + C::SMEM_BAR);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + SMEM_BAR);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -155,13 +139,10 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------------
     if (lane == 0) {
-      const int tok = k_start + kv0;
-      mbar_expect_tx(&bars->kv_full, 2 * KV_TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::CHUNKS; ++c) {
-        tma_load_3d(smem + C::SMEM_K + c * KV_CHUNK_BYTES, &tmap_k, &bars->kv_full, c * 64, kv_head, tok);
-        tma_load_3d(smem + C::SMEM_V + c * KV_CHUNK_BYTES, &tmap_v, &bars->kv_full, c * 64, kv_head, tok);
-      }
+      const int tok = seq_start + kv0;
+      mbar_expect_tx(&bars->kv_full, 2 * KV_CHUNK_BYTES);
+      tma_load_3d(smem + SMEM_K, &tmap_k, &bars->kv_full, 0, kv_head, tok);
+      tma_load_3d(smem + SMEM_V, &tmap_v, &bars->kv_full, 0, kv_head, tok);
       bool ok = true;
       int issued = 0;
       for (int t = 0; t < n_steps && ok; ++t) {
@@ -173,12 +154,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           ok = false;
           break;
         }
-        mbar_expect_tx(&bars->q_full[s], 2 * Q_TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::CHUNKS; ++c) {
-          tma_load_3d(smem + C::q(s) + c * Q_CHUNK_BYTES, &tmap_q, &bars->q_full[s], c * 64, head, qtok);
-          tma_load_3d(smem + C::dout(s) + c * Q_CHUNK_BYTES, &tmap_do, &bars->q_full[s], c * 64, head, qtok);
-        }
+        mbar_expect_tx(&bars->q_full[s], 2 * Q_CHUNK_BYTES);
+        tma_load_3d(smem + at_q(s), &tmap_q, &bars->q_full[s], 0, head, qtok);
+        tma_load_3d(smem + at_do(s), &tmap_do, &bars->q_full[s], 0, head, qtok);
         issued = t + 1;
       }
       if (!ok) {
@@ -194,11 +172,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     // ------------------------------- MMA issuer ---------------------------------------
     if (lane == 0) {
       constexpr uint32_t idesc_s = xb_idesc(1, 1, BQ, BKV, 0, 0);   // Q K^T, dO V^T
-      constexpr uint32_t idesc_t = xb_idesc(1, 1, 128, C::SPLIT ? 2 * BKV : BKV, 1, 1);  // dO^T P, Q^T dS (both MN-major)
+      constexpr uint32_t idesc_t = xb_idesc(1, 1, 2 * D, 2 * BKV, 1, 1);   // [dO | Q]^T [P | dS], both MN-major
       constexpr uint64_t kmaj = xb_smem_desc_base_sw128(16, 1024);
       constexpr uint64_t mn_q = xb_smem_desc_base_sw128(Q_CHUNK_BYTES, 1024);    // Q/dO as A^T
       constexpr uint64_t mn_ps = xb_smem_desc_base_sw128(PS_BYTES, 1024);        // P/dS as B (1 chunk)
-      const uint32_t sk = xb_smem_u32(smem + C::SMEM_K), sv = xb_smem_u32(smem + C::SMEM_V);
+      const uint32_t sk = xb_smem_u32(smem + SMEM_K), sv = xb_smem_u32(smem + SMEM_V);
       bool ok = mbar_wait(&bars->kv_full, 0, abort_flag, p.status, XB_K_ATTN_BWD, 810);
       auto issue_sdp = [&](int t) -> bool {
         const int s = t & 1;
@@ -206,19 +184,17 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         if (!mbar_wait(&bars->q_full[s], ph, abort_flag, p.status, XB_K_ATTN_BWD, 820 + s)) return false;
         if (!mbar_wait(&bars->sdp_empty[s], ph ^ 1, abort_flag, p.status, XB_K_ATTN_BWD, 830 + s)) return false;
         tc_fence_after();
-        const uint32_t sq = xb_smem_u32(smem + C::q(s));
-        const uint32_t sdo = xb_smem_u32(smem + C::dout(s));
+        const uint32_t sq = xb_smem_u32(smem + at_q(s));
+        const uint32_t sdo = xb_smem_u32(smem + at_do(s));
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t a_off = (k >> 2) * Q_CHUNK_BYTES + (k & 3) * 32;
-          const uint32_t b_off = (k >> 2) * KV_CHUNK_BYTES + (k & 3) * 32;
+          const uint32_t a_off = k * 32, b_off = k * 32;
           tc_mma_f16_ss(tmem_base + COL_S + 128 * s, xb_smem_desc(kmaj, sq + a_off),
                         xb_smem_desc(kmaj, sk + b_off), idesc_s, k > 0 ? 1u : 0u);
         }
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t a_off = (k >> 2) * Q_CHUNK_BYTES + (k & 3) * 32;
-          const uint32_t b_off = (k >> 2) * KV_CHUNK_BYTES + (k & 3) * 32;
+          const uint32_t a_off = k * 32, b_off = k * 32;
           tc_mma_f16_ss(tmem_base + COL_DP + 128 * s, xb_smem_desc(kmaj, sdo + a_off),
                         xb_smem_desc(kmaj, sv + b_off), idesc_s, k > 0 ? 1u : 0u);
         }
@@ -236,30 +212,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           break;
         }
         tc_fence_after();
-        const uint32_t sdo = xb_smem_u32(smem + C::dout(s));
-        const uint32_t spp = xb_smem_u32(smem + C::pr(s));
+        const uint32_t sdo = xb_smem_u32(smem + at_do(s));
+        const uint32_t spp = xb_smem_u32(smem + at_p(s));
         // dV^T += dO^T P ; dK^T += Q^T dS   (reduction over the 128 query rows, 16 per MMA)
-        if constexpr (C::SPLIT) {
 #pragma unroll
-          for (int k = 0; k < BQ / 16; ++k) {
-            tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
-                          xb_smem_desc(mn_ps, spp + k * 2048), idesc_t, (t > 0 || k > 0) ? 1u : 0u);
-            tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
-                          xb_smem_desc(mn_ps, spp + C::REST + k * 2048), idesc_t, 1u);
-          }
-        } else {
-          const uint32_t sq = xb_smem_u32(smem + C::q(s));
-          const uint32_t sds = xb_smem_u32(smem + C::ds(s));
-#pragma unroll
-          for (int k = 0; k < BQ / 16; ++k) {
-            tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
-                          xb_smem_desc(mn_ps, spp + k * 2048), idesc_t, (t > 0 || k > 0) ? 1u : 0u);
-          }
-#pragma unroll
-          for (int k = 0; k < BQ / 16; ++k) {
-            tc_mma_f16_ss(tmem_base + COL_DK, xb_smem_desc(mn_q, sq + k * 2048),
-                          xb_smem_desc(mn_ps, sds + k * 2048), idesc_t, (t > 0 || k > 0) ? 1u : 0u);
-          }
+        for (int k = 0; k < BQ / 16; ++k) {
+          tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
+                        xb_smem_desc(mn_ps, spp + k * 2048), idesc_t, (t > 0 || k > 0) ? 1u : 0u);
+          tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
+                        xb_smem_desc(mn_ps, spp + REST + k * 2048), idesc_t, 1u);
         }
         tc_commit(&bars->q_empty[s]);
         tc_commit(&bars->pds_free[s]);
@@ -314,8 +275,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         // dS here is P o (dP - delta); the softmax scale is applied once, to dK, at the end.
         // Tiles entirely below the diagonal and inside the sequence (the common case) need no mask.
         const int q_lo = (qt0 + t % per_head) * BQ;
-        const bool no_mask = (q_lo + BQ <= seq_len) && (kv0 + BKV <= seq_len) && (!p.causal || kv0 + BKV - 1 <= q_lo) &&
-                             (p.window <= 0 || kv0 >= q_lo + BQ - p.window);
+        const bool no_mask = (q_lo + BQ <= seq_len) && (kv0 + BKV <= seq_len) && (!p.causal || kv0 + BKV - 1 <= q_lo);
         if (no_mask) {                               // CTA-uniform
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -326,10 +286,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         } else {
           const int lim = p.causal ? min(seq_len - 1, q_pos) : seq_len - 1;  // last visible kv position
           const int nvis = row_valid ? (lim - (kv0 + half * 32) + 1) : 0;     // visible columns of this thread
-          const int nlo = p.window > 0 ? (q_pos - p.window + 1) - (kv0 + half * 32) : 0;
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const float pe = (i < nvis && i >= nlo) ? xb_ex2(fmaf(__uint_as_float(a[i]), p.scale_log2, -lse)) : 0.f;
+            const float pe = i < nvis ? xb_ex2(fmaf(__uint_as_float(a[i]), p.scale_log2, -lse)) : 0.f;
             pv[i] = pe;
             ds[i] = pe * (__uint_as_float(b[i]) - delta);
           }
@@ -341,8 +300,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         break;
       }
       // P and dS rows (bf16) -> shared memory, [128 rows][128 B] with the 128B swizzle
-      uint8_t* sp = smem + C::pr(s) + r * 128;
-      uint8_t* sd = smem + C::ds(s) + r * 128;
+      uint8_t* sp = smem + at_p(s) + r * 128;
+      uint8_t* sd = smem + at_ds(s) + r * 128;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint4 v, w;
@@ -357,19 +316,17 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         const int slot = (half * 4 + c) ^ (r & 7);
         *reinterpret_cast<uint4*>(sp + slot * 16) = v;
         *reinterpret_cast<uint4*>(sd + slot * 16) = w;
-        if constexpr (C::SPLIT) {
-          uint4 v2, w2;
-          v2.x = pack_bf16x2_rest(pv[c * 8 + 0], pv[c * 8 + 1], v.x);
-          v2.y = pack_bf16x2_rest(pv[c * 8 + 2], pv[c * 8 + 3], v.y);
-          v2.z = pack_bf16x2_rest(pv[c * 8 + 4], pv[c * 8 + 5], v.z);
-          v2.w = pack_bf16x2_rest(pv[c * 8 + 6], pv[c * 8 + 7], v.w);
-          w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
-          w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
-          w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
-          w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
-          *reinterpret_cast<uint4*>(sp + C::REST + slot * 16) = v2;
-          *reinterpret_cast<uint4*>(sd + C::REST + slot * 16) = w2;
-        }
+        uint4 v2, w2;
+        v2.x = pack_bf16x2_rest(pv[c * 8 + 0], pv[c * 8 + 1], v.x);
+        v2.y = pack_bf16x2_rest(pv[c * 8 + 2], pv[c * 8 + 3], v.y);
+        v2.z = pack_bf16x2_rest(pv[c * 8 + 4], pv[c * 8 + 5], v.z);
+        v2.w = pack_bf16x2_rest(pv[c * 8 + 6], pv[c * 8 + 7], v.w);
+        w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
+        w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
+        w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
+        w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
+        *reinterpret_cast<uint4*>(sp + REST + slot * 16) = v2;
+        *reinterpret_cast<uint4*>(sd + REST + slot * 16) = w2;
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -381,44 +338,23 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       tc_fence_after();
       // dV^T / dK^T: this thread holds feature d = r for 32 of the 64 kv rows of the tile.  For a
       // fixed kv row the 32 lanes of a warp write 32 consecutive features.
-      if constexpr (C::SPLIT) {
-        // lanes 0..63 of the columns 0..63 are dV^T, lanes 64..127 of the columns 64..127 are dK^T
-        const bool is_dk = q4 >= 2;                // warp-uniform
-        uint32_t a[32];
-        if (n_steps > 0) {
-          tmem_ld_32x32(tmem_base + lane_addr + COL_DV + (is_dk ? BKV : 0) + half * 32, a);
-          tc_wait_ld();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) a[i] = 0;
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int kv_pos = kv0 + half * 32 + i;
-          if (kv_pos < seq_len) {
-            const size_t tok = (size_t)k_start + kv_pos;
-            if (is_dk) p.dk[(tok * p.Hkv + kv_head) * D + r - 64] = __uint_as_float(a[i]) * p.scale;
-            else p.dv[tok * p.lddv + (size_t)kv_head * D + r] = __float2bfloat16(__uint_as_float(a[i]));
-          }
-        }
+      // lanes 0..63 of the columns 0..63 are dV^T, lanes 64..127 of the columns 64..127 are dK^T
+      const bool is_dk = q4 >= 2;                // warp-uniform
+      uint32_t a[32];
+      if (n_steps > 0) {
+        tmem_ld_32x32(tmem_base + lane_addr + COL_DV + (is_dk ? BKV : 0) + half * 32, a);
+        tc_wait_ld();
       } else {
-        uint32_t a[32], b[32];
-        if (n_steps > 0) {                          // CTA-uniform
-          tmem_ld_32x32(tmem_base + lane_addr + COL_DV + half * 32, a);
-          tmem_ld_32x32(tmem_base + lane_addr + COL_DK + half * 32, b);
-          tc_wait_ld();
-        } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) { a[i] = 0; b[i] = 0; }
-        }
+        for (int i = 0; i < 32; ++i) a[i] = 0;
+      }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int kv_pos = kv0 + half * 32 + i;
-          if (kv_pos < seq_len) {
-            const size_t tok = (size_t)k_start + kv_pos;
-            p.dv[tok * p.lddv + (size_t)kv_head * D + r] = __float2bfloat16(__uint_as_float(a[i]));
-            p.dk[(tok * p.Hkv + kv_head) * D + r] = __uint_as_float(b[i]) * p.scale;
-          }
+      for (int i = 0; i < 32; ++i) {
+        const int kv_pos = kv0 + half * 32 + i;
+        if (kv_pos < seq_len) {
+          const size_t tok = (size_t)seq_start + kv_pos;
+          if (is_dk) p.dk[(tok * p.Hkv + kv_head) * D + r - 64] = __uint_as_float(a[i]) * p.scale;
+          else p.dv[tok * p.lddv + (size_t)kv_head * D + r] = __float2bfloat16(__uint_as_float(a[i]));
         }
       }
     }
@@ -432,44 +368,24 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   }
 }
 
-template <int D>
-static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                  const Params& p, int tiles, cudaStream_t stream) {
-  static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!configured[dev & 63]) {
-    if (cudaFuncSetAttribute(attn_bwd_dkv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Cfg<D>::SMEM_BYTES) != cudaSuccess)
-      return -10;
-    configured[dev & 63] = true;
-  }
-  attn_bwd_dkv_kernel<D><<<dim3(tiles, p.Hkv), NUM_THREADS, Cfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
-
 }  // namespace xb_attn_dkv_ns
 
-// dk fp32 [Tk, Hkv, D], dv bf16 [Tk, Hkv, D] (token stride lddv) for the K/V rows covered by the
-// call; lse / delta [Hq, T] must be ready.  max_tiles bounds the number of 64-row key tiles (0 =
-// derive from T).
-XB_API int xb_attn_bwd_dkv(const void* q, const void* k, const void* v, const void* dout, const float* lse,
-                           const float* delta, float* dk, void* dv, const int* cu_seqlens, const int* k_starts,
-                           long long ldq, long long ldk, long long ldv, long long lddo, long long lddv,
-                           int num_seqs, int T, int Tk, int Hq, int Hkv, int D, int causal, float scale,
-                           int max_tiles, void* stream) {
+// dk fp32 [T, Hkv, 64], dv bf16 [T, Hkv, 64] (token stride lddv); lse / delta [Hq, T] must be ready.  Called by
+// xb_attn_bwd_hd64.
+int xb_attn_dkv_hd64(const void* q, const void* k, const void* v, const void* dout, const float* lse,
+                     const float* delta, float* dk, void* dv, const int* cu_seqlens, long long ldq, long long ldk,
+                     long long ldv, long long lddo, long long lddv, int num_seqs, int T, int Hq, int Hkv, int causal,
+                     float scale, cudaStream_t stream) {
   using namespace xb_attn_dkv_ns;
-  if (D != 128 && D != 64) return -1;
-  if (T <= 0 || num_seqs <= 0) return 0;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || Hq % Hkv) return -1;
   CUtensorMap tq, tk, tv, tdo;
   if (xb_make_tmap_3d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hq, D, ldq, D, BQ, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -2;
-  if (xb_make_tmap_3d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, Hkv, D, ldk, D, BKV, 1, 64,
+  if (xb_make_tmap_3d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hkv, D, ldk, D, BKV, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
-  if (xb_make_tmap_3d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, Hkv, D, ldv, D, BKV, 1, 64,
+  if (xb_make_tmap_3d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hkv, D, ldv, D, BKV, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -4;
   if (xb_make_tmap_3d(&tdo, dout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hq, D, lddo, D, BQ, 1, 64,
@@ -477,11 +393,19 @@ XB_API int xb_attn_bwd_dkv(const void* q, const void* k, const void* v, const vo
     return -5;
   Params p;
   p.lse = lse; p.delta = delta; p.dk = dk; p.dv = (__nv_bfloat16*)dv; p.lddv = lddv;
-  p.cu_seqlens = cu_seqlens; p.k_starts = k_starts; p.num_seqs = num_seqs;
-  p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1; p.window = causal >> 1; p.scale = scale;
+  p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs;
+  p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1; p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = xb_status_ptr();
-  const int tiles = max_tiles > 0 ? max_tiles : (T + BKV - 1) / BKV + num_seqs;
-  return D == 128 ? launch<128>(tq, tk, tv, tdo, p, tiles, (cudaStream_t)stream)
-                  : launch<64>(tq, tk, tv, tdo, p, tiles, (cudaStream_t)stream);
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    if (cudaFuncSetAttribute(attn_bwd_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+      return -10;
+    configured[dev & 63] = true;
+  }
+  const int tiles = (T + BKV - 1) / BKV + num_seqs;
+  attn_bwd_dkv_kernel<<<dim3(tiles, Hkv), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

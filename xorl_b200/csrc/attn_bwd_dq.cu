@@ -1,16 +1,14 @@
 // dQ of flash-attention backward without atomics (sm_100a; packed varlen, causal or full, GQA,
-// head_dim 128 or 64).
+// head_dim 64; head_dim 128: attn_bwd_hd128.cu).
 //
 // One CTA owns a 128-row query tile of one query head and walks the 64-row key/value tiles it can
 // see.  Per step three tcgen05 GEMM groups:
 //     S  = Q K^T   (128 x 64, K = d)      dP = dO V^T   (128 x 64, K = d)
-//     dQ += dS K   (128 x 128, K = 64 kv rows)          dS = P o (dP - delta) * scale
+//     dQ += dS K   (128 x 64, K = 64 kv rows)           dS = P o (dP - delta) * scale
 // dQ stays in TMEM for the CTA's lifetime and is written once, with plain stores: every (row,
 // head) of dQ belongs to exactly one CTA.  S / dP are double-buffered in TMEM and dS in shared
 // memory, so the MMAs of step j+1 run while the row threads turn step j into dS.
-// Together with the dK/dV kernel (attn_bwd.cu with its dQ part switched off) this replaces the
-// single kernel that added 128 x 128 fp32 dQ partials to global memory with vector reductions at
-// every step; the price is a second evaluation of S and dP.
+// Together with the dK / dV kernel this needs no atomics; the price is a second evaluation of S and dP.
 //   warp 0 : TMA producer (Q, dO once; K, V three-stage ring)     warp 1 : MMA issuer
 //   warps 2..9 : two threads per query row (32 of the 64 key columns each), two warps per scheduler
 //                so that dependent-issue latency of the softmax arithmetic is hidden
@@ -31,33 +29,24 @@ constexpr int KV_CHUNK_BYTES = BKV * 128;
 constexpr int Q_CHUNK_BYTES = BQ * 128;
 constexpr int DS_BYTES = BQ * BKV * 2;         // 16 KB : [128 q rows][64 kv = 128 B]
 
-// Shared-memory layout by head dim; at 64, dS is the sum of two bf16 tiles (see attn_fwd.cu).
-template <int D>
-struct Cfg {
-  static constexpr bool SPLIT = D == 64;
-  static constexpr int CHUNKS = D / 64;
-  static constexpr int KV_TILE_BYTES = CHUNKS * KV_CHUNK_BYTES;
-  static constexpr int Q_TILE_BYTES = CHUNKS * Q_CHUNK_BYTES;
-  static constexpr int SMEM_Q = 0;
-  static constexpr int SMEM_DO = SMEM_Q + Q_TILE_BYTES;
-  static constexpr int SMEM_KV = SMEM_DO + Q_TILE_BYTES;                 // NS x (K tile, V tile)
-  static constexpr int SMEM_DS = SMEM_KV + NS * 2 * KV_TILE_BYTES;       // 2 buffers (high part, remainder)
-  static constexpr int DS_BUF = (SPLIT ? 2 : 1) * DS_BYTES;
-  static constexpr int SMEM_BAR = SMEM_DS + 2 * DS_BUF;
-  static constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
-};
+constexpr int D = 64;
+// dS is the sum of two bf16 tiles (see attn_fwd.cu)
+constexpr int SMEM_Q = 0;
+constexpr int SMEM_DO = SMEM_Q + Q_CHUNK_BYTES;
+constexpr int SMEM_KV = SMEM_DO + Q_CHUNK_BYTES;                  // NS x (K tile, V tile)
+constexpr int SMEM_DS = SMEM_KV + NS * 2 * KV_CHUNK_BYTES;        // 2 buffers of high part and remainder
+constexpr int DS_BUF = 2 * DS_BYTES;
+constexpr int SMEM_BAR = SMEM_DS + 2 * DS_BUF;
+constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
 
 struct Params {
   const float* lse;     // [Hq, T]
   const float* delta;   // [Hq, T]
   float* dq;            // [T, Hq, D] fp32
   const int* cu_seqlens;
-  const int* k_starts;
   int num_seqs;
   int T, Hq, Hkv;
   int causal;
-  int window;
-  int accumulate;       // dq already holds partial sums of earlier key blocks: add to it
   float scale, scale_log2;
   int* status;
 };
@@ -72,13 +61,10 @@ struct __align__(8) Barriers {
   int abort_flag;
 };
 
-template <int D>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                    const Params p) {
-  using C = Cfg<D>;
-  constexpr int KV_TILE_BYTES = C::KV_TILE_BYTES, Q_TILE_BYTES = C::Q_TILE_BYTES;
   // tiles are numbered so that, inside a sequence, the last (most expensive under a causal mask)
   // query tile comes first
   const int tile_id = blockIdx.x;
@@ -96,20 +82,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
   }
   if (seq < 0) return;
-  const int k_start = p.k_starts ? p.k_starts[seq] : seq_start;
-  if (k_start < 0) return;
   const int head = blockIdx.y;
   const int kv_head = head / (p.Hq / p.Hkv);
   const int q0 = qt * BQ;
   const int n_kv_all = (seq_len + BKV - 1) / BKV;
   const int n_hi = p.causal ? min(n_kv_all, (min(q0 + BQ, seq_len) - 1) / BKV + 1) : n_kv_all;
-  const int jt0 = p.window > 0 ? max(0, q0 - p.window + 1) / BKV : 0;   // first key tile inside the window
-  const int n_steps = max(0, n_hi - jt0);
+  const int n_steps = n_hi;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~(uintptr_t)1023);
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + C::SMEM_BAR);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + SMEM_BAR);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -147,12 +130,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // ------------------------------- TMA producer -------------------------------------
     if (lane == 0) {
       const int qtok = seq_start + q0;
-      mbar_expect_tx(&bars->q_full, 2 * Q_TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::CHUNKS; ++c) {
-        tma_load_3d(smem + C::SMEM_Q + c * Q_CHUNK_BYTES, &tmap_q, &bars->q_full, c * 64, head, qtok);
-        tma_load_3d(smem + C::SMEM_DO + c * Q_CHUNK_BYTES, &tmap_do, &bars->q_full, c * 64, head, qtok);
-      }
+      mbar_expect_tx(&bars->q_full, 2 * Q_CHUNK_BYTES);
+      tma_load_3d(smem + SMEM_Q, &tmap_q, &bars->q_full, 0, head, qtok);
+      tma_load_3d(smem + SMEM_DO, &tmap_do, &bars->q_full, 0, head, qtok);
       bool ok = true;
       int issued = 0;
       for (int j = 0; j < n_steps && ok; ++j) {
@@ -162,15 +142,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           ok = false;
           break;
         }
-        const int tok = k_start + (jt0 + j) * BKV;
-        uint8_t* sk = smem + C::SMEM_KV + s * 2 * KV_TILE_BYTES;
-        uint8_t* sv = sk + KV_TILE_BYTES;
-        mbar_expect_tx(&bars->kv_full[s], 2 * KV_TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::CHUNKS; ++c) {
-          tma_load_3d(sk + c * KV_CHUNK_BYTES, &tmap_k, &bars->kv_full[s], c * 64, kv_head, tok);
-          tma_load_3d(sv + c * KV_CHUNK_BYTES, &tmap_v, &bars->kv_full[s], c * 64, kv_head, tok);
-        }
+        const int tok = seq_start + j * BKV;
+        uint8_t* sk = smem + SMEM_KV + s * 2 * KV_CHUNK_BYTES;
+        uint8_t* sv = sk + KV_CHUNK_BYTES;
+        mbar_expect_tx(&bars->kv_full[s], 2 * KV_CHUNK_BYTES);
+        tma_load_3d(sk, &tmap_k, &bars->kv_full[s], 0, kv_head, tok);
+        tma_load_3d(sv, &tmap_v, &bars->kv_full[s], 0, kv_head, tok);
         issued = j + 1;
       }
       if (!ok) {
@@ -190,7 +167,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       constexpr uint32_t idesc_q = xb_idesc(1, 1, BQ, D, 0, 1);     // dS K (K tile MN-major)
       constexpr uint64_t kmaj = xb_smem_desc_base_sw128(16, 1024);
       constexpr uint64_t mn_kv = xb_smem_desc_base_sw128(KV_CHUNK_BYTES, 1024);
-      const uint32_t sq = xb_smem_u32(smem + C::SMEM_Q), sdo = xb_smem_u32(smem + C::SMEM_DO);
+      const uint32_t sq = xb_smem_u32(smem + SMEM_Q), sdo = xb_smem_u32(smem + SMEM_DO);
       bool ok = mbar_wait(&bars->q_full, 0, abort_flag, p.status, XB_K_ATTN_BWD, 600);
       auto issue_sdp = [&](int j) -> bool {
         const int s = j % NS, b = j & 1;
@@ -199,19 +176,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         if (!mbar_wait(&bars->sdp_empty[b], ((j >> 1) & 1) ^ 1, abort_flag, p.status, XB_K_ATTN_BWD, 620 + b))
           return false;
         tc_fence_after();
-        const uint32_t sk = xb_smem_u32(smem + C::SMEM_KV + s * 2 * KV_TILE_BYTES);
-        const uint32_t sv = sk + KV_TILE_BYTES;
+        const uint32_t sk = xb_smem_u32(smem + SMEM_KV + s * 2 * KV_CHUNK_BYTES);
+        const uint32_t sv = sk + KV_CHUNK_BYTES;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t a_off = (k >> 2) * Q_CHUNK_BYTES + (k & 3) * 32;
-          const uint32_t b_off = (k >> 2) * KV_CHUNK_BYTES + (k & 3) * 32;
+          const uint32_t a_off = k * 32, b_off = k * 32;
           tc_mma_f16_ss(tmem_base + COL_S + 128 * b, xb_smem_desc(kmaj, sq + a_off),
                         xb_smem_desc(kmaj, sk + b_off), idesc_s, k > 0 ? 1u : 0u);
         }
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t a_off = (k >> 2) * Q_CHUNK_BYTES + (k & 3) * 32;
-          const uint32_t b_off = (k >> 2) * KV_CHUNK_BYTES + (k & 3) * 32;
+          const uint32_t a_off = k * 32, b_off = k * 32;
           tc_mma_f16_ss(tmem_base + COL_DP + 128 * b, xb_smem_desc(kmaj, sdo + a_off),
                         xb_smem_desc(kmaj, sv + b_off), idesc_s, k > 0 ? 1u : 0u);
         }
@@ -229,15 +204,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           break;
         }
         tc_fence_after();
-        const uint32_t sk = xb_smem_u32(smem + C::SMEM_KV + s * 2 * KV_TILE_BYTES);
-        const uint32_t sds = xb_smem_u32(smem + C::SMEM_DS + b * C::DS_BUF);
+        const uint32_t sk = xb_smem_u32(smem + SMEM_KV + s * 2 * KV_CHUNK_BYTES);
+        const uint32_t sds = xb_smem_u32(smem + SMEM_DS + b * DS_BUF);
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k) {
           tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + k * 32),
                         xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, (j > 0 || k > 0) ? 1u : 0u);
-          if constexpr (C::SPLIT)
-            tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + DS_BYTES + k * 32),
-                          xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, 1u);
+          tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + DS_BYTES + k * 32),
+                        xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, 1u);
         }
         tc_commit(&bars->kv_empty[s]);   // K_j (and V_j, read earlier) no longer needed
         tc_commit(&bars->ds_free[b]);
@@ -272,26 +246,24 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
       tc_fence_after();
       float ds[32];
-      const int kv0 = (jt0 + j) * BKV + half * 32;
+      const int kv0 = j * BKV + half * 32;
       {
         uint32_t a[32], d2[32];
         tmem_ld_32x32(tmem_base + lane_addr + COL_S + 128 * b + half * 32, a);
         tmem_ld_32x32(tmem_base + lane_addr + COL_DP + 128 * b + half * 32, d2);
         tc_wait_ld();
         // dS here is P o (dP - delta); the softmax scale is applied once, to dQ, at the end
-        const int kt = (jt0 + j) * BKV;
-        const bool no_mask = (q0 + BQ <= seq_len) && (kt + BKV <= seq_len) && (!p.causal || kt + BKV - 1 <= q0) &&
-                             (p.window <= 0 || kt >= q0 + BQ - p.window);     // CTA-uniform
+        const int kt = j * BKV;
+        const bool no_mask = (q0 + BQ <= seq_len) && (kt + BKV <= seq_len) && (!p.causal || kt + BKV - 1 <= q0);   // CTA-uniform
         if (no_mask) {
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             ds[i] = xb_ex2(fmaf(__uint_as_float(a[i]), p.scale_log2, -lse)) * (__uint_as_float(d2[i]) - delta);
         } else {
           const int nvis = row_valid ? (lim - kv0 + 1) : 0;
-          const int nlo = p.window > 0 ? (q_pos - p.window + 1) - kv0 : 0;   // columns below it are outside the window
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            ds[i] = (i < nvis && i >= nlo) ? xb_ex2(fmaf(__uint_as_float(a[i]), p.scale_log2, -lse)) *
+            ds[i] = i < nvis ? xb_ex2(fmaf(__uint_as_float(a[i]), p.scale_log2, -lse)) *
                                    (__uint_as_float(d2[i]) - delta)
                              : 0.f;
         }
@@ -303,7 +275,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         ok = false;
         break;
       }
-      uint8_t* sd = smem + C::SMEM_DS + b * C::DS_BUF + r * 128;
+      uint8_t* sd = smem + SMEM_DS + b * DS_BUF + r * 128;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int c16 = half * 4 + c;
@@ -313,14 +285,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         w.z = pack_bf16x2(ds[c * 8 + 4], ds[c * 8 + 5]);
         w.w = pack_bf16x2(ds[c * 8 + 6], ds[c * 8 + 7]);
         *reinterpret_cast<uint4*>(sd + ((c16 ^ (r & 7)) * 16)) = w;
-        if constexpr (C::SPLIT) {
-          uint4 w2;
-          w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
-          w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
-          w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
-          w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
-          *reinterpret_cast<uint4*>(sd + DS_BYTES + ((c16 ^ (r & 7)) * 16)) = w2;
-        }
+        uint4 w2;
+        w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
+        w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
+        w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
+        w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
+        *reinterpret_cast<uint4*>(sd + DS_BYTES + ((c16 ^ (r & 7)) * 16)) = w2;
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -349,10 +319,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             float4 o = make_float4(__uint_as_float(a[i]) * p.scale, __uint_as_float(a[i + 1]) * p.scale,
                                    __uint_as_float(a[i + 2]) * p.scale, __uint_as_float(a[i + 3]) * p.scale);
             float4* d4 = reinterpret_cast<float4*>(dst + c * 32 + i);
-            if (p.accumulate) {
-              const float4 old = *d4;
-              o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-            }
             *d4 = o;
           }
         }
@@ -368,54 +334,43 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   }
 }
 
-template <int D>
-static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                  const Params& p, int tiles, cudaStream_t stream) {
-  static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!configured[dev & 63]) {
-    if (cudaFuncSetAttribute(attn_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Cfg<D>::SMEM_BYTES) != cudaSuccess)
-      return -10;
-    configured[dev & 63] = true;
-  }
-  attn_bwd_dq_kernel<D><<<dim3(tiles, p.Hq), NUM_THREADS, Cfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
-
 }  // namespace xb_attn_dq_ns
 
-// dq[T, Hq, D] fp32 (= or +=) dS K for every query row; same tensor-map inputs as xb_attn_bwd_ex.
-// max_q_tiles bounds the grid (>= sum over sequences of ceil(len / 128)); 0 = derive from T.
-XB_API int xb_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dout, const float* lse,
-                          const float* delta, float* dq, const int* cu_seqlens, const int* k_starts,
-                          long long ldq, long long ldk, long long ldv, long long lddo, int num_seqs, int T,
-                          int Tk, int Hq, int Hkv, int D, int causal, float scale, int accumulate,
-                          int max_q_tiles, void* stream) {
+// dq fp32 [T, Hq, 64] for every query row of a sequence; lse / delta [Hq, T] must be ready.  Called by
+// xb_attn_bwd_hd64.
+int xb_attn_dq_hd64(const void* q, const void* k, const void* v, const void* dout, const float* lse,
+                    const float* delta, float* dq, const int* cu_seqlens, long long ldq, long long ldk, long long ldv,
+                    long long lddo, int num_seqs, int T, int Hq, int Hkv, int causal, float scale,
+                    cudaStream_t stream) {
   using namespace xb_attn_dq_ns;
-  if (D != 128 && D != 64) return -1;
-  if (T <= 0 || num_seqs <= 0) return 0;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || Hq % Hkv) return -1;
   CUtensorMap tq, tk, tv, tdo;
   if (xb_make_tmap_3d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hq, D, ldq, D, BQ, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -2;
-  if (xb_make_tmap_3d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, Hkv, D, ldk, D, BKV, 1, 64,
+  if (xb_make_tmap_3d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hkv, D, ldk, D, BKV, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
-  if (xb_make_tmap_3d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, Hkv, D, ldv, D, BKV, 1, 64,
+  if (xb_make_tmap_3d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hkv, D, ldv, D, BKV, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -4;
   if (xb_make_tmap_3d(&tdo, dout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hq, D, lddo, D, BQ, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -5;
   Params p;
-  p.lse = lse; p.delta = delta; p.dq = dq; p.cu_seqlens = cu_seqlens; p.k_starts = k_starts;
-  p.num_seqs = num_seqs; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1; p.window = causal >> 1; p.accumulate = accumulate;
+  p.lse = lse; p.delta = delta; p.dq = dq; p.cu_seqlens = cu_seqlens;
+  p.num_seqs = num_seqs; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.status = xb_status_ptr();
-  const int tiles = max_q_tiles > 0 ? max_q_tiles : (T + BQ - 1) / BQ + num_seqs;
-  return D == 128 ? launch<128>(tq, tk, tv, tdo, p, tiles, (cudaStream_t)stream)
-                  : launch<64>(tq, tk, tv, tdo, p, tiles, (cudaStream_t)stream);
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    if (cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
+      return -10;
+    configured[dev & 63] = true;
+  }
+  const int tiles = (T + BQ - 1) / BQ + num_seqs;
+  attn_bwd_dq_kernel<<<dim3(tiles, Hq), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

@@ -1,5 +1,6 @@
 // Flash-attention forward for sm_100a: packed variable-length sequences (cu_seqlens), causal or
-// full, grouped-query heads, head_dim 128 or 64, bf16 in / bf16 out, log-sum-exp saved for backward.
+// full, grouped-query heads, bf16 in / bf16 out, log-sum-exp saved for backward.  The kernel of this file
+// serves head dim 64; head dim 128 runs in attn_fwd_hd128.cu.
 //
 // One CTA per (128-row query tile, query head):
 //   warp 0     : TMA producer   (Q once; K and V tiles in two 2-deep rings)
@@ -24,21 +25,16 @@ constexpr int TMEM_COLS = 512;
 constexpr int S_COL0 = 0, O_COL = 256;
 constexpr int P_BYTES = 2 * CHUNK_BYTES;  // [128 query rows][128 keys]
 
-// Shared-memory layout by head dim.  Head dim 64 carries P as the sum of two bf16 tiles (high part
-// and remainder, about 2^-17 relative): callers of that width had fp32 probabilities before they had
-// this kernel and keep them.  The second P V product costs little there, its N is 64.
-template <int D>
-struct Cfg {
-  static constexpr bool SPLIT = D == 64;
-  static constexpr int CHUNKS = D / 64;
-  static constexpr int TILE_BYTES = CHUNKS * CHUNK_BYTES;
-  static constexpr int SMEM_Q = 0;
-  static constexpr int SMEM_K = SMEM_Q + TILE_BYTES;      // 2 stages
-  static constexpr int SMEM_V = SMEM_K + 2 * TILE_BYTES;  // 2 stages
-  static constexpr int SMEM_P = SMEM_V + 2 * TILE_BYTES;  // high part, then the remainder
-  static constexpr int SMEM_BAR = SMEM_P + (SPLIT ? 2 : 1) * P_BYTES;
-  static constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
-};
+// P enters its product as the sum of two bf16 tiles (high part and remainder, about 2^-17 relative): callers
+// of this width had fp32 probabilities before they had this kernel and keep them.  The second product costs
+// little, its N is 64.
+constexpr int D = 64;
+constexpr int SMEM_Q = 0;
+constexpr int SMEM_K = SMEM_Q + CHUNK_BYTES;      // 2 stages
+constexpr int SMEM_V = SMEM_K + 2 * CHUNK_BYTES;  // 2 stages
+constexpr int SMEM_P = SMEM_V + 2 * CHUNK_BYTES;  // high part, then the remainder
+constexpr int SMEM_BAR = SMEM_P + 2 * P_BYTES;
+constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
 
 struct Params {
   __nv_bfloat16* out;
@@ -46,12 +42,9 @@ struct Params {
   float* out_f32;  // optional [T, Hq, D]: the output before its rounding to bf16
   float* lse;  // [Hq, T]
   const int* cu_seqlens;
-  const int* k_starts;  // optional: first K/V row of every sequence (defaults to cu_seqlens)
   int num_seqs;
   int T, Hq, Hkv;
   int causal;
-  int window;          // > 0: a query sees only keys with q_pos - k_pos < window
-  const float* sinks;  // optional fp32 [Hq]: one more logit per head in the softmax denominator
   float scale_log2;
   int* status;
 };
@@ -66,13 +59,9 @@ struct __align__(8) Barriers {
   int abort_flag;
 };
 
-template <int D>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const Params p) {
-  using C = Cfg<D>;
-  constexpr int TILE_BYTES = C::TILE_BYTES, SMEM_Q = C::SMEM_Q, SMEM_K = C::SMEM_K, SMEM_V = C::SMEM_V,
-                SMEM_P = C::SMEM_P, SMEM_BAR = C::SMEM_BAR;
   // ---- which (sequence, query tile) does this CTA own?  Heavy (late) tiles are scheduled first.
   const int tile_id = (int)gridDim.x - 1 - (int)blockIdx.x;
   int seq = -1, qt = 0, seq_start = 0, seq_len = 0;
@@ -89,15 +78,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
   }
   if (seq < 0) return;  // uniform for the whole CTA, nothing allocated yet
-  const int k_start = p.k_starts ? p.k_starts[seq] : seq_start;
-  if (k_start < 0) return;  // this query block takes no part in the call
   const int head = blockIdx.y;
   const int kv_head = head / (p.Hq / p.Hkv);
   const int q_row0 = qt * BQ;  // position inside the sequence
   const int kv_end = p.causal ? min(seq_len, q_row0 + BQ) : seq_len;
-  // first key tile any row of this query tile can see under a sliding window
-  const int kt0 = p.window > 0 ? max(0, q_row0 - p.window + 1) / BKV : 0;
-  const int n_kv = max(0, (kv_end + BKV - 1) / BKV - kt0);
+  const int n_kv = (kv_end + BKV - 1) / BKV;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -137,34 +122,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------------
     if (lane == 0) {
-      mbar_expect_tx(&bars->q_full, TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::CHUNKS; ++c)
-        tma_load_3d(smem + SMEM_Q + c * CHUNK_BYTES, &tmap_q, &bars->q_full, c * 64, head, seq_start + q_row0);
+      mbar_expect_tx(&bars->q_full, CHUNK_BYTES);
+      tma_load_3d(smem + SMEM_Q, &tmap_q, &bars->q_full, 0, head, seq_start + q_row0);
       bool ok = true;
       int issued = 0;
       for (int j = 0; j < n_kv && ok; ++j) {
         const int s = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        const int tok = k_start + (kt0 + j) * BKV;
+        const int tok = seq_start + j * BKV;
         if (!mbar_wait(&bars->k_empty[s], ph ^ 1, abort_flag, p.status, XB_K_ATTN_FWD, 100 + s)) {
           ok = false;
           break;
         }
-        mbar_expect_tx(&bars->k_full[s], TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::CHUNKS; ++c)
-          tma_load_3d(smem + SMEM_K + s * TILE_BYTES + c * CHUNK_BYTES, &tmap_k, &bars->k_full[s], c * 64,
-                      kv_head, tok);
+        mbar_expect_tx(&bars->k_full[s], CHUNK_BYTES);
+        tma_load_3d(smem + SMEM_K + s * CHUNK_BYTES, &tmap_k, &bars->k_full[s], 0, kv_head, tok);
         if (!mbar_wait(&bars->v_empty[s], ph ^ 1, abort_flag, p.status, XB_K_ATTN_FWD, 110 + s)) {
           ok = false;
           break;
         }
-        mbar_expect_tx(&bars->v_full[s], TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::CHUNKS; ++c)
-          tma_load_3d(smem + SMEM_V + s * TILE_BYTES + c * CHUNK_BYTES, &tmap_v, &bars->v_full[s], c * 64,
-                      kv_head, tok);
+        mbar_expect_tx(&bars->v_full[s], CHUNK_BYTES);
+        tma_load_3d(smem + SMEM_V + s * CHUNK_BYTES, &tmap_v, &bars->v_full[s], 0, kv_head, tok);
         issued = j + 1;
       }
       if (!ok) {
@@ -198,10 +175,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (!mbar_wait(&bars->s_empty[s], ph ^ 1, abort_flag, p.status, XB_K_ATTN_FWD, 220 + s))
           return false;
         tc_fence_after();
-        const uint32_t sk = xb_smem_u32(smem + SMEM_K + s * TILE_BYTES);
+        const uint32_t sk = xb_smem_u32(smem + SMEM_K + s * CHUNK_BYTES);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * CHUNK_BYTES + (k & 3) * 32;
+          const uint32_t off = k * 32;
           tc_mma_f16_ss(tmem_base + S_COL0 + s * BKV, xb_smem_desc(kmaj, sq + off),
                         xb_smem_desc(kmaj, sk + off), idesc_s, k > 0 ? 1u : 0u);
         }
@@ -225,16 +202,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           break;
         }
         tc_fence_after();
-        const uint32_t sv = xb_smem_u32(smem + SMEM_V + s * TILE_BYTES);
+        const uint32_t sv = xb_smem_u32(smem + SMEM_V + s * CHUNK_BYTES);
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k) {
           const uint32_t a_off = (k >> 2) * CHUNK_BYTES + (k & 3) * 32;  // P: K-major over kv
           const uint32_t b_off = k * 2048;                               // V: 16 kv rows per step
           tc_mma_f16_ss(tmem_base + O_COL, xb_smem_desc(kmaj, sp + a_off),
                         xb_smem_desc(mnmaj, sv + b_off), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-          if constexpr (C::SPLIT)
-            tc_mma_f16_ss(tmem_base + O_COL, xb_smem_desc(kmaj, sp + P_BYTES + a_off),
-                          xb_smem_desc(mnmaj, sv + b_off), idesc_o, 1u);
+          tc_mma_f16_ss(tmem_base + O_COL, xb_smem_desc(kmaj, sp + P_BYTES + a_off),
+                        xb_smem_desc(mnmaj, sv + b_off), idesc_o, 1u);
         }
         tc_commit(&bars->v_empty[s]);
         tc_commit(&bars->pv_done);
@@ -271,15 +247,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       tc_fence_before();
       mbar_arrive(&bars->s_empty[s]);
 
-      const int col0 = (kt0 + j) * BKV;
-      const bool need_mask = (col0 + BKV > seq_len) || (p.causal && col0 + BKV - 1 > q_row0) ||
-                             (p.window > 0 && col0 < q_row0 + BQ - p.window);
+      const int col0 = j * BKV;
+      const bool need_mask = (col0 + BKV > seq_len) || (p.causal && col0 + BKV - 1 > q_row0);
       if (need_mask) {
         const int lim = p.causal ? min(seq_len - 1, row_pos) : seq_len - 1;  // last valid column
-        const int lo = p.window > 0 ? row_pos - p.window + 1 : 0;            // first valid column
 #pragma unroll
         for (int i = 0; i < BKV; ++i)
-          if (col0 + i > lim || col0 + i < lo) sc[i] = -INFINITY;
+          if (col0 + i > lim) sc[i] = -INFINITY;
       }
       float mx_raw = -INFINITY;
 #pragma unroll
@@ -329,14 +303,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         v.w = pack_bf16x2(sc[c16 * 8 + 6], sc[c16 * 8 + 7]);
         const int half = c16 >> 3, slot = (c16 & 7) ^ (r & 7);
         *reinterpret_cast<uint4*>(sp + half * CHUNK_BYTES + r * 128 + slot * 16) = v;
-        if constexpr (C::SPLIT) {
-          uint4 w;
-          w.x = pack_bf16x2_rest(sc[c16 * 8 + 0], sc[c16 * 8 + 1], v.x);
-          w.y = pack_bf16x2_rest(sc[c16 * 8 + 2], sc[c16 * 8 + 3], v.y);
-          w.z = pack_bf16x2_rest(sc[c16 * 8 + 4], sc[c16 * 8 + 5], v.z);
-          w.w = pack_bf16x2_rest(sc[c16 * 8 + 6], sc[c16 * 8 + 7], v.w);
-          *reinterpret_cast<uint4*>(sp + P_BYTES + half * CHUNK_BYTES + r * 128 + slot * 16) = w;
-        }
+        uint4 w;
+        w.x = pack_bf16x2_rest(sc[c16 * 8 + 0], sc[c16 * 8 + 1], v.x);
+        w.y = pack_bf16x2_rest(sc[c16 * 8 + 2], sc[c16 * 8 + 3], v.y);
+        w.z = pack_bf16x2_rest(sc[c16 * 8 + 4], sc[c16 * 8 + 5], v.z);
+        w.w = pack_bf16x2_rest(sc[c16 * 8 + 6], sc[c16 * 8 + 7], v.w);
+        *reinterpret_cast<uint4*>(sp + P_BYTES + half * CHUNK_BYTES + r * 128 + slot * 16) = w;
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -349,12 +321,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (ok) {
       tc_fence_after();
       const bool valid = row_pos < seq_len;
-      if (p.sinks != nullptr) {
-        // the sink logit joins the denominator (and the LSE) and contributes no value
-        const float sk = __ldg(p.sinks + head) * 1.4426950408889634f;
-        if (m == -INFINITY) { m = sk; l = 1.f; }
-        else l += xb_ex2(sk - m);
-      }
       const float inv = (l > 0.f) ? 1.f / l : 0.f;
       __nv_bfloat16* orow =
           p.out + (size_t)(seq_start + row_pos) * p.ldo + (size_t)head * D;
@@ -378,15 +344,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             o.w = pack_bf16x2(__uint_as_float(t[v4 * 8 + 6]) * inv, __uint_as_float(t[v4 * 8 + 7]) * inv);
             *reinterpret_cast<uint4*>(orow + c * 32 + v4 * 8) = o;
           }
-          if constexpr (C::SPLIT) {
-            if (p.out_f32 != nullptr) {
-              float* frow = p.out_f32 + ((size_t)(seq_start + row_pos) * p.Hq + head) * D + c * 32;
+          if (p.out_f32 != nullptr) {
+            float* frow = p.out_f32 + ((size_t)(seq_start + row_pos) * p.Hq + head) * D + c * 32;
 #pragma unroll
-              for (int i = 0; i < 32; i += 4)
-                *reinterpret_cast<float4*>(frow + i) =
-                    make_float4(__uint_as_float(t[i]) * inv, __uint_as_float(t[i + 1]) * inv,
-                                __uint_as_float(t[i + 2]) * inv, __uint_as_float(t[i + 3]) * inv);
-            }
+            for (int i = 0; i < 32; i += 4)
+              *reinterpret_cast<float4*>(frow + i) =
+                  make_float4(__uint_as_float(t[i]) * inv, __uint_as_float(t[i + 1]) * inv,
+                              __uint_as_float(t[i + 2]) * inv, __uint_as_float(t[i + 3]) * inv);
           }
         }
       }
@@ -440,47 +404,39 @@ XB_API int xb_attn_fwd_ex(const void* q, const void* k, const void* v, void* out
 }
 
 namespace xb_attn_fwd_ns {
-template <int D>
-static int launch(const void* q, const void* k, const void* v, Params& p, long long ldq, long long ldk,
-                  long long ldv, int Tk, int max_tiles, cudaStream_t stream) {
+static int launch(const void* q, const void* k, const void* v, const Params& p, long long ldq, long long ldk,
+                  long long ldv, cudaStream_t stream) {
   CUtensorMap tq, tk, tv;
   if (xb_make_tmap_3d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.T, p.Hq, D, ldq, D, BQ, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -2;
-  if (xb_make_tmap_3d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, p.Hkv, D, ldk, D, BKV, 1, 64,
+  if (xb_make_tmap_3d(&tk, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.T, p.Hkv, D, ldk, D, BKV, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
-  if (xb_make_tmap_3d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, p.Hkv, D, ldv, D, BKV, 1, 64,
+  if (xb_make_tmap_3d(&tv, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.T, p.Hkv, D, ldv, D, BKV, 1, 64,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -4;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[dev & 63]) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Cfg<D>::SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SMEM_BYTES) != cudaSuccess)
       return -10;
     configured[dev & 63] = true;
   }
   // upper bound on the number of query tiles: every sequence adds at most one partial tile
-  const int tiles = max_tiles > 0 ? max_tiles : (p.T + BQ - 1) / BQ + p.num_seqs;
+  const int tiles = (p.T + BQ - 1) / BQ + p.num_seqs;
   dim3 grid(tiles, p.Hq);
-  attn_fwd_kernel<D><<<grid, NUM_THREADS, Cfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  attn_fwd_kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
-
-static Params make_params(void* out, float* lse, const int* cu_seqlens, const int* k_starts, const float* sinks,
-                          long long ldo, int num_seqs, int T, int Hq, int Hkv, int causal, float scale) {
-  Params p;
-  p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.out_f32 = nullptr; p.lse = lse; p.cu_seqlens = cu_seqlens;
-  p.k_starts = k_starts;
-  p.num_seqs = num_seqs; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1;
-  p.window = causal >> 1; p.sinks = sinks;
-  p.scale_log2 = scale * 1.4426950408889634f;
-  p.status = xb_status_ptr();
-  return p;
-}
 }  // namespace xb_attn_fwd_ns
+
+int xb_attn_fwd_hd128(const void* q, const void* k, const void* v, void* out, float* lse, const int* cu_seqlens,
+                      const int* k_starts, const float* sinks, long long ldq, long long ldk, long long ldv,
+                      long long ldo, int num_seqs, int T, int Tk, int Hq, int Hkv, int causal, float scale,
+                      int max_tiles, cudaStream_t stream);
 
 // As xb_attn_fwd_ex with two more features.  ``causal``: bit 0 is the causal flag, the bits above it
 // hold a sliding-window length (0: none): a query sees the keys with q_pos - k_pos < window.
@@ -489,23 +445,25 @@ XB_API int xb_attn_fwd_sink(const void* q, const void* k, const void* v, void* o
                             const int* cu_seqlens, const int* k_starts, const float* sinks, long long ldq,
                             long long ldk, long long ldv, long long ldo, int num_seqs, int T, int Tk, int Hq,
                             int Hkv, int D, int causal, float scale, int max_tiles, void* stream) {
-  using namespace xb_attn_fwd_ns;
   if (D != 128) return -1;
   if (T <= 0 || num_seqs <= 0) return 0;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || Hq % Hkv) return -1;
-  Params p = make_params(out, lse, cu_seqlens, k_starts, sinks, ldo, num_seqs, T, Hq, Hkv, causal, scale);
-  return launch<128>(q, k, v, p, ldq, ldk, ldv, Tk, max_tiles, (cudaStream_t)stream);
+  return xb_attn_fwd_hd128(q, k, v, out, lse, cu_seqlens, k_starts, sinks, ldq, ldk, ldv, ldo, num_seqs, T, Tk, Hq,
+                           Hkv, causal, scale, max_tiles, (cudaStream_t)stream);
 }
 
-// Head dim 64 with probabilities of fp32 quality (see Cfg).  out_f32: optional [T, Hq, 64], the
-// unrounded output, which the backward takes its row sums of dO o O from.
+// Head dim 64, see the head of the file.  out_f32: optional [T, Hq, 64], the unrounded output, which the
+// backward takes its row sums of dO o O from.
 XB_API int xb_attn_fwd_hd64(const void* q, const void* k, const void* v, void* out, float* out_f32, float* lse,
                             const int* cu_seqlens, long long ldq, long long ldk, long long ldv, long long ldo,
                             int num_seqs, int T, int Hq, int Hkv, int causal, float scale, void* stream) {
   using namespace xb_attn_fwd_ns;
   if (T <= 0 || num_seqs <= 0) return 0;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || Hq % Hkv) return -1;
-  Params p = make_params(out, lse, cu_seqlens, nullptr, nullptr, ldo, num_seqs, T, Hq, Hkv, causal & 1, scale);
-  p.out_f32 = out_f32;
-  return launch<64>(q, k, v, p, ldq, ldk, ldv, T, 0, (cudaStream_t)stream);
+  Params p;
+  p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.out_f32 = out_f32; p.lse = lse; p.cu_seqlens = cu_seqlens;
+  p.num_seqs = num_seqs; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal & 1;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.status = xb_status_ptr();
+  return launch(q, k, v, p, ldq, ldk, ldv, (cudaStream_t)stream);
 }
