@@ -116,6 +116,18 @@ embedding_bwd_bf16_kernel(const long long* __restrict__ ids, const __nv_bfloat16
   }
 }
 
+// cos / sin of pos[t] * inv_freq[i], times a factor: [T, n] each
+__global__ void __launch_bounds__(256)
+rope_tables_kernel(const long long* __restrict__ pos, const float* __restrict__ inv_freq, float factor,
+                   float* __restrict__ cosb, float* __restrict__ sinb, long long total, int n) {
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+    const long long t = i / n;
+    const float a = (float)pos[t] * inv_freq[i - t * n];
+    cosb[i] = cosf(a) * factor;
+    sinb[i] = sinf(a) * factor;
+  }
+}
+
 __global__ void __launch_bounds__(256)
 add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                 __nv_bfloat16* __restrict__ out, long long nvec) {
@@ -199,6 +211,14 @@ XB_API int xb_embedding_bwd(const long long* ids, const void* dout, void* dtable
   else
     embedding_bwd_bf16_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
         ids, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dtable, T, H, V);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+XB_API int xb_rope_tables(const long long* pos, const float* inv_freq, float factor, float* cosb, float* sinb, int T,
+                          int n, void* stream) {
+  const long long total = (long long)T * n;
+  if (total <= 0) return 0;
+  rope_tables_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)stream>>>(pos, inv_freq, factor, cosb, sinb, total, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -224,7 +224,7 @@ constexpr int REDUCE_ROWS = 16;
 __global__ void __launch_bounds__(32 * REDUCE_ROWS)
 reduce_partials_kernel(const float* __restrict__ partial, int P, int H, __nv_bfloat16* __restrict__ out_bf16,
                        float* __restrict__ out_f32, int accumulate, __nv_bfloat16* __restrict__ out2_bf16,
-                       int split) {
+                       float* __restrict__ out2_f32, int split) {
   __shared__ float sh[REDUCE_ROWS][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + tx;
@@ -239,9 +239,10 @@ reduce_partials_kernel(const float* __restrict__ partial, int P, int H, __nv_bfl
   s = 0.f;
 #pragma unroll
   for (int i = 0; i < REDUCE_ROWS; ++i) s += sh[i][tx];
-  if (out_f32) out_f32[h] = accumulate ? out_f32[h] + s : s;
   __nv_bfloat16* o = h < split ? out_bf16 : out2_bf16;
+  float* f = h < split ? out_f32 : out2_f32;
   const int c = h < split ? h : h - split;
+  if (f) f[c] = accumulate ? f[c] + s : s;
   if (o) o[c] = __float2bfloat16(accumulate ? __bfloat162float(o[c]) + s : s);
 }
 
@@ -256,6 +257,34 @@ reduce_partials_kernel(const float* __restrict__ partial, int P, int H, __nv_bfl
 // of all its heads are issued before the first is used (32-bit loads of bf16 pairs, 2 * QKR_HPW in
 // flight per lane).
 constexpr int QKR_HPW = 4;
+
+// PER consecutive values of a lane; rows are multiples of 64 values, so pairs are aligned
+template <int PER>
+__device__ __forceinline__ void load_f32(const float* p, float (&f)[PER]) {
+  if constexpr (PER % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < PER; i += 2) {
+      const float2 v = __ldg(reinterpret_cast<const float2*>(p + i));
+      f[i] = v.x; f[i + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) f[i] = __ldg(p + i);
+  }
+}
+template <int PER>
+__device__ __forceinline__ void load_bf16(const __nv_bfloat16* p, float (&f)[PER]) {
+  if constexpr (PER % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < PER; i += 2) {
+      const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + i));
+      f[i] = v.x; f[i + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) f[i] = __bfloat162float(p[i]);
+  }
+}
 
 template <int D>
 __global__ void __launch_bounds__(256)
@@ -401,36 +430,24 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout_bf16,
         if (dout_f32_q != nullptr) {
           const float* s = (h < Hq) ? dout_f32_q + ((size_t)t * Hq + h) * D
                                     : dout_f32_k + ((size_t)t * Hkv + (h - Hq)) * D;
-#pragma unroll
-          for (int i = 0; i < PER; ++i) {
-            d1[g][i] = s[lane * PER + i];
-            d2[g][i] = s[HALF + lane * PER + i];
-          }
+          load_f32<PER>(s + lane * PER, d1[g]);
+          load_f32<PER>(s + HALF + lane * PER, d2[g]);
         } else {
           const __nv_bfloat16* s = dout_bf16 + (size_t)t * ld_dout + (size_t)h * D;
-#pragma unroll
-          for (int i = 0; i < PER; ++i) {
-            d1[g][i] = __bfloat162float(s[lane * PER + i]);
-            d2[g][i] = __bfloat162float(s[HALF + lane * PER + i]);
-          }
+          load_bf16<PER>(s + lane * PER, d1[g]);
+          load_bf16<PER>(s + HALF + lane * PER, d2[g]);
         }
         if (do_norm) {
           const __nv_bfloat16* src = qkv + (size_t)t * ld_in + (size_t)h * D;
-#pragma unroll
-          for (int i = 0; i < PER; ++i) {
-            x1[g][i] = __bfloat162float(src[lane * PER + i]);
-            x2[g][i] = __bfloat162float(src[HALF + lane * PER + i]);
-          }
+          load_bf16<PER>(src + lane * PER, x1[g]);
+          load_bf16<PER>(src + HALF + lane * PER, x2[g]);
           rs[g] = rstd_in[(size_t)t * heads + h];
         }
       }
     }
     float c[PER], sn[PER];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      c[i] = __ldg(cosb + (size_t)t * HALF + lane * PER + i);
-      sn[i] = __ldg(sinb + (size_t)t * HALF + lane * PER + i);
-    }
+    load_f32<PER>(cosb + (size_t)t * HALF + lane * PER, c);
+    load_f32<PER>(sinb + (size_t)t * HALF + lane * PER, sn);
 #pragma unroll
     for (int g = 0; g < QKR_HPW; ++g) {
       const int h = h0 + g;
@@ -544,7 +561,7 @@ XB_API int xb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const fl
   else rmsnorm_bwd_kernel<8><<<rows, NORM_THREADS, 0, st>>>(XB_ARGS);
 #undef XB_ARGS
   reduce_partials_kernel<<<(H + 31) / 32, 32 * REDUCE_ROWS, 0, st>>>(partial, rows, H, (__nv_bfloat16*)dw_bf16, dw_f32,
-                                                                     accumulate, nullptr, H);
+                                                                     accumulate, nullptr, nullptr, H);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -571,7 +588,8 @@ XB_API int xb_qk_norm_rope_fwd(const void* qkv, long long ld_in, const void* wq,
 XB_API int xb_qk_norm_rope_bwd_partial_rows() { return xb_sm_count() * 4; }
 
 // dout is either bf16 [T, (Hq+Hkv)*D] or two fp32 buffers [T,Hq,D] / [T,Hkv,D].
-// partial: fp32 [xb_qk_norm_rope_bwd_partial_rows() * 2 * D]; dwq/dwk (bf16) accumulate flag.
+// partial: fp32 [xb_qk_norm_rope_bwd_partial_rows() * 2 * D]; accumulate: bit 0 adds to dwq / dwk, bit 1 says
+// that they are fp32 (else bf16).
 XB_API int xb_qk_norm_rope_bwd(const void* dout_bf16, const float* dq_f32, const float* dk_f32,
                                long long ld_dout, const void* qkv, long long ld_in, const void* wq,
                                const void* wk, const float* cosb, const float* sinb,
@@ -593,8 +611,10 @@ XB_API int xb_qk_norm_rope_bwd(const void* dout_bf16, const float* dq_f32, const
 #undef XB_LAUNCH
   if (do_norm && partial) {
     // partial rows are [2][D]: q weights, then k weights
+    const bool f32 = accumulate & 2;
     reduce_partials_kernel<<<(2 * D + 31) / 32, 32 * REDUCE_ROWS, 0, st>>>(
-        partial, grid, 2 * D, (__nv_bfloat16*)dwq, nullptr, accumulate, (__nv_bfloat16*)dwk, D);
+        partial, grid, 2 * D, f32 ? nullptr : (__nv_bfloat16*)dwq, f32 ? (float*)dwq : nullptr, accumulate & 1,
+        f32 ? nullptr : (__nv_bfloat16*)dwk, f32 ? (float*)dwk : nullptr, D);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -672,6 +692,6 @@ XB_API int xb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* w, 
 #undef XB_ARGS
   // every one of the `rows` partial rows was just written by the kernel above
   reduce_partials_kernel<<<(H + 31) / 32, 32 * REDUCE_ROWS, 0, st>>>(partial, rows, H, (__nv_bfloat16*)dw_bf16, dw_f32,
-                                                                     accumulate, nullptr, H);
+                                                                     accumulate, nullptr, nullptr, H);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

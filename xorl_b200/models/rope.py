@@ -11,6 +11,8 @@ from typing import Optional, Tuple
 
 import torch
 
+from ..ops import _lib
+
 
 def _default(dim: int, theta: float) -> torch.Tensor:
     return 1.0 / (theta ** (torch.arange(0, dim, 2, dtype=torch.float32) / dim))
@@ -89,6 +91,15 @@ class RotaryEmbedding(torch.nn.Module):
         self.rot_dim = inv.numel() * 2
         self.max_position_embeddings = max_position_embeddings
 
+    def _tables(self, position_ids: torch.Tensor, inv: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+        """Both tables in one kernel: five element-wise launches otherwise, which a short call notices."""
+        T, n = position_ids.numel(), inv.numel()
+        cos, sin = (torch.empty((T, n), device=position_ids.device, dtype=torch.float32) for _ in range(2))
+        _lib.check(_lib.cuda_lib().xb_rope_tables(position_ids.data_ptr(), inv.data_ptr(), float(self.attention_factor),
+                                                  cos.data_ptr(), sin.data_ptr(), T, n, _lib.stream_ptr()),
+                   "xb_rope_tables")
+        return cos, sin
+
     @torch.no_grad()
     def forward(self, position_ids: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """position_ids [T] -> (cos, sin) fp32 [T, rot_dim/2]."""
@@ -102,6 +113,9 @@ class RotaryEmbedding(torch.nn.Module):
                 base = self.theta * ((factor * seq_len / self.max_position_embeddings)
                                      - (factor - 1)) ** (dim / (dim - 2))
                 inv = _default(dim, base).to(position_ids.device)
+        if (position_ids.is_cuda and position_ids.dtype == torch.int64 and position_ids.is_contiguous()
+                and inv.is_contiguous() and position_ids.numel() < 2 ** 31):
+            return self._tables(position_ids, inv)
         ang = position_ids.reshape(-1, 1).to(torch.float32) * inv.reshape(1, -1)
         return (ang.cos() * self.attention_factor).contiguous(), \
                (ang.sin() * self.attention_factor).contiguous()

@@ -47,6 +47,7 @@ _SIGNATURES = {
     "xb_quant_mx_rows_lim": [P, L, P, L, P, I, L, I, P, P],
     "xb_embedding_fwd": [P, P, P, I, I, L, P],
     "xb_embedding_bwd": [P, P, P, I, I, I, L, P],
+    "xb_rope_tables": [P, P, F, P, P, I, I, P],
     "xb_add_bf16": [P, P, P, L, P],
     "xb_cross_entropy": [P, L, P, P, P, I, I, L, F, I, F, P],
     "xb_cross_entropy_rows": [P, L, P, P, P, P, I, I, L, F, I, P],

@@ -13,7 +13,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib
-from .grad_sink import deliver_param_grad
+from .grad_sink import deliver_param_grad, grad_target, mark_written
 
 _launches = 0
 
@@ -201,6 +201,21 @@ def _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv) -> bool:
             and torch.autograd.forward_ad._current_level < 0)
 
 
+def _qk_weight_grads(wq, wk, D: int, T: int, device):
+    """Where the backward of qk-norm leaves the two weight gradients: (dwq, dwk, flags of xb_qk_norm_rope_bwd,
+    function that delivers them).  An engine's fp32 gradient buffers are written in place."""
+    (tq, fq), (tk, fk) = grad_target(wq), grad_target(wk)
+    if T > 0 and tq is not None and tk is not None and fq == fk and tq.dtype == tk.dtype == torch.float32 \
+            and tq.is_contiguous() and tk.is_contiguous():
+        def written():
+            mark_written(wq)
+            mark_written(wk)
+            return None, None
+        return tq, tk, 2 | int(not fq), written
+    dwq, dwk = (torch.zeros(D, device=device, dtype=torch.bfloat16) for _ in range(2))
+    return dwq, dwk, 0, lambda: (deliver_param_grad(wq, dwq), deliver_param_grad(wk, dwk))
+
+
 class _FlashAttn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens, causal, scale, window, sinks):
@@ -308,22 +323,19 @@ class _QKNormRopeAttn(torch.autograd.Function):
             dq, dk = _attn_bwd(q, k, v, out, dout, lse, cu, causal, scale, dv)
         lib = _lib.cuda_lib()
         partial = dwq = dwk = None
+        flags = 0
         if do_norm:
             rows = lib.xb_qk_norm_rope_bwd_partial_rows()
             partial = torch.empty(rows * 2 * D, device=qkv.device, dtype=torch.float32)
-            dwq = torch.zeros(D, device=qkv.device, dtype=torch.bfloat16)
-            dwk = torch.zeros(D, device=qkv.device, dtype=torch.bfloat16)
+            dwq, dwk, flags, deliver = _qk_weight_grads(wq, wk, D, T, qkv.device)
         _lib.check(lib.xb_qk_norm_rope_bwd(None, dq.data_ptr(), dk.data_ptr(), 0, qkv.data_ptr(),
                                            qkv.stride(0), _lib.ptr(wq), _lib.ptr(wk), cos.data_ptr(),
                                            sin.data_ptr(), _lib.ptr(rstd), dqkv.data_ptr(),
                                            dqkv.stride(0), _lib.ptr(partial), _lib.ptr(dwq),
-                                           _lib.ptr(dwk), 0, T, Hq, Hkv, D, int(do_norm),
+                                           _lib.ptr(dwk), flags, T, Hq, Hkv, D, int(do_norm),
                                            _lib.stream_ptr()), "xb_qk_norm_rope_bwd")
-        _launches += 4 if do_norm else 1
-        gq = gk = None
-        if do_norm:
-            gq = deliver_param_grad(wq, dwq)
-            gk = deliver_param_grad(wk, dwk)
+        _launches += 2 if do_norm else 1
+        gq, gk = deliver() if do_norm else (None, None)
         return dqkv, gq, gk, None, None, None, None, None, None, None, None, None
 
 
@@ -364,19 +376,18 @@ class _QKNormRope(torch.autograd.Function):
         dqkv[:, (Hq + Hkv) * D:] = dv.reshape(T, Hkv * D)
         lib = _lib.cuda_lib()
         partial = dwq = dwk = None
+        flags = 0
         if do_norm:
             rows = lib.xb_qk_norm_rope_bwd_partial_rows()
             partial = torch.empty(rows * 2 * D, device=qkv.device, dtype=torch.float32)
-            dwq = torch.zeros(D, device=qkv.device, dtype=torch.bfloat16)
-            dwk = torch.zeros(D, device=qkv.device, dtype=torch.bfloat16)
+            dwq, dwk, flags, deliver = _qk_weight_grads(wq, wk, D, T, qkv.device)
         _lib.check(lib.xb_qk_norm_rope_bwd(dqk.data_ptr(), None, None, dqk.stride(0), qkv.data_ptr(), qkv.stride(0),
                                            _lib.ptr(wq), _lib.ptr(wk), cos.data_ptr(), sin.data_ptr(), _lib.ptr(rstd),
                                            dqkv.data_ptr(), dqkv.stride(0), _lib.ptr(partial), _lib.ptr(dwq),
-                                           _lib.ptr(dwk), 0, T, Hq, Hkv, D, int(do_norm), _lib.stream_ptr()),
+                                           _lib.ptr(dwk), flags, T, Hq, Hkv, D, int(do_norm), _lib.stream_ptr()),
                    "xb_qk_norm_rope_bwd")
-        _launches += 4 if do_norm else 1
-        gq = deliver_param_grad(wq, dwq) if do_norm else None
-        gk = deliver_param_grad(wk, dwk) if do_norm else None
+        _launches += 2 if do_norm else 1
+        gq, gk = deliver() if do_norm else (None, None)
         return dqkv, gq, gk, None, None, None, None, None, None
 
 

@@ -29,12 +29,13 @@ def cross_entropy_sum_reference(logits: torch.Tensor, labels: torch.Tensor,
 
 
 def ce_chunk_(logits: torch.Tensor, labels: torch.Tensor, grad_scale: float, write_grad: bool,
-              ignore_index: int = IGNORE_INDEX, z_loss: float = 0.0):
-    """Per-row losses and LSE of a bf16 logits chunk; rewrites ``logits`` with d(loss)/d(logits)
-    times ``grad_scale`` when ``write_grad``."""
+              ignore_index: int = IGNORE_INDEX, z_loss: float = 0.0, loss: torch.Tensor | None = None):
+    """Per-row losses (into ``loss`` if given) and LSE of a bf16 logits chunk; rewrites ``logits`` with
+    d(loss)/d(logits) times ``grad_scale`` when ``write_grad``."""
     global _launches
     rows, V = logits.shape
-    loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
+    if loss is None:
+        loss = torch.empty(rows, device=logits.device, dtype=torch.float32)
     lse = torch.empty(rows, device=logits.device, dtype=torch.float32)
     _lib.check(_lib.cuda_lib().xb_cross_entropy(logits.data_ptr(), logits.stride(0),
                                                 labels.data_ptr(), loss.data_ptr(), lse.data_ptr(),
@@ -67,9 +68,7 @@ class _FusedLinearCE(torch.autograd.Function):
             h = hidden[s:e]
             logits = buf[: e - s, :V]
             gemm(h, weight, out=logits)
-            l, _ = ce_chunk_(logits, labels[s:e], grad_scale, need_dh or need_dw, ignore_index,
-                             z_loss)
-            losses[s:e] = l
+            ce_chunk_(logits, labels[s:e], grad_scale, need_dh or need_dw, ignore_index, z_loss, losses[s:e])
             if need_dh:
                 gemm(logits, weight, b_mn=True, out=dh[s:e])
             if need_dw:
@@ -169,8 +168,8 @@ def fused_linear_token_loss(hidden: torch.Tensor, weight: torch.Tensor, labels: 
             e = min(T, s + chunk_tokens)
             logits = buf[: e - s, :V]
             gemm(h2[s:e], weight, out=logits)
-            l, _ = ce_chunk_(logits, lab[s:e], 0.0, False, ignore_index)
-            lp[s:e] = -l
+            ce_chunk_(logits, lab[s:e], 0.0, False, ignore_index, loss=lp[s:e])
+        lp.neg_()
     if not torch.is_grad_enabled():
         # evaluation (log-probabilities only): there is nothing to differentiate
         loss, metrics = loss_fn(lp, mask)

@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .grad_sink import deliver_param_grad
+from .grad_sink import deliver_param_grad, grad_target, mark_written
 
 _launches = 0
 
@@ -77,14 +77,21 @@ class _RMSNorm(torch.autograd.Function):
         rows = lib.xb_rmsnorm_bwd_partial_rows(T)
         partial = torch.empty(rows * H, device=h.device, dtype=torch.float32)
         dx = torch.empty_like(h)
-        dw = torch.empty(H, device=h.device, dtype=torch.float32)
+        # the reduction over the partial rows writes, or adds, straight into an engine's fp32 gradient buffer
+        tgt, fresh = grad_target(w) if ctx.needs_input_grad[2] else (None, False)
+        direct = tgt is not None and tgt.dtype == torch.float32 and tgt.is_contiguous() and T > 0
+        dw = tgt if direct else torch.empty(H, device=h.device, dtype=torch.float32)
         _lib.check(lib.xb_rmsnorm_bwd(dy2.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr(),
                                       _lib.ptr(dres), dx.data_ptr(), partial.data_ptr(), None,
-                                      dw.data_ptr(), 0, T, H, int(ctx.zero_centered),
+                                      dw.data_ptr(), int(direct and not fresh), T, H, int(ctx.zero_centered),
                                       _lib.stream_ptr()), "xb_rmsnorm_bwd")
         _launches += 2
         dx = dx.reshape(ctx.shape)
-        dwg = deliver_param_grad(w, dw) if ctx.needs_input_grad[2] else None
+        dwg = None
+        if direct:
+            mark_written(w)
+        elif ctx.needs_input_grad[2]:
+            dwg = deliver_param_grad(w, dw)
         return dx, (dx if ctx.has_res else None), dwg, None, None
 
 
