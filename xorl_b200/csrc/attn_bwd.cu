@@ -430,6 +430,25 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo,
   if (lane == 0) delta[(size_t)h * T + t] = s;
 }
 
+// Zeroes the rows of up to three gradients that lie outside every sequence (a fill of all of them costs as
+// much as the row sums below: 190 us for the 268 MB of dQ of 16,384 tokens and 32 heads).
+struct Rows {
+  void* base;
+  long long pitch;      // bytes from row to row
+  int vecs;             // 16-byte vectors of a row
+};
+__global__ void __launch_bounds__(256)
+zero_outside_kernel(const int* __restrict__ cu, int num_seqs, int T, const Rows a, const Rows b, const Rows c) {
+  const int first = min(max(cu[0], 0), T), last = min(max(cu[num_seqs], first), T);
+  const int n = first + T - last;
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const long long t = i < first ? i : last + (i - first);
+    for (const Rows* r : {&a, &b, &c})
+      for (int v = threadIdx.x; v < r->vecs; v += 256)
+        reinterpret_cast<uint4*>(reinterpret_cast<char*>(r->base) + t * r->pitch)[v] = make_uint4(0, 0, 0, 0);
+  }
+}
+
 // as above from the unrounded output, head dim 64 (out: [T, Hq, 64] fp32)
 __global__ void __launch_bounds__(256)
 attn_delta_hd64_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ dout, long long lddo,
@@ -518,7 +537,12 @@ XB_API int xb_attn_bwd_ex(const void* q, const void* k, const void* v, const voi
   if (xb_make_tmap_3d(&tdo, dout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, Hq, D, lddo, D, BQ, 1,
                       64, CU_TENSOR_MAP_SWIZZLE_128B))
     return -5;
-  if (!(flags & 1)) {
+  const bool split = g_split || (causal >> 1);       // sliding windows are implemented by the split kernels only
+  if (!(flags & 1) && split && k_starts == nullptr) {
+    // every row of a sequence is written with a plain store
+    const Rows r{dq_accum, (long long)Hq * D * 4, Hq * D / 4}, none{nullptr, 0, 0};
+    zero_outside_kernel<<<xb_sm_count(), 256, 0, st>>>(cu_seqlens, num_seqs, T, r, none, none);
+  } else if (!(flags & 1)) {
     if (cudaMemsetAsync(dq_accum, 0, (size_t)T * Hq * D * sizeof(float), st) != cudaSuccess)
       return -6;
   }
@@ -527,9 +551,8 @@ XB_API int xb_attn_bwd_ex(const void* q, const void* k, const void* v, const voi
     attn_delta_kernel<<<(int)((rows + 7) / 8), 256, 0, st>>>(
         (const __nv_bfloat16*)out, ldo, (const __nv_bfloat16*)dout, lddo, delta, T, Hq);
   }
-  if (g_split || (causal >> 1)) {     // sliding windows are implemented by the split kernels only
-    // dq_accum is written with plain stores (added to when flags bit 0 is set); rows outside every
-    // sequence keep the zeros of the memset above
+  if (split) {
+    // dq_accum is written with plain stores (added to when flags bit 0 is set)
     const int tiles = max_tiles > 0 ? (max_tiles + 1) / 2 + num_seqs : 0;     // 128-row tiles
     return xb_attn_bwd_hd128(q, k, v, dout, lse, delta, dq_accum, dk, dv, cu_seqlens, k_starts, ldq, ldk, ldv, lddo,
                              lddv, num_seqs, T, Tk, Hq, Hkv, causal, scale, (flags & 1) ? 1 : 0, tiles, st);
@@ -564,10 +587,10 @@ XB_API int xb_attn_bwd_hd64(const void* q, const void* k, const void* v, const f
   using namespace xb_attn_bwd_ns;
   if (T <= 0 || num_seqs <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
-  if (cudaMemsetAsync(dq, 0, (size_t)T * Hq * 64 * sizeof(float), st) != cudaSuccess ||
-      cudaMemsetAsync(dk, 0, (size_t)T * Hkv * 64 * sizeof(float), st) != cudaSuccess ||
-      cudaMemset2DAsync(dv, (size_t)lddv * 2, 0, (size_t)Hkv * 64 * 2, T, st) != cudaSuccess)
-    return -6;
+  if ((lddv % 8) || (reinterpret_cast<uintptr_t>(dv) % 16)) return -1;
+  zero_outside_kernel<<<xb_sm_count(), 256, 0, st>>>(cu_seqlens, num_seqs, T, Rows{dq, (long long)Hq * 256, Hq * 16},
+                                                     Rows{dk, (long long)Hkv * 256, Hkv * 16},
+                                                     Rows{dv, lddv * 2, Hkv * 8});
   const long long rows = (long long)T * Hq;
   attn_delta_hd64_kernel<<<(int)((rows + 7) / 8), 256, 0, st>>>(out_f32, (const __nv_bfloat16*)dout, lddo, delta, T, Hq);
   const int rc = xb_attn_dkv_hd64(q, k, v, dout, lse, delta, dk, dv, cu_seqlens, ldq, ldk, ldv, lddo, lddv, num_seqs,
