@@ -46,15 +46,15 @@ def ce_chunk_(logits: torch.Tensor, labels: torch.Tensor, grad_scale: float, wri
     return loss, lse
 
 
-# Memory that a loss may keep in gradients of logits.  The weight gradient of the lm-head takes several chunks
-# of tokens at once: per chunk it would read and write its whole fp32 buffer (524 MB at 32,000 x 4096) for
-# 1024 tokens of math, 0.37 ms instead of 0.21.  Logits, loss and hidden gradient stay per chunk, whose logits
-# (65 MB there) fit the L2.
+# Memory that a loss may keep in gradients of logits.  The gradient GEMMs of the lm-head take several chunks
+# of tokens at once.  Per chunk the weight gradient would read and write its whole fp32 buffer (524 MB at
+# 32,000 x 4096) for 1024 tokens of math, 0.37 ms instead of 0.21, and the hidden gradient would have half as
+# many tiles as there are SMs.  Logits and loss stay per chunk, whose logits (65 MB there) fit the L2.
 KEPT_LOGITS_BYTES = 5 << 28
 
 
 def _kept_chunks(T: int, chunk_tokens: int, ldv: int) -> int:
-    """Chunks of logit gradients that are kept for one weight-gradient GEMM."""
+    """Chunks of logit gradients that are kept for one pair of gradient GEMMs."""
     return max(1, min(-(-T // chunk_tokens), KEPT_LOGITS_BYTES // (2 * chunk_tokens * ldv)))
 
 
@@ -73,7 +73,7 @@ class _FusedLinearCE(torch.autograd.Function):
             dw_local = torch.zeros((V, H), device=hidden.device, dtype=torch.float32)
         losses = torch.empty(T, device=hidden.device, dtype=torch.float32)
         ldv = (V + 7) // 8 * 8
-        kept = chunk_tokens * (_kept_chunks(T, chunk_tokens, ldv) if need_dw else 1)     # tokens
+        kept = chunk_tokens * (_kept_chunks(T, chunk_tokens, ldv) if need_dw or need_dh else 1)     # tokens
         buf = torch.empty((min(kept, T), ldv), device=hidden.device, dtype=torch.bfloat16)
         first = True
         for s in range(0, T, chunk_tokens):
@@ -82,10 +82,12 @@ class _FusedLinearCE(torch.autograd.Function):
             logits = buf[s - k0:e - k0, :V]
             gemm(hidden[s:e], weight, out=logits)
             ce_chunk_(logits, labels[s:e], grad_scale, need_dh or need_dw, ignore_index, z_loss, losses[s:e])
+            if e < T and e < k0 + kept:
+                continue
+            dlogits, h = buf[:e - k0, :V], hidden[k0:e]
             if need_dh:
-                gemm(logits, weight, b_mn=True, out=dh[s:e])
-            if need_dw and (e == T or e == k0 + kept):
-                dlogits, h = buf[:e - k0, :V], hidden[k0:e]
+                gemm(dlogits, weight, b_mn=True, out=dh[k0:e])
+            if need_dw:
                 if tgt is not None:
                     gemm(dlogits, h, a_mn=True, b_mn=True, out=tgt, accumulate=not (fresh and first))
                 else:
@@ -207,7 +209,7 @@ class _TokenLossBackward(torch.autograd.Function):
         dw_local = torch.zeros((V, H), device=hidden.device, dtype=torch.float32) \
             if (need_dw and tgt is None) else None
         ldv = (V + 7) // 8 * 8
-        kept = chunk_tokens * (_kept_chunks(T, chunk_tokens, ldv) if need_dw else 1)     # tokens
+        kept = chunk_tokens * (_kept_chunks(T, chunk_tokens, ldv) if need_dw or need_dh else 1)     # tokens
         buf = torch.empty((min(kept, T), ldv), device=hidden.device, dtype=torch.bfloat16)
         lib = _lib.cuda_lib()
         scratch = torch.empty(min(chunk_tokens, T), device=hidden.device, dtype=torch.float32)
@@ -223,10 +225,12 @@ class _TokenLossBackward(torch.autograd.Function):
                                                  grad_scale, 1, _lib.stream_ptr()),
                        "xb_cross_entropy_rows")
             _launches += 1
+            if e < T and e < k0 + kept:
+                continue
+            dlogits, h = buf[:e - k0, :V], hidden[k0:e]
             if need_dh:
-                gemm(logits, weight, b_mn=True, out=dh[s:e])
-            if need_dw and (e == T or e == k0 + kept):
-                dlogits, h = buf[:e - k0, :V], hidden[k0:e]
+                gemm(dlogits, weight, b_mn=True, out=dh[k0:e])
+            if need_dw:
                 if tgt is not None:
                     gemm(dlogits, h, a_mn=True, b_mn=True, out=tgt, accumulate=not (fresh and first))
                 else:
