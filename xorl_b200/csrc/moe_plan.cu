@@ -140,8 +140,6 @@ renorm_bwd_kernel(const float* __restrict__ dw, const float* __restrict__ p, con
                   float* __restrict__ dprobs, int T, int E, int k, int renorm, float scale) {
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= T) return;
-  float* row = dprobs + (size_t)t * E;
-  for (int e = lane; e < E; e += 32) row[e] = 0.f;
   const float pj = lane < k ? p[(size_t)t * k + lane] : 0.f;
   const float dj = lane < k ? dw[(size_t)t * k + lane] * scale : 0.f;
   float g = dj;
@@ -149,12 +147,17 @@ renorm_bwd_kernel(const float* __restrict__ dw, const float* __restrict__ p, con
     const float s = warp_sum(pj), c = fmaxf(s, 1e-20f), dot = warp_sum(dj * pj);
     g = dj / c - (s >= 1e-20f ? dot / (c * c) : 0.f);
   }
-  const long long ej = lane < k ? idx[(size_t)t * k + lane] : -1;
-  __syncwarp();
-  // in slot order: an expert that was given twice collects both
-  for (int j = 0; j < k; ++j) {
-    if (lane == j && ej >= 0 && ej < E) row[ej] += g;
-    __syncwarp();
+  const int ej = lane < k ? (int)idx[(size_t)t * k + lane] : -1;
+  float* row = dprobs + (size_t)t * E;
+  for (int e0 = 0; e0 < E; e0 += 32) {
+    // in slot order: an expert that was given twice collects both
+    float v = 0.f;
+    for (int j = 0; j < k; ++j) {
+      const int e = __shfl_sync(0xffffffffu, ej, j);
+      const float gj = __shfl_sync(0xffffffffu, g, j);
+      if (e == e0 + lane) v += gj;
+    }
+    if (e0 + lane < E) row[e0 + lane] = v;
   }
 }
 
