@@ -427,6 +427,24 @@ def test_grouped_gemm_writes_all_rows_and_experts(counts, K, N, dtype, accumulat
     assert _lib.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("K,N", [(8, 64), (40, 128), (168, 72)])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.float32, False), (torch.bfloat16, True)])
+def test_grouped_weight_gradient_of_ragged_heights(K, N, dtype, accumulate):
+    """Output rows that end inside a warp's 32, or before it."""
+    from xorl_b200.ops import _lib, moe
+    torch.manual_seed(K)
+    seg = torch.tensor([0, 128, 384, 384], device="cuda", dtype=torch.int32)
+    x, dy = (torch.randn(384, n, device="cuda").bfloat16() for n in (K, N))
+    out0 = torch.randn(3, K, N, device="cuda").to(dtype)
+    out = out0.clone() if accumulate else torch.full_like(out0, float("nan"))
+    moe._grouped_wgrad_cuda(x, dy, seg, out, accumulate)
+    for e, (a, b) in enumerate([(0, 128), (128, 384), (384, 384)]):
+        ref = x[a:b].double().t() @ dy[a:b].double() + (out0[e].double() if accumulate else 0)
+        # fp32 sums of up to 256 products, one bf16 rounding where the output has it
+        torch.testing.assert_close(out[e].double(), ref, rtol=2 ** -8 if dtype == torch.bfloat16 else 1e-4, atol=1e-3)
+    assert _lib.read_status()[0] == 0
+
+
 def test_mx_scale_of_every_bf16_magnitude():
     """The power-of-two scale from the bits of the maximum, for every finite bf16 value of a block."""
     from xorl_b200.ops import fp8_grouped as fg

@@ -19,11 +19,12 @@ constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16, STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int NUM_THREADS = 192, TMEM_COLS = 512;
 constexpr int MAX_E = 512;
-constexpr int SLAB_COLS = 64;                      // rows-mode epilogue staging: 128 rows x 64 columns bf16
-constexpr int SLAB_BYTES = BM * SLAB_COLS * 2;
+constexpr int SLAB_COLS = 64;                      // epilogue staging: 64 columns of bf16 (32 of fp32)
+constexpr int SLAB_BYTES = 32 * SLAB_COLS * 2;     // a warp's 32 rows of it; two per warp
 constexpr int OFF_SLAB = STAGES * STAGE_BYTES;
-constexpr int OFF_BARS = OFF_SLAB + SLAB_BYTES;
-constexpr int SMEM_BYTES = OFF_BARS + 1024 + 256 + (MAX_E + 1) * 4;
+constexpr int OFF_BARS = OFF_SLAB + 8 * SLAB_BYTES;
+constexpr int SMEM_BYTES = OFF_BARS + 256 + (MAX_E + 1) * 4;
+static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
 
 struct Params {
   int mode;  // 0 rows, 1 wgrad
@@ -85,9 +86,7 @@ __device__ __forceinline__ Tile get_tile(const Params& p, const int* sseg, int t
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_c, const Params p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];
   Barriers* bars = reinterpret_cast<Barriers*>(smem + OFF_BARS);
   int* sseg = reinterpret_cast<int*>(smem + OFF_BARS + 256);
   volatile int* abort_flag = &bars->abort_flag;
@@ -195,6 +194,7 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   } else {
     const int q = warp & 3;
     uint32_t tcount = 0;
+    int slab_at = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       const Tile tl = get_tile(p, sseg, t);
@@ -219,16 +219,21 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       if (p.tma_out) {
         // Stage 128-byte wide slabs (64 bf16 or 32 fp32 columns) in 128B-swizzled shared memory and let
         // TMA write them, or add them, so that global memory sees whole 128-byte row segments.  A thread
-        // holds one row: its own stores would touch 32 rows at once, 16 bytes of each.
-        const int r = q * 32 + lane;
+        // holds one row: its own stores would touch 32 rows at once, 16 bytes of each.  Every warp stages
+        // and sends its own 32 rows in two buffers: with one slab for the tile and a barrier of all four
+        // warps around it, the output of an expert with few rows took longer than its math: weight
+        // gradients of 128 experts of 2048 x 1536 and 768 x 2048 from 256 rows each, fp32, 472 -> 396 and 236 ->
+        // 201 us, of which writing them takes 243 and 122.
         const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
-        uint8_t* slab = smem + OFF_SLAB;
-        uint8_t* srow = slab + r * 128;
+        uint8_t* slabs = smem + OFF_SLAB + q * 2 * SLAB_BYTES;
         const int slab_cols = p.out_fp32 ? SLAB_COLS / 2 : SLAB_COLS;
+        const int row0 = tl.m0 + q * 32;
+        // a store may not begin behind the last row of an expert (or of the buffer)
+        const bool rows_left = row0 < p.M;
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += slab_cols) {
           const int col0 = tl.n0 + c0;
-          if (col0 >= p.N) break;
+          if (col0 >= p.N || !rows_left) break;
           uint32_t v[2][32];
           if (has_acc) {
             tmem_ld_32x32(taddr + c0, v[0]);
@@ -238,12 +243,15 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[0][i] = v[1][i] = 0;
           }
-          if (warp == 2 && lane == 0) tma_store_wait_read<0>();
-          asm volatile("bar.sync 2, 128;" ::: "memory");
+          uint8_t* slab = slabs + slab_at * SLAB_BYTES;
+          uint8_t* srow = slab + lane * 128;
+          slab_at ^= 1;
+          if (lane == 0) tma_store_wait_read<1>();           // the store before the last has left this buffer
+          __syncwarp();
           if (p.out_fp32) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<uint4*>(srow + ((j ^ (r & 7)) * 16)) =
+              *reinterpret_cast<uint4*>(srow + ((j ^ (lane & 7)) * 16)) =
                   make_uint4(v[0][4 * j], v[0][4 * j + 1], v[0][4 * j + 2], v[0][4 * j + 3]);
           } else {
 #pragma unroll
@@ -255,15 +263,15 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
                 o.y = pack_bf16x2(__uint_as_float(v[h][8 * j + 2]), __uint_as_float(v[h][8 * j + 3]));
                 o.z = pack_bf16x2(__uint_as_float(v[h][8 * j + 4]), __uint_as_float(v[h][8 * j + 5]));
                 o.w = pack_bf16x2(__uint_as_float(v[h][8 * j + 6]), __uint_as_float(v[h][8 * j + 7]));
-                *reinterpret_cast<uint4*>(srow + (((h * 4 + j) ^ (r & 7)) * 16)) = o;
+                *reinterpret_cast<uint4*>(srow + (((h * 4 + j) ^ (lane & 7)) * 16)) = o;
               }
           }
           fence_proxy_async_smem();
-          asm volatile("bar.sync 2, 128;" ::: "memory");
-          if (warp == 2 && lane == 0) {
-            if (p.mode == 0) tma_store_2d(&tmap_c, slab, col0, tl.m0);
-            else if (p.accumulate) tma_reduce_add_3d(&tmap_c, slab, col0, tl.m0, tl.e);
-            else tma_store_3d(&tmap_c, slab, col0, tl.m0, tl.e);
+          __syncwarp();
+          if (lane == 0) {
+            if (p.mode == 0) tma_store_2d(&tmap_c, slab, col0, row0);
+            else if (p.accumulate) tma_reduce_add_3d(&tmap_c, slab, col0, row0, tl.e);
+            else tma_store_3d(&tmap_c, slab, col0, row0, tl.e);
             tma_store_commit();
           }
         }
@@ -346,7 +354,7 @@ ggemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         ++tcount;
       }
     }
-    if (p.tma_out && warp == 2 && lane == 0) tma_store_wait<0>();
+    if (p.tma_out && lane == 0) tma_store_wait<0>();
   }
   tc_fence_before();
   __syncthreads();
@@ -387,7 +395,7 @@ XB_API int xb_grouped_gemm_rows(const void* A, const void* B, void* C, const int
   CUtensorMap ta, tb, tc;
   if (xb_make_tmap_2d(&ta, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, R, K, lda, BM, BK,
                       CU_TENSOR_MAP_SWIZZLE_128B)) return -2;
-  if (xb_make_tmap_2d(&tc, C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, R, N, ldc, BM, SLAB_COLS,
+  if (xb_make_tmap_2d(&tc, C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, R, N, ldc, 32, SLAB_COLS,
                       CU_TENSOR_MAP_SWIZZLE_128B)) return -4;
   int rc;
   if (b_mn)
@@ -422,7 +430,7 @@ XB_API int xb_grouped_gemm_wgrad(const void* A, const void* B, void* C, const in
   const bool tma_out = (reinterpret_cast<uintptr_t>(C) % 16) == 0 && (out_fp32 || !accumulate);
   CUtensorMap tc = ta;
   if (tma_out && xb_make_tmap_3d(&tc, C, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                                 out_fp32 ? 4 : 2, E, M, N, (uint64_t)M * N, N, 1, BM,
+                                 out_fp32 ? 4 : 2, E, M, N, (uint64_t)M * N, N, 1, 32,
                                  out_fp32 ? SLAB_COLS / 2 : SLAB_COLS, CU_TENSOR_MAP_SWIZZLE_128B))
     return -4;
   Params p{};
