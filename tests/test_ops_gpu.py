@@ -470,3 +470,18 @@ def test_lora_linear_against_float64(T, slices, out, rank, scaling):
     for g, o, e in zip(got, old, exact):
         eg, eo = ((t.double() - e).norm().item() / e.norm().item() for t in (g, o))
         assert eg <= 1.05 * eo + 2 ** -12, (eg, eo)
+
+
+@pytest.mark.parametrize("M,I,K", [(384, 128, 64), (1000, 264, 328), (4096, 1536, 512), (2500, 5000, 192), (513, 8, 72)])
+def test_linear_swiglu_has_the_bits_of_both_kernels(M, I, K):
+    """The activation in the GEMM's epilogue: whole and cut tiles, widths that end inside one."""
+    from xorl_b200.ops import _lib, activation as act, gemm as g
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = (torch.randn(2 * I, K, device=DEV) * K ** -0.5).bfloat16()
+    with torch.no_grad():
+        before = g.launch_count() + act.launch_count()
+        got = act.linear_swiglu(x, w)
+        assert g.launch_count() + act.launch_count() - before == 2      # one kernel, counted by both
+        assert torch.equal(got, act.swiglu(g.linear(x, w)))
+    assert _lib.read_status()[0] == 0

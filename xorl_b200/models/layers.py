@@ -236,4 +236,8 @@ class MLP(nn.Module):
             from ..parallel.tp import copy_to_tp, reduce_from_tp
             x = copy_to_tp(x, self.tp_group)
             return reduce_from_tp(self.down_proj(self._act(self.gate_up_proj(x))), self.tp_group)
+        up = self.gate_up_proj
+        if type(up) is Linear and up.bias is None and self.swiglu_limit is None \
+                and not (up._forward_hooks or up._forward_pre_hooks or up._backward_hooks or up._backward_pre_hooks):
+            return self.down_proj(act_ops.linear_swiglu(x, up.weight))
         return self.down_proj(self._act(self.gate_up_proj(x)))

@@ -33,6 +33,7 @@ _SIGNATURES = {
     "xb_gemm_set_batch_invariant": [I],
     "xb_gemm_bf16_pair": [P, P, P, I, I, I, L, L, L, I, I, I, I, P],
     "xb_gemm_bf16_pair_ext": [P, P, P, P, P, I, I, I, I, L, L, L, L, L, I, P],
+    "xb_gemm_bf16_swiglu": [P, P, P, I, I, I, L, L, L, P],
     "xb_lora_pack": [P, P, P, P, P, I, P, P, I, I, P],
     "xb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, I, P],
     "xb_rmsnorm_bwd_partial_rows": [I],
@@ -192,13 +193,16 @@ class _NoGrad:
         pass
 
 
+def forward_only() -> bool:
+    """Gradients are off, and no function transform or forward-mode derivative is active."""
+    return not (torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._are_functorch_transforms_active())
+
+
 def apply(fn, *args):
-    """``fn.apply(*args)``; with gradients off, and no function transform or forward-mode derivative active,
-    its forward alone: an autograd node that is thrown away costs as much host time as the launch."""
-    if torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0 \
-            or torch._C._are_functorch_transforms_active():
-        return fn.apply(*args)
-    return fn.forward(_NoGrad(), *args)
+    """``fn.apply(*args)``, or its forward alone where nothing will be differentiated: an autograd node that is
+    thrown away costs as much host time as the launch."""
+    return fn.forward(_NoGrad(), *args) if forward_only() else fn.apply(*args)
 
 
 def ptr(t) -> int | None:

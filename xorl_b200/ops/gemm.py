@@ -59,6 +59,16 @@ def _splits_k(M: int, N: int, K: int) -> bool:
     return K >= 2048 and -(-M // 128) * -(-N // 256) <= 37
 
 
+def takes_pair_kernel(M: int, N: int, K: int) -> bool:
+    """Whether a product of this size runs in the CTA-pair kernel (csrc/gemm2.cu)."""
+    return _BATCH_INVARIANT or (_VARIANT == "pair" and M >= 384 and not _splits_k(M, N, K))
+
+
+def count_launch() -> None:
+    global _launches
+    _launches += 1
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None,
          accumulate: bool = False) -> torch.Tensor:
@@ -102,7 +112,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     lib = _lib.cuda_lib()
     args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
             out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate))
-    if _BATCH_INVARIANT or (_VARIANT == "pair" and M >= 384 and not _splits_k(M, N, K)):
+    if takes_pair_kernel(M, N, K):
         rc = lib.xb_gemm_bf16_pair(*args, _lib.stream_ptr())
     else:
         rc = lib.xb_gemm_bf16(*args, _lib.stream_ptr())
