@@ -186,8 +186,12 @@ SIDE_STREAM_MIN_MACS = 2 ** 31
 def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
     """dW = dy2^T @ x2 for weight ``w``: written straight into the flat gradient buffer of the ZeRO
     unit (returns None), deferred to a W slot of a zero-bubble schedule, or returned as a tensor."""
-    tgt, fresh = grad_target(w)
     store = current_wgrad_store()
+    side = None
+    if store is None and dy2.is_cuda and dy2.shape[0] * dy2.shape[1] * x2.shape[1] >= SIDE_STREAM_MIN_MACS:
+        side = wgrad_stream(dy2.device)
+    # a short product after a long one of the same weight waits for it: both add to one buffer
+    tgt, fresh = grad_target(w, on_side=side is not None)
     if tgt is not None and store is not None:
         # zero-bubble: the buffer slice is claimed now, the GEMM runs in a later W slot
         mark_written(w)
@@ -195,8 +199,6 @@ def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
                      gemm(a, b, a_mn=True, b_mn=True, out=o, accumulate=acc))
         return None
     if tgt is not None:
-        macs = dy2.shape[0] * dy2.shape[1] * x2.shape[1]
-        side = wgrad_stream(dy2.device) if dy2.is_cuda and macs >= SIDE_STREAM_MIN_MACS else None
         if side is not None:
             # overlap with the input-gradient GEMM that follows on the main stream
             side.wait_stream(_lib.current_stream())
@@ -204,7 +206,7 @@ def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
                 gemm(dy2, x2, a_mn=True, b_mn=True, out=tgt, accumulate=not fresh)
             dy2.record_stream(side)
             x2.record_stream(side)
-            note_wgrad_issued()
+            note_wgrad_issued(w)
         else:
             gemm(dy2, x2, a_mn=True, b_mn=True, out=tgt, accumulate=not fresh)
         mark_written(w)

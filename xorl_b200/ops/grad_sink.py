@@ -13,12 +13,15 @@ import torch
 from . import _lib
 
 
-def grad_target(p: torch.Tensor):
+def grad_target(p: torch.Tensor, on_side: bool = False):
     """(buffer view or None, fresh) — ``fresh`` means nothing has been written yet in this
-    backward pass, so the first writer may overwrite instead of accumulate."""
+    backward pass, so the first writer may overwrite instead of accumulate.  ``on_side``: the caller writes on
+    the weight-gradient stream.  Any other writer of a buffer with a product pending there waits for it first."""
     buf = getattr(p, "_xb_grad_buf", None)
     if buf is None:
         return None, False
+    if not on_side and _wgrad_pending and getattr(p, "_xb_grad_side", None) == _wgrad_joins:
+        join_wgrad_stream()
     return buf, getattr(p, "_xb_grad_fresh", False)
 
 
@@ -76,6 +79,7 @@ import os as _os
 _WGRAD_OVERLAP = _os.environ.get("XORL_B200_WGRAD_STREAM", "1") == "1"
 _wgrad_stream = {}
 _wgrad_pending = False
+_wgrad_joins = 0         # joins so far: products that a parameter noted before the last one have been waited for
 
 
 def wgrad_stream(device: torch.device):
@@ -89,15 +93,18 @@ def wgrad_stream(device: torch.device):
     return st
 
 
-def note_wgrad_issued() -> None:
+def note_wgrad_issued(p: torch.Tensor) -> None:
+    """The gradient of ``p`` is being written on the side stream."""
     global _wgrad_pending
     _wgrad_pending = True
+    p._xb_grad_side = _wgrad_joins
 
 
 def join_wgrad_stream() -> None:
     """Makes the current stream wait for every weight-gradient GEMM issued on the side stream."""
-    global _wgrad_pending
+    global _wgrad_pending, _wgrad_joins
     if _wgrad_pending:
         for st in _wgrad_stream.values():
             _lib.current_stream().wait_stream(st)
         _wgrad_pending = False
+        _wgrad_joins += 1
