@@ -370,6 +370,75 @@ def test_moe_plan_matches_the_sorting_path(S, E):
     assert _lib.read_status()[0] == 0
 
 
+def _moe_inputs(T, E, k, H=64, I=64):
+    from types import SimpleNamespace
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *shape: (torch.randn(*shape, generator=gen, device="cuda") * 0.1).bfloat16()
+    experts = SimpleNamespace(gate_up_proj=rnd(E, H, 2 * I), down_proj=rnd(E, I, H))
+    ids = torch.rand(T, E, generator=gen, device="cuda").topk(k, -1)[1]
+    return rnd(T, H), torch.rand(T, k, generator=gen, device="cuda"), ids, experts
+
+
+@pytest.mark.parametrize("bad", [-1, 8, 2 ** 31 - 1, -2 ** 40])
+@pytest.mark.parametrize("T", [1, 700])
+def test_expert_id_out_of_range_is_refused(T, bad):
+    from xorl_b200.ops import moe
+    x, w, ids, experts = _moe_inputs(T, 8, 2)
+    good = moe.local_moe_forward(x, w, ids, experts, 8)
+    broken = ids.clone()
+    broken[T // 2, 1] = bad
+    with pytest.raises(RuntimeError, match="1 of %d expert ids" % (2 * T)):
+        moe.local_moe_forward(x, w, broken, experts, 8)
+    assert torch.equal(moe.local_moe_forward(x, w, ids, experts, 8), good)
+
+
+def test_slots_without_a_row_touch_no_other_token():
+    """Where nobody can raise (a captured graph): NaN for the token of the slot, in both directions, and the
+    values of the clean plan for every other token."""
+    from xorl_b200.ops import moe
+    T, E, k = 300, 8, 2
+    x, w, ids, _ = _moe_inputs(T, E, k)
+    w[17, 1] = 0.0                                            # a weight of zero hides nothing
+    rows = moe.buffer_rows(T * k, E)
+    dout = torch.randn_like(x)
+
+    def run(ids):
+        dest, _, slot = moe.sort_plan(ids.reshape(-1), E, rows)
+        xi, wi = x.clone().requires_grad_(), w.clone().requires_grad_()
+        y = moe._Combine.apply(moe._Permute.apply(xi, dest.view(T, k), slot), wi, dest.view(T, k), slot)
+        y.backward(dout)
+        return y.detach(), xi.grad, wi.grad
+
+    broken = ids.clone()
+    broken[17, 1], broken[250, 0] = E, -3
+    hit = torch.zeros(T, dtype=torch.bool, device="cuda")
+    hit[[17, 250]] = True
+    clean, got = run(ids), run(broken)
+    for c, g in zip(clean[:2], got[:2]):
+        assert g[hit].isnan().all() and torch.equal(g[~hit], c[~hit])
+    lost = broken != ids
+    assert got[2][lost].isnan().all() and torch.equal(got[2][~lost], clean[2][~lost])
+
+
+def test_router_on_logits_that_are_not_numbers_is_refused():
+    from xorl_b200.models import ModelConfig
+    from xorl_b200.models.context import StepContext
+    from xorl_b200.models.moe import MoEBlock
+    cfg = ModelConfig.from_dict(dict(model_type="qwen3_moe", vocab_size=64, hidden_size=64, num_hidden_layers=1,
+                                     num_attention_heads=2, num_key_value_heads=2, head_dim=32, intermediate_size=64,
+                                     num_experts=8, num_experts_per_tok=2, moe_intermediate_size=64))
+    block = MoEBlock(cfg, 0, dtype=torch.bfloat16, device="cuda")
+    for p in block.parameters():
+        torch.nn.init.normal_(p, 0.0, 0.02)
+    x = torch.randn(50, 64, device="cuda").bfloat16()
+    ctx = StepContext(cu_seqlens=torch.tensor([0, 50], device="cuda", dtype=torch.int32),
+                      position_ids=torch.arange(50, device="cuda"), causal=True, training=True)
+    assert block(x, ctx).isfinite().all()
+    x[7, 3] = float("nan")
+    with pytest.raises(RuntimeError, match="expert ids"):
+        block(x, ctx)
+
+
 @pytest.mark.parametrize("T,E,k,renorm,scale", [(1, 1, 1, True, 1.0), (300, 8, 2, True, 1.0), (513, 128, 8, True, 2.5),
                                                 (77, 60, 3, False, 0.5), (64, 512, 32, True, 1.0)])
 def test_chosen_weights_and_balancing_loss_match_torch(T, E, k, renorm, scale):

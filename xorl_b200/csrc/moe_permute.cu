@@ -7,7 +7,7 @@
 //   xb_moe_gather_rows   out[r] = scale[r] * in[src[r]]   (src[r] < 0 -> zero row)
 //                        forward permutation into expert-sorted, segment-aligned rows; backward of
 //                        the weighted combine
-//   xb_moe_gather_sum    out[t] = sum_j w[t,j] * in[idx[t,j]]   (fp32 accumulation)
+//   xb_moe_gather_sum    out[t] = sum_j w[t,j] * in[idx[t,j]]   (fp32 accumulation; idx < 0 -> NaN)
 //                        weighted combine of the k expert outputs of a token; backward of the
 //                        permutation (w = null)
 //   xb_moe_slot_dots     dw[t,j] = <dout[t], y[idx[t,j]]>        gradient of the routing weights
@@ -61,12 +61,14 @@ gather_sum_kernel(uint4* __restrict__ out, long long ld_out, const uint4* __rest
                   const long long* __restrict__ idx, const float* __restrict__ w, int T, int k, int vecs) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  // what a slot without a row contributes: no number, rather than some other token's row
+  const uint4 nan8 = make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
   for (int t = warp; t < T; t += nwarps) {
     for (int v = lane; v < vecs; v += 32) {
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       for (int j = 0; j < k; ++j) {
         const long long r = idx[(long long)t * k + j];
-        fma8(acc, in[r * ld_in + v], w ? w[(long long)t * k + j] : 1.f);
+        fma8(acc, r >= 0 ? in[r * ld_in + v] : nan8, w ? w[(long long)t * k + j] : 1.f);
       }
       out[(long long)t * ld_out + v] = pack8(acc);
     }
@@ -100,9 +102,12 @@ slot_dots_kernel(float* __restrict__ dw, const uint4* __restrict__ dout, long lo
 __global__ void __launch_bounds__(256)
 combine_bwd_kernel(uint4* __restrict__ dy, long long ld_dy, float* __restrict__ dw, const uint4* __restrict__ dout,
                    long long ld_do, const uint4* __restrict__ y, long long ld_y, const int* __restrict__ slot,
-                   const float* __restrict__ w, int k, int rows, int vecs) {
+                   const long long* __restrict__ dest, const float* __restrict__ w, long long slots, int k, int rows,
+                   int vecs) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < slots; s += (long long)gridDim.x * blockDim.x)
+    if (dest[s] < 0) dw[s] = __int_as_float(0x7fc00000);     // no row: nobody below writes it
   for (int r = warp; r < rows; r += nwarps) {
     const int s = slot[r];
     uint4* o = dy + (long long)r * ld_dy;
@@ -158,14 +163,16 @@ XB_API int xb_moe_gather_slots(void* out, long long ld_out, const void* in, long
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
-// y, dy [rows, width]; dout [T, width]; w, dw fp32 [T * k]; slot int32 [rows] names every slot once
+// y, dy [rows, width]; dout [T, width]; w, dw fp32 [slots], slots = T * k; slot int32 [rows] names every slot
+// once whose dest int64 [slots] is not negative; the others' dw is NaN
 XB_API int xb_moe_combine_bwd(void* dy, long long ld_dy, float* dw, const void* dout, long long ld_do, const void* y,
-                              long long ld_y, const int* slot, const float* w, int k, int rows, int width,
-                              void* stream) {
+                              long long ld_y, const int* slot, const long long* dest, const float* w, long long slots,
+                              int k, int rows, int width, void* stream) {
   if (rows <= 0) return 0;
   if (width % 8 || ld_dy % 8 || ld_do % 8 || ld_y % 8 || k <= 0) return -1;
   combine_bwd_kernel<<<grid_for(rows), 256, 0, (cudaStream_t)stream>>>(
-      (uint4*)dy, ld_dy / 8, dw, (const uint4*)dout, ld_do / 8, (const uint4*)y, ld_y / 8, slot, w, k, rows, width / 8);
+      (uint4*)dy, ld_dy / 8, dw, (const uint4*)dout, ld_do / 8, (const uint4*)y, ld_y / 8, slot, dest, w, slots, k, rows,
+      width / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -6,7 +6,8 @@
 // 16 experts and 4096 tokens went from 14.0 to 11.6 ms, one of the small preset from 7.3 to 5.5 ms.
 //
 //   xb_moe_plan          expert ids -> row of every slot in the expert-sorted, 128-row-aligned buffer,
-//                        segment table, and the inverse map; stable, no host synchronisation
+//                        segment table, inverse map and number of placed slots; stable, no host
+//                        synchronisation
 //   xb_moe_renorm        w = scale * p / max(sum p, 1e-20) of the chosen probabilities
 //   xb_moe_renorm_bwd    its gradient, scattered into a dense [T, E]
 //   xb_moe_route_bwd     gradient of scores -> top-k weights (moe_route.cu) with respect to the logits
@@ -39,7 +40,7 @@ plan_count_kernel(const long long* __restrict__ ids, int S, int E, int chunk, in
 __global__ void __launch_bounds__(PLAN_THREADS)
 plan_place_kernel(const long long* __restrict__ ids, int S, int E, int chunk, int align, int rows,
                   const int* __restrict__ hist, long long* __restrict__ dest, int* __restrict__ seg,
-                  int* __restrict__ slot_of_row, int* status) {
+                  int* __restrict__ slot_of_row, int* __restrict__ placed) {
   extern __shared__ int sh[];
   int* total = sh;               // [E]
   int* start = sh + E;           // [E + 1] aligned segment starts
@@ -72,6 +73,13 @@ plan_place_kernel(const long long* __restrict__ ids, int S, int E, int chunk, in
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (lane == 0) start[E] = carry;
+    if (placed && blockIdx.x == 0) {
+      int n = 0;
+      for (int e = lane; e < E; e += 32) n += total[e];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+      if (lane == 0) *placed = n;
+    }
   }
   // this warp's part of the chunk: whole groups of 32 slots
   const int c0 = blockIdx.x * chunk, c1 = min(S, c0 + chunk);
@@ -97,8 +105,7 @@ plan_place_kernel(const long long* __restrict__ ids, int S, int E, int chunk, in
     if (s < w1) {
       e = ids[s];
       if (e < 0 || e >= E) {
-        xb_report(status, XB_ERR_BOUNDS, XB_K_GROUPED_GEMM, 900);
-        dest[s] = 0;             // a row that exists
+        dest[s] = -1;
         e = -1;
       }
     }
@@ -265,17 +272,18 @@ XB_API int xb_moe_plan_workspace(int S, int E) {
   return nb * E;
 }
 
-// ids int64 [S] -> dest int64 [S], seg int32 [E + 1], slot_of_row int32 [rows] (-1: padding).  rows must
-// hold every segment: at least S + E * (align - 1).
+// ids int64 [S] -> dest int64 [S] (-1: the id is no expert), seg int32 [E + 1], slot_of_row int32 [rows] (-1:
+// padding), placed int32 [1] (or null): how many ids were experts.  rows must hold every segment: at least
+// S + E * (align - 1).
 XB_API int xb_moe_plan(const long long* ids, int S, int E, int align, int rows, int* workspace, long long* dest,
-                       int* seg, int* slot_of_row, void* stream) {
+                       int* seg, int* slot_of_row, int* placed, void* stream) {
   if (E <= 0 || E > PLAN_MAX_E || S < 0 || align <= 0 || rows < S) return -1;
   const int chunk = plan_chunk(S);
   const int nb = S > 0 ? (S + chunk - 1) / chunk : 1;
   cudaStream_t st = (cudaStream_t)stream;
   plan_count_kernel<<<nb, PLAN_THREADS, E * sizeof(int), st>>>(ids, S, E, chunk, workspace);
   plan_place_kernel<<<nb, PLAN_THREADS, (E * (2 + PLAN_WARPS) + 1) * sizeof(int), st>>>(
-      ids, S, E, chunk, align, rows, workspace, dest, seg, slot_of_row, xb_status_ptr());
+      ids, S, E, chunk, align, rows, workspace, dest, seg, slot_of_row, placed);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

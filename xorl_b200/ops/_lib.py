@@ -82,9 +82,9 @@ _SIGNATURES = {
     "xb_moe_gather_sum": [P, L, P, L, P, P, I, I, I, P],
     "xb_moe_slot_dots": [P, P, L, P, L, P, I, I, I, P],
     "xb_moe_gather_slots": [P, L, P, L, P, I, I, I, P],
-    "xb_moe_combine_bwd": [P, L, P, P, L, P, L, P, P, I, I, I, P],
+    "xb_moe_combine_bwd": [P, L, P, P, L, P, L, P, P, P, L, I, I, I, P],
     "xb_moe_plan_workspace": [I, I],
-    "xb_moe_plan": [P, I, I, I, I, P, P, P, P, P],
+    "xb_moe_plan": [P, I, I, I, I, P, P, P, P, P, P],
     "xb_moe_renorm": [P, P, I, I, I, F, P],
     "xb_moe_renorm_bwd": [P, P, P, P, I, I, I, I, F, P],
     "xb_moe_route_bwd": [P, P, L, P, P, P, P, I, I, I, I, I, F, P],

@@ -293,10 +293,10 @@ def aligned_sort_indices(expert_ids: torch.Tensor, num_experts: int, align: int 
 PLAN_MAX_EXPERTS = 1024
 
 
-def sort_plan(expert_ids: torch.Tensor, num_experts: int, rows: int):
+def sort_plan(expert_ids: torch.Tensor, num_experts: int, rows: int, placed: Optional[torch.Tensor] = None):
     """``aligned_sort_indices`` for int64 ids on the GPU in two launches, without the host waiting for the
     counts: (dest int64 [S], seg int32 [E+1], slot_of_row int32 [rows], -1 for padding rows).  An id
-    outside the experts is placed nowhere (``dest`` 0) and raises the status word."""
+    outside the experts is placed nowhere (``dest`` -1); ``placed`` int32 [1] receives the number of the others."""
     global _launches
     S, dev = expert_ids.numel(), expert_ids.device
     lib = _lib.cuda_lib()
@@ -305,9 +305,37 @@ def sort_plan(expert_ids: torch.Tensor, num_experts: int, rows: int):
     seg = torch.empty(num_experts + 1, device=dev, dtype=torch.int32)
     slot_of_row = torch.empty(rows, device=dev, dtype=torch.int32)
     _lib.check(lib.xb_moe_plan(expert_ids.data_ptr(), S, num_experts, SEG_ALIGN, rows, ws.data_ptr(), dest.data_ptr(),
-                               seg.data_ptr(), slot_of_row.data_ptr(), _lib.stream_ptr()), "xb_moe_plan")
+                               seg.data_ptr(), slot_of_row.data_ptr(), _lib.ptr(placed), _lib.stream_ptr()), "xb_moe_plan")
     _launches += 2
     return dest, seg, slot_of_row
+
+
+class _PlacedCheck:
+    """Raises when a plan could not place every slot (an id that is no expert: a bad replay record, or the
+    router's choice among logits that are not numbers).  The count travels to the host behind the plan and is read
+    once the expert MLP has been launched: the host waits for the plan only, with the GPU busy.  A stream under
+    capture cannot be waited for; the rows of such tokens are NaN there as anywhere."""
+
+    def __init__(self, device):
+        self.count = torch.empty(1, device=device, dtype=torch.int32)
+        self.event = None
+
+    def send(self) -> None:
+        if torch.cuda.is_current_stream_capturing():
+            return
+        self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        self.host.copy_(self.count, non_blocking=True)
+        self.event = torch.cuda.Event()
+        self.event.record(_lib.current_stream())
+
+    def raise_if_short(self, slots: int, num_experts: int) -> None:
+        if self.event is None:
+            return
+        self.event.synchronize()
+        missing = slots - self.host.item()
+        if missing:
+            raise RuntimeError(f"{missing} of {slots} expert ids lie outside [0, {num_experts}): "
+                               "router logits that are not numbers, or bad recorded choices")
 
 
 def buffer_rows(num_slots: int, num_experts: int, align: int = SEG_ALIGN) -> int:
@@ -580,8 +608,9 @@ class _Combine(torch.autograd.Function):
         dy = torch.empty_like(y)
         dw = torch.empty_like(w)
         _lib.check(_lib.cuda_lib().xb_moe_combine_bwd(dy.data_ptr(), H, dw.data_ptr(), dout.data_ptr(), H,
-                                                      y.data_ptr(), H, slot_of_row.data_ptr(), w.data_ptr(),
-                                                      dest.shape[1], rows, H, _lib.stream_ptr()),
+                                                      y.data_ptr(), H, slot_of_row.data_ptr(), dest.data_ptr(),
+                                                      w.data_ptr(), dest.numel(), dest.shape[1], rows, H,
+                                                      _lib.stream_ptr()),
                    "xb_moe_combine_bwd")
         _launches += 1
         return dy, dw, None, None
@@ -621,11 +650,15 @@ def local_moe_forward(x: torch.Tensor, weights: torch.Tensor, indices: torch.Ten
     flat = indices.reshape(-1)
     if (_permute_kernels_ok(x) and not canonical and flat.dtype == torch.int64 and num_experts <= PLAN_MAX_EXPERTS
             and rows < 2 ** 31):
-        dest, seg, slot_of_row = sort_plan(flat.contiguous(), num_experts, rows)
+        check = _PlacedCheck(x.device)
+        dest, seg, slot_of_row = sort_plan(flat.contiguous(), num_experts, rows, check.count)
+        check.send()
         dest2 = dest.view(T, k)
         buf = _Permute.apply(x, dest2, slot_of_row)
         y = expert_mlp_aligned(buf, seg, experts.gate_up_proj, experts.down_proj, **experts_mlp_kwargs(experts))
-        return _Combine.apply(y, weights, dest2, slot_of_row)
+        out = _Combine.apply(y, weights, dest2, slot_of_row)
+        check.raise_if_short(T * k, num_experts)
+        return out
     dest, seg, _ = aligned_sort_indices(flat, num_experts)
     token_of_slot = torch.arange(T, device=x.device).repeat_interleave(k)
     buf = x.new_zeros((rows, H)).index_copy(0, dest, x.index_select(0, token_of_slot))
