@@ -351,6 +351,42 @@ def test_hd64_attention_loses_no_precision(lens, Hq, Hkv, causal, do_norm):
         assert eg <= 1.02 * er + (2 ** -9 if name in ("dwq", "dwk") else 2e-5), (name, eg, er)
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("lens,causal", [([70, 65, 1, 200, 127], True), ([129, 300, 63], False), ([64, 128, 1], True)])
+def test_hd64_documents_do_not_see_each_others_infinities(lens, causal, value):
+    """One document holds a non-finite value, and so do rows behind the last document.  Tiles of its neighbours
+    run on into those rows; outputs and gradients of every other document have the bits of the clean call."""
+    from xorl_b200.ops import attention as A
+    torch.manual_seed(2)
+    Hq, Hkv, D, tail = 4, 2, 64, 30
+    n = sum(lens)
+    cu = _make_cu(lens)
+    base = torch.randn(n + tail, (Hq + 2 * Hkv) * D, device=DEV, dtype=torch.bfloat16)
+    go = torch.randn(n + tail, Hq * D, device=DEV, dtype=torch.bfloat16)
+    cos, sin = torch.ones(n + tail, D // 2, device=DEV), torch.zeros(n + tail, D // 2, device=DEV)
+
+    def run(x, g):
+        x = x.clone().requires_grad_()
+        y = A.qk_norm_rope_attention(x, None, None, cos, sin, cu, Hq, Hkv, D, 1e-6, causal)
+        y.backward(g)
+        return y.detach(), x.grad
+
+    before = A.launch_count()
+    clean = run(base, go)
+    assert A.launch_count() > before
+    for bad in range(len(lens)):
+        s = sum(lens[:bad])
+        x, g = base.clone(), go.clone()
+        for t in (x, g):
+            t[s] = t[s + lens[bad] - 1] = t[n:] = value
+        got = run(x, g)
+        keep = torch.ones(n + tail, dtype=torch.bool, device=DEV)
+        keep[s:s + lens[bad]] = keep[n:] = False
+        for a, b in zip(got, clean):
+            assert torch.equal(a[keep], b[keep])
+        assert not got[1][n:].any()                           # rows of no document have no gradient
+
+
 def test_status_words_clean():
     from xorl_b200.ops import _lib
     assert _lib.read_status()[0] == 0

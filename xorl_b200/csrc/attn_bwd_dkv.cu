@@ -83,7 +83,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   {
     int acc = 0;
     for (int b = 0; b < p.num_seqs; ++b) {
-      const int s0 = p.cu_seqlens[b], s1 = p.cu_seqlens[b + 1];
+      const int s0 = p.cu_seqlens[b], s1 = min(p.cu_seqlens[b + 1], p.T);
       const int nt = (s1 - s0 + BKV - 1) / BKV;
       if (tile_id < acc + nt) {
         seq = b; kt = tile_id - acc; seq_start = s0; seq_len = s1 - s0;
@@ -290,8 +290,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int i = 0; i < 32; ++i) {
             const float pe = i < nvis ? xb_ex2(fmaf(__uint_as_float(a[i]), p.scale_log2, -lse)) : 0.f;
             pv[i] = pe;
-            ds[i] = pe * (__uint_as_float(b[i]) - delta);
+            ds[i] = i < nvis ? pe * (__uint_as_float(b[i]) - delta) : 0.f;    // dP of another sequence may be Inf
           }
+        }
+        if (q_lo + BQ > seq_len) {                   // CTA-uniform
+          // rows of the next sequence: the products sum over the queries, and their scores are done
+          if (!__all_sync(0xffffffffu, mbar_wait(&bars->q_full[s], ph, abort_flag, p.status, XB_K_ATTN_BWD, 930 + s))) {
+            ok = false;
+            break;
+          }
+          if (!row_valid) xb_zero_row128(smem + (half ? at_do(s) : at_q(s)) + r * 128);
         }
       }
       // the dV / dK MMAs of step t-2 read this P / dS buffer: wait until they are done

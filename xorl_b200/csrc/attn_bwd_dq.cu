@@ -72,7 +72,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   {
     int acc = 0;
     for (int b = 0; b < p.num_seqs; ++b) {
-      const int s0 = p.cu_seqlens[b], s1 = p.cu_seqlens[b + 1];
+      const int s0 = p.cu_seqlens[b], s1 = min(p.cu_seqlens[b + 1], p.T);
       const int nt = (s1 - s0 + BQ - 1) / BQ;
       if (tile_id < acc + nt) {
         seq = b; qt = nt - 1 - (tile_id - acc); seq_start = s0; seq_len = s1 - s0;
@@ -274,6 +274,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       if (!__all_sync(0xffffffffu, mbar_wait(&bars->ds_free[b], ph ^ 1, abort_flag, p.status, XB_K_ATTN_BWD, 710 + b))) {
         ok = false;
         break;
+      }
+      if (j * BKV + BKV > seq_len) {                  // CTA-uniform
+        // keys of the next sequence: dS K sums over the keys, and their scores are done
+        const int st = j % NS;
+        if (!__all_sync(0xffffffffu, mbar_wait(&bars->kv_full[st], (j / NS) & 1, abort_flag, p.status, XB_K_ATTN_BWD, 730 + st))) {
+          ok = false;
+          break;
+        }
+        if (half == 0 && r < BKV && j * BKV + r >= seq_len)
+          xb_zero_row128(smem + SMEM_KV + st * 2 * KV_CHUNK_BYTES + r * 128);
       }
       uint8_t* sd = smem + SMEM_DS + b * DS_BUF + r * 128;
 #pragma unroll

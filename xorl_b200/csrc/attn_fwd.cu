@@ -68,7 +68,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   {
     int acc = 0;
     for (int b = 0; b < p.num_seqs; ++b) {
-      const int s0 = p.cu_seqlens[b], s1 = p.cu_seqlens[b + 1];
+      const int s0 = p.cu_seqlens[b], s1 = min(p.cu_seqlens[b + 1], p.T);
       const int nt = (s1 - s0 + BQ - 1) / BQ;
       if (tile_id < acc + nt) {
         seq = b; qt = tile_id - acc; seq_start = s0; seq_len = s1 - s0;
@@ -292,6 +292,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           }
           tc_wait_st();
         }
+      }
+      if (col0 + BKV > seq_len) {
+        // the tile runs on into the next sequence, whose P is 0: its V may hold no infinities or NaN
+        if (!__all_sync(0xffffffffu, mbar_wait(&bars->v_full[s], (j >> 1) & 1, abort_flag, p.status, XB_K_ATTN_FWD, 330 + s))) {
+          ok = false;
+          break;
+        }
+        if (col0 + r >= seq_len) xb_zero_row128(smem + SMEM_V + s * CHUNK_BYTES + r * 128);
       }
       // P (bf16) -> shared memory, 128B-swizzled K-major: 16-byte slot index XOR (row & 7)
 #pragma unroll

@@ -359,6 +359,12 @@ __device__ __forceinline__ float xb_ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Zeroes one 128-byte row of a swizzled tile.  Tiles of a short sequence hold rows of the next one; products that
+// sum over such rows multiply them by 0, and 0 x Inf is NaN.
+__device__ __forceinline__ void xb_zero_row128(uint8_t* row) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) reinterpret_cast<uint4*>(row)[i] = make_uint4(0, 0, 0, 0);
+}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
