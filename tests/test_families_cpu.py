@@ -500,3 +500,30 @@ def test_causal_conv1d_tensor_form_matches_per_document_convolution():
     ref = torch.nn.functional.silu(causal_depthwise_conv(x, w, cu) + b)
     torch.testing.assert_close(y[:33], ref[:33], rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(y[35], torch.nn.functional.silu(w[:, 3] * x[35] + b), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("where", ["module", "all", "all pre", "replaced"])
+def test_mlp_calls_its_projection_when_someone_listens(where, grad):
+    """The fused projection + activation stands in for the module's call only where nothing can tell."""
+    from torch.nn.modules import module as M
+    from xorl_b200.models.layers import MLP
+    mlp = MLP(16, 32, tensor_parallel=False)
+    up, seen, handle = mlp.gate_up_proj, [], None
+    note = lambda m, *rest: seen.append(m)
+    if where == "module":
+        handle = up.register_forward_hook(note)
+    elif where == "all":
+        handle = M.register_module_forward_hook(note)
+    elif where == "all pre":
+        handle = M.register_module_forward_pre_hook(note)
+    else:
+        call = up.forward
+        up.forward = lambda x: (note(up), call(x))[1]
+    try:
+        with torch.set_grad_enabled(grad):
+            mlp(torch.randn(3, 16))
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert up in seen

@@ -12,6 +12,7 @@ from typing import Optional
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from ..ops import activation as act_ops
 from ..ops import attention as attn_ops
@@ -196,6 +197,13 @@ class Attention(nn.Module):
         return q, k, v
 
 
+def _calls_nothing_else(m: nn.Module) -> bool:
+    """A call of ``m`` is ``Linear.forward`` and nothing more: no other class, no replaced ``forward``, no hook of
+    its own or of all modules."""
+    return not (type(m) is not Linear or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks
+                or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook())
+
+
 class MLP(nn.Module):
     """SwiGLU feed-forward with a fused gate_up projection ``[2I, H]`` (gate rows first)."""
 
@@ -237,7 +245,6 @@ class MLP(nn.Module):
             x = copy_to_tp(x, self.tp_group)
             return reduce_from_tp(self.down_proj(self._act(self.gate_up_proj(x))), self.tp_group)
         up = self.gate_up_proj
-        if type(up) is Linear and up.bias is None and self.swiglu_limit is None \
-                and not (up._forward_hooks or up._forward_pre_hooks or up._backward_hooks or up._backward_pre_hooks):
+        if up.bias is None and self.swiglu_limit is None and _calls_nothing_else(up):
             return self.down_proj(act_ops.linear_swiglu(x, up.weight))
         return self.down_proj(self._act(self.gate_up_proj(x)))
