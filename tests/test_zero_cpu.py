@@ -102,6 +102,38 @@ def test_engine_without_recompute_matches_autograd():
         assert abs(a - b) < 1e-5 and abs(a - c) < 1e-5, (ref, got, got2)
 
 
+def test_offloaded_embedding_output_is_not_kept_by_its_graph():
+    """With activations offloaded, nothing holds the embedding's output while the head runs."""
+    from torch.multiprocessing.reductions import StorageWeakRef
+    from xorl_b200.models.config import preset
+    from xorl_b200.models.decoder import DecoderLM
+    from xorl_b200.parallel.state import get_parallel_state, init_parallel_state, reset_parallel_state
+    from xorl_b200.parallel.zero import Zero3Engine
+    reset_parallel_state()
+    init_parallel_state(device_type="cpu")
+    m = DecoderLM(preset("tiny-qwen3"), dtype=torch.float32, device="meta")
+    eng = Zero3Engine(m, get_parallel_state(), compute_dtype=torch.float32, device=torch.device("cpu"), seed=0,
+                      activation_offload=True)
+    alive, embed, head = [], m.forward_embed, m.head_loss
+
+    def forward_embed(*a):
+        out = embed(*a)
+        alive.append(StorageWeakRef(out[0].untyped_storage()))
+        return out
+
+    def head_loss(*a, **kw):
+        assert alive and alive[0].expired()
+        return head(*a, **kw)
+
+    m.forward_embed, m.head_loss = forward_embed, head_loss
+    x, y = _data(0)
+    eng.forward_backward(x, y, grad_scale=1.0 / y.numel())
+    eng.finish_grad_sync()
+    root = next(g for g in eng.all_groups() if any("embed" in n for n, _ in g.named_params))
+    assert any(v.abs().sum() > 0 for (n, _), v in zip(root.named_params, root.param_views(root.grad_shard))
+               if "embed" in n)
+
+
 def test_muon_single_process_descends_and_orthogonalises():
     from xorl_b200.optim.muon import gram_newton_schulz, newton_schulz
     from xorl_b200.parallel.state import init_parallel_state, reset_parallel_state

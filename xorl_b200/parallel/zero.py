@@ -880,14 +880,21 @@ class Zero3Engine:
             join_wgrad_stream()
         return loss.detach(), tuple(a.grad if a is not None else None for a in head_in)
 
+    @staticmethod
+    def _edges(outputs):
+        """What a backward pass needs to know of ``outputs``, without their memory (an offloaded or released
+        activation is gone although its graph is kept)."""
+        return tuple(torch.autograd.graph.get_gradient_edge(o) if o is not None and o.requires_grad else None
+                     for o in outputs)
+
     def embed_backward(self, input_ids, ctx, dacts, emb=None) -> None:
-        """``emb``: the embedding's outputs with their graph; looked up again where the caller has not kept
-        them."""
+        """``emb``: where the embedding's outputs hang in their graph (``_edges``); looked up again where the
+        caller has not kept it."""
         if emb is None:
             with torch.enable_grad():
-                emb = self.model.forward_embed(input_ids, ctx)
+                emb = self._edges(self.model.forward_embed(input_ids, ctx))
         pairs = [(o, d) for o, d in zip(emb, dacts) if o is not None and d is not None]
-        if pairs and pairs[0][0].requires_grad:
+        if pairs:
             with torch.autograd.set_multithreading_enabled(False):
                 torch.autograd.backward([o for o, _ in pairs], [d for _, d in pairs])
         if self.is_cuda:
@@ -908,6 +915,7 @@ class Zero3Engine:
         with torch.enable_grad():
             emb = model.forward_embed(input_ids, ctx)
         acts = tuple(e.detach() if e is not None else None for e in emb)
+        emb = self._edges(emb)
         acts, saved = self.chunk_forward(layers, acts, ctx, keep_last_gathered=True)
         self._prepare_grad_buffers(root)
         loss_value, dacts = self.head_forward_backward(acts, labels, ctx, grad_scale, extra_loss_fn)
