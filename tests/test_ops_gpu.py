@@ -101,6 +101,60 @@ def test_fused_linear_ce():
     _close(w.grad, wr.grad, 5e-2, 0.03 * wr.grad.abs().max().item(), "dw")
 
 
+@pytest.mark.parametrize("kept_chunks", [0, 1, 2, 4, 9])
+@pytest.mark.parametrize("buffer", [None, "fresh", "adds"])
+@pytest.mark.parametrize("token_loss", [False, True])
+def test_lm_head_gradients_over_groups_of_chunks(kept_chunks, buffer, token_loss):
+    """Five chunks, the last one ragged, in groups of one, two (2 + 2 + 1), four (4 + 1) and all: hidden and weight
+    gradients, the latter also in an engine's fp32 buffer, and the memory that the logits take.  bf16 logits and
+    gradients of logits: each within 2^-9, 4e-3 of the norm together with the fp32 sums."""
+    from xorl_b200.ops.loss import fused_linear_cross_entropy, fused_linear_token_loss
+    torch.manual_seed(0)
+    T, H, V, chunk = 1100, 128, 1000, 256
+    h = (torch.randn(T, H, device=DEV) * 0.5).bfloat16().requires_grad_()
+    w = (torch.randn(V, H, device=DEV) * 0.05).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (T,), device=DEV)
+    labels[::9] = -100
+    start = torch.randn(V, H, device=DEV)
+    if buffer:
+        w._xb_grad_buf, w._xb_grad_fresh = start.clone(), buffer == "fresh"
+    kept = kept_chunks * chunk * V * 2
+    if token_loss:
+        loss, _, _ = fused_linear_token_loss(h, w, labels, lambda lp, mask: (-(lp * mask).sum(), {}), 1.0,
+                                             chunk_tokens=chunk, kept_logits_bytes=kept)
+    else:
+        loss = fused_linear_cross_entropy(h, w, labels, chunk_tokens=chunk, kept_logits_bytes=kept)
+    loss.backward()
+    hr, wr = h.detach().float().requires_grad_(), w.detach().float().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(hr @ wr.t(), labels, ignore_index=-100, reduction="sum")
+    ref.backward()
+    dw = w._xb_grad_buf - (start if buffer == "adds" else 0) if buffer else w.grad.float()
+    assert abs(loss.item() - ref.item()) < 4e-3 * ref.item()
+    for name, g, r in (("dh", h.grad.float(), hr.grad), ("dw", dw, wr.grad)):
+        assert (g - r).norm() < 4e-3 * r.norm(), (name, float((g - r).norm() / r.norm()))
+
+
+def test_lm_head_logits_stay_within_the_chunk_that_was_asked_for():
+    from xorl_b200.ops.loss import fused_linear_cross_entropy
+    T, H, V = 4096, 64, 16384
+    h = torch.randn(T, H, device=DEV).bfloat16().requires_grad_()
+    w = (torch.randn(V, H, device=DEV) * 0.05).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (T,), device=DEV)
+
+    def peak(**kw):
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        base = torch.cuda.memory_allocated()
+        fused_linear_cross_entropy(h, w, labels, **kw).backward()
+        h.grad = w.grad = None
+        return torch.cuda.max_memory_allocated() - base
+
+    slack = 4 * (V * H * 4 + T * H * 4)                       # gradients of weight and hidden states, in fp32
+    assert peak(chunk_tokens=256) < 256 * V * 2 + slack
+    assert peak(chunk_tokens=1024, kept_logits_bytes=0) < 1024 * V * 2 + slack
+    assert peak() > T * V * 2                                 # nothing asked for: all of it at once
+
+
 def test_embedding():
     from xorl_b200.ops.embedding import embedding
     torch.manual_seed(0)

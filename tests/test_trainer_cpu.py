@@ -233,3 +233,26 @@ def test_evaluation_on_an_unsupported_layout_is_refused_at_start_up(tmp_path, mo
     with pytest.raises(NotImplementedError, match="evaluation pass"):
         Trainer(args, model_config=preset("tiny-qwen3"))
     pstate.reset_parallel_state()
+
+
+def test_lm_head_logits_budget(monkeypatch):
+    """How many tokens' logit gradients the loss keeps: the default, a smaller chunk, an explicit budget, and a card
+    without the room."""
+    from xorl_b200.ops import loss as L
+    size = lambda T, chunk, kept=None, V=32000: (lambda b, k: (b.shape[0], k))(*L._logits_buffer(T, chunk, V, kept, "meta"))
+    assert size(100, 1024) == (100, 1024)
+    assert size(16384, 1024) == (16384, 16384)
+    assert size(16384, 1024, V=152064) == (4096, 4096)                      # 1.25 GiB
+    assert size(16384, 512) == (512, 512)                                   # less was asked for
+    assert size(16384, 2048, 0) == (2048, 2048)
+    assert size(16384, 512, 3 * 512 * 32000 * 2) == (1536, 1536)
+    assert size(0, 1024) == (0, 1024)
+    empty = torch.empty
+
+    def full(shape, **kw):
+        if shape[0] > 1024:
+            raise torch.OutOfMemoryError("no room")
+        return empty(shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", full)
+    assert size(16384, 1024) == (1024, 1024)

@@ -134,6 +134,7 @@ class TrainingArguments:
     moe_global_load_balancing: bool = False
     ce_mode: Optional[str] = None
     ce_num_chunks: int = 8
+    ce_kept_logits_mb: Optional[int] = None
     micro_batch_size: int = 1
     gradient_accumulation_steps: int = 1
     defer_grad_sync_in_accumulation: bool = False

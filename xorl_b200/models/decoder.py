@@ -157,6 +157,7 @@ class DecoderLM(nn.Module):
             if has_head:
                 self.norm.weight._xb_tp_reduce = True
         self.loss_chunk_tokens = 1024
+        self.loss_kept_logits_bytes = None      # see ops/loss.py
         self.cp_strategy = None
         self.ctx_defaults = {}          # copied into every StepContext.aux (ep_dispatch, ...)
         self.aux_loss_enabled = False   # MoE load-balancing loss (set by the trainer)
@@ -252,7 +253,8 @@ class DecoderLM(nn.Module):
                                         vocab_chunk=int(getattr(self, "distill_vocab_chunk", 16384))).sum()
             ce = loss_ops.fused_linear_cross_entropy(hidden, self.lm_head.weight, labels.reshape(-1), grad_scale,
                                                      self.loss_chunk_tokens,
-                                                     z_loss=float(getattr(self, "z_loss_coef", 0.0)))
+                                                     z_loss=float(getattr(self, "z_loss_coef", 0.0)),
+                                                     kept_logits_bytes=self.loss_kept_logits_bytes)
             ctx.aux["distill_kl"] = kl.detach() * grad_scale
             total = ce + kl * (weight * grad_scale)
             return (total, None) if return_token_losses else total
@@ -274,7 +276,8 @@ class DecoderLM(nn.Module):
         return loss_ops.fused_linear_cross_entropy(hidden, self.lm_head.weight, labels.reshape(-1),
                                                    grad_scale, self.loss_chunk_tokens,
                                                    z_loss=float(getattr(self, "z_loss_coef", 0.0)),
-                                                   return_token_losses=return_token_losses)
+                                                   return_token_losses=return_token_losses,
+                                                   kept_logits_bytes=self.loss_kept_logits_bytes)
 
     def unit_modules(self):
         """(name, modules) per ZeRO unit, in execution order.  The root unit (embedding, final

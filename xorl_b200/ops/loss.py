@@ -46,22 +46,35 @@ def ce_chunk_(logits: torch.Tensor, labels: torch.Tensor, grad_scale: float, wri
     return loss, lse
 
 
-# Memory that a loss may keep in gradients of logits.  The gradient GEMMs of the lm-head take several chunks
-# of tokens at once.  Per chunk the weight gradient would read and write its whole fp32 buffer (524 MB at
-# 32,000 x 4096) for 1024 tokens of math, 0.37 ms instead of 0.21, and the hidden gradient would have half as
-# many tiles as there are SMs.  Logits and loss stay per chunk, whose logits (65 MB there) fit the L2.
+# Memory that a loss may keep in gradients of logits where its caller set neither a budget nor a chunk size below
+# the default: a smaller chunk asks for less memory, and then one chunk is all there is.  The gradient GEMMs of
+# the lm-head take several chunks of tokens at once.  Per chunk the weight gradient would read and write its whole
+# fp32 buffer (524 MB at 32,000 x 4096) for 1024 tokens of math, 0.37 ms instead of 0.21, and the hidden gradient
+# would have half as many tiles as there are SMs.  Logits and loss stay per chunk, whose logits (65 MB there) fit
+# the L2.
+DEFAULT_CHUNK_TOKENS = 1024
 KEPT_LOGITS_BYTES = 5 << 28
 
 
-def _kept_chunks(T: int, chunk_tokens: int, ldv: int) -> int:
-    """Chunks of logit gradients that are kept for one pair of gradient GEMMs."""
-    return max(1, min(-(-T // chunk_tokens), KEPT_LOGITS_BYTES // (2 * chunk_tokens * ldv)))
+def _logits_buffer(T: int, chunk_tokens: int, ldv: int, kept_bytes: int | None, device):
+    """(bf16 buffer, tokens whose logit gradients it keeps for one pair of gradient GEMMs).  ``kept_bytes``: what
+    more than one chunk may take, 0 for one chunk, None for the rule above.  One chunk also where the card has
+    no room for more."""
+    if kept_bytes is None:
+        kept_bytes = KEPT_LOGITS_BYTES if chunk_tokens >= DEFAULT_CHUNK_TOKENS else 0
+    chunks = max(1, min(-(-T // chunk_tokens), kept_bytes // (2 * chunk_tokens * ldv)))
+    if chunks > 1:
+        try:
+            return torch.empty((min(chunks * chunk_tokens, T), ldv), device=device, dtype=torch.bfloat16), chunks * chunk_tokens
+        except torch.OutOfMemoryError:
+            pass
+    return torch.empty((min(chunk_tokens, T), ldv), device=device, dtype=torch.bfloat16), chunk_tokens
 
 
 class _FusedLinearCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, labels, grad_scale, chunk_tokens, ignore_index, z_loss,
-                want_logprobs):
+                want_logprobs, kept_bytes):
         T, H = hidden.shape
         V = weight.shape[0]
         need_dh = hidden.requires_grad
@@ -73,8 +86,7 @@ class _FusedLinearCE(torch.autograd.Function):
             dw_local = torch.zeros((V, H), device=hidden.device, dtype=torch.float32)
         losses = torch.empty(T, device=hidden.device, dtype=torch.float32)
         ldv = (V + 7) // 8 * 8
-        kept = chunk_tokens * (_kept_chunks(T, chunk_tokens, ldv) if need_dw or need_dh else 1)     # tokens
-        buf = torch.empty((min(kept, T), ldv), device=hidden.device, dtype=torch.bfloat16)
+        buf, kept = _logits_buffer(T, chunk_tokens, ldv, kept_bytes if need_dw or need_dh else 0, hidden.device)
         first = True
         for s in range(0, T, chunk_tokens):
             e = min(T, s + chunk_tokens)
@@ -113,15 +125,18 @@ class _FusedLinearCE(torch.autograd.Function):
         if ctx.dw_local is not None:
             dw = deliver_param_grad(ctx.weight, ctx.dw_local * g)
         ctx.dh = ctx.dw_local = None
-        return dh, dw, None, None, None, None, None, None
+        return dh, dw, None, None, None, None, None, None, None
 
 
 def fused_linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor,
                                grad_scale: float = 1.0, chunk_tokens: int = 1024,
                                ignore_index: int = IGNORE_INDEX, z_loss: float = 0.0,
-                               return_token_losses: bool = False):
+                               return_token_losses: bool = False, kept_logits_bytes: int | None = None):
     """``grad_scale * sum_t CE(hidden[t] @ weight.T, labels[t])``.
 
+    ``chunk_tokens`` x vocabulary logits exist at a time.  With gradients several chunks of them are kept for one
+    pair of gradient GEMMs, up to ``kept_logits_bytes``; None: 1.25 GiB, or one chunk where ``chunk_tokens`` is
+    below its default.
     The lm-head weight gradient is produced during the forward call with the scale folded in, so
     the returned scalar must be back-propagated with an upstream gradient of 1 (``loss.backward()``
     directly on it or on a sum it is part of).
@@ -129,7 +144,8 @@ def fused_linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, label
     if hidden.is_cuda and hidden.dtype == torch.bfloat16 and hidden.shape[-1] % 8 == 0:
         loss, tl = _FusedLinearCE.apply(hidden.reshape(-1, hidden.shape[-1]), weight,
                                         labels.reshape(-1), float(grad_scale), int(chunk_tokens),
-                                        int(ignore_index), float(z_loss), bool(return_token_losses))
+                                        int(ignore_index), float(z_loss), bool(return_token_losses),
+                                        kept_logits_bytes)
         return (loss, tl) if return_token_losses else loss
     # CPU / fp32 lane: chunked plain torch, same reduction
     h2 = hidden.reshape(-1, hidden.shape[-1])
@@ -154,13 +170,13 @@ def fused_linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, label
 # --------------------------------------------------------------------------------------------
 def fused_linear_token_loss(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor,
                             loss_fn, grad_scale: float = 1.0, chunk_tokens: int = 1024,
-                            ignore_index: int = IGNORE_INDEX):
+                            ignore_index: int = IGNORE_INDEX, kept_logits_bytes: int | None = None):
     """``loss_fn(logprobs [T], mask [T]) -> (scalar, metrics)`` evaluated on the log-probabilities of
     the label tokens, without materialising the logits: pass 1 computes the log-probs chunk by
     chunk, the loss function runs on that small vector, pass 2 recomputes each logits chunk and
     back-propagates d(loss)/d(logprob) through the lm-head.  Returns (grad_scale * loss, logprobs,
     metrics); the hidden-state and lm-head gradients are produced like in
-    ``fused_linear_cross_entropy`` (back-propagate the returned scalar with gradient 1)."""
+    ``fused_linear_cross_entropy`` (back-propagate the returned scalar with gradient 1), in the same memory."""
     global _launches
     h2 = hidden.reshape(-1, hidden.shape[-1])
     lab = labels.reshape(-1)
@@ -194,12 +210,13 @@ def fused_linear_token_loss(hidden: torch.Tensor, weight: torch.Tensor, labels: 
     loss, metrics = loss_fn(lp_leaf, mask)
     (coef,) = torch.autograd.grad(loss, lp_leaf)
     return _TokenLossBackward.apply(h2, weight, lab, (-coef).contiguous(), float(grad_scale),
-                                    int(chunk_tokens), int(ignore_index), loss.detach()), lp, metrics
+                                    int(chunk_tokens), int(ignore_index), loss.detach(), kept_logits_bytes), lp, metrics
 
 
 class _TokenLossBackward(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, hidden, weight, labels, row_scale, grad_scale, chunk_tokens, ignore_index, loss_value):
+    def forward(ctx, hidden, weight, labels, row_scale, grad_scale, chunk_tokens, ignore_index, loss_value,
+                kept_bytes):
         global _launches
         T, H = hidden.shape
         V = weight.shape[0]
@@ -209,8 +226,7 @@ class _TokenLossBackward(torch.autograd.Function):
         dw_local = torch.zeros((V, H), device=hidden.device, dtype=torch.float32) \
             if (need_dw and tgt is None) else None
         ldv = (V + 7) // 8 * 8
-        kept = chunk_tokens * (_kept_chunks(T, chunk_tokens, ldv) if need_dw or need_dh else 1)     # tokens
-        buf = torch.empty((min(kept, T), ldv), device=hidden.device, dtype=torch.bfloat16)
+        buf, kept = _logits_buffer(T, chunk_tokens, ldv, kept_bytes if need_dw or need_dh else 0, hidden.device)
         lib = _lib.cuda_lib()
         scratch = torch.empty(min(chunk_tokens, T), device=hidden.device, dtype=torch.float32)
         first = True
@@ -246,7 +262,7 @@ class _TokenLossBackward(torch.autograd.Function):
         dh = ctx.dh * g.to(ctx.dh.dtype) if ctx.dh is not None else None
         dw = deliver_param_grad(ctx.weight, ctx.dw_local * g) if ctx.dw_local is not None else None
         ctx.dh = ctx.dw_local = None
-        return dh, dw, None, None, None, None, None, None
+        return dh, dw, None, None, None, None, None, None, None
 
 
 # --------------------------------------------------------------------------------------------

@@ -195,7 +195,8 @@ class ModelRunner:
             def head(h, res, labels, ctx, grad_scale, _c=closure, _h=holder):
                 hidden = self.model.forward_head(h, res, ctx)
                 loss, lp, metrics = fused_linear_token_loss(hidden, self.model.lm_head.weight, labels,
-                                                            _c, grad_scale, self.model.loss_chunk_tokens)
+                                                            _c, grad_scale, self.model.loss_chunk_tokens,
+                                                            kept_logits_bytes=self.model.loss_kept_logits_bytes)
                 _h["lp"], _h["metrics"] = lp, metrics
                 return loss
 
@@ -267,7 +268,8 @@ class ModelRunner:
             hidden = self.model.forward_head(h, res, ctx)
             fn = (lambda lp, mask: (lp.sum() * 0, {})) if zero_loss else closures[i]
             loss, lp, _ = fused_linear_token_loss(hidden, self.model.lm_head.weight, labels, fn, grad_scale,
-                                                  self.model.loss_chunk_tokens)
+                                                  self.model.loss_chunk_tokens,
+                                                  kept_logits_bytes=self.model.loss_kept_logits_bytes)
             lps[i] = lp
             return loss
 

@@ -118,6 +118,9 @@ class Trainer:
         if t.ce_num_chunks and t.ce_num_chunks > 0:
             self.model.loss_chunk_tokens = max(256, -(-int(a.data.sample_packing_sequence_len or 4096)
                                                       * t.micro_batch_size // t.ce_num_chunks))
+        if t.ce_kept_logits_mb is not None:
+            # gradients of logits that the lm-head's gradient GEMMs take at once, in MiB; 0: one chunk at a time
+            self.model.loss_kept_logits_bytes = max(0, int(t.ce_kept_logits_mb)) << 20
         if t.fsdp_sharded_lm_head_loss and getattr(self.ps, "lm_head_tp_size", 1) > 1:
             # tokens of the whole group per chunk of the streamed loss
             local = int(a.data.sample_packing_sequence_len or 4096) * t.micro_batch_size
