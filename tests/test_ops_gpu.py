@@ -343,6 +343,21 @@ def test_attention_128_against_the_single_backward_kernel(lens, Hq, Hkv, causal,
     assert _lib.read_status()[0] == 0
 
 
+def test_attention_128_takes_more_tiles_than_a_grid_is_high():
+    """66,000 documents of one token: every query sees its own key only."""
+    from xorl_b200.ops import attention as A
+    T, D = 66000, 128
+    cu = torch.arange(T + 1, device=DEV, dtype=torch.int32)
+    q, k, v, go = (torch.randn(T, 1, D, device=DEV, dtype=torch.bfloat16) for _ in range(4))
+    out, lse = A._attn_fwd(q, k, v, cu, True, D ** -0.5)
+    assert torch.equal(out, v)
+    dv = torch.empty_like(v)
+    dq, dk = A._attn_bwd(q, k, v, out, go, lse, cu, True, D ** -0.5, dv)
+    # P and dP - delta: the two fp32 sums over 128 products and the lse round differently
+    assert (dv.float() - go.float()).abs().max() <= 2 ** -8 * go.float().abs().max()
+    assert dq.abs().max() < 1e-4 and dk.abs().max() < 1e-4
+
+
 def _attention_float64(qkv, wq, wk, cos, sin, lens, Hq, Hkv, D, eps, causal):
     """The block in float64 without any rounding inside."""
     T = qkv.shape[0]

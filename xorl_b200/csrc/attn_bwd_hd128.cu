@@ -138,12 +138,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
        const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do, const Params p,
        const int split) {
-  const Where w = find_tile(p, blockIdx.y, false);
+  // one grid dimension, the other two end at 65,535
+  const unsigned group = (unsigned)(p.Hkv * split);
+  const Where w = find_tile(p, (int)(blockIdx.x / group), false);
   if (w.seq < 0) return;                                   // the whole cluster leaves
   const int k_start = p.k_starts ? p.k_starts[w.seq] : w.start;
   if (k_start < 0) return;                                 // this block takes no part in the call
   const int rank = split > 1 ? (int)cluster_ctarank() : 0;
-  const int kv_head = (int)blockIdx.x / split;
+  const int kv_head = (int)(blockIdx.x % group) / split;
   const int G = p.Hq / p.Hkv / split;
   const int head0 = kv_head * (p.Hq / p.Hkv) + rank * G;
   const int kv0 = w.tile * BT;                             // position inside the sequence
@@ -513,11 +515,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
        const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do, const Params p) {
   // the last (under a causal mask the longest) query tile of a sequence comes first
-  const Where w = find_tile(p, blockIdx.y, true);
+  const Where w = find_tile(p, (int)(blockIdx.x / (unsigned)p.Hq), true);
   if (w.seq < 0) return;
   const int k_start = p.k_starts ? p.k_starts[w.seq] : w.start;
   if (k_start < 0) return;
-  const int head = blockIdx.x;
+  const int head = (int)(blockIdx.x % (unsigned)p.Hq);
   const int kv_head = head / (p.Hq / p.Hkv);
   const int q0 = w.tile * BT;
   const int n_kv = (w.len + BT - 1) / BT;
@@ -778,7 +780,7 @@ int xb_attn_bwd_hd128(const void* q, const void* k, const void* v, const void* d
     return rc;
   const int full_tiles = (T + BT - 1) / BT;
   const int tiles = max_tiles > 0 ? max_tiles : full_tiles + num_seqs;
-  // With the heads as the fast dimension of the grids the long tiles of all heads start first: both kernels 680 ->
+  // With the heads as the fast index of the grids the long tiles of all heads start first: both kernels 680 ->
   // 592 us on one document of 4096 tokens, dK / dV 418 -> 316 us on four of 2048 with 4 KV heads, no change at
   // 16,384 tokens.
   // about three CTAs per SM even out the lengths of the key tiles under a causal mask
@@ -788,9 +790,10 @@ int xb_attn_bwd_hd128(const void* q, const void* k, const void* v, const void* d
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(Hkv * split, tiles); cfg.blockDim = dim3(dkv::NUM_THREADS);
+  if ((long long)tiles * Hq > 0x7fffffffll) return -1;
+  cfg.gridDim = dim3(Hkv * split * tiles); cfg.blockDim = dim3(dkv::NUM_THREADS);
   cfg.dynamicSmemBytes = dkv::SMEM_BYTES; cfg.stream = stream; cfg.attrs = attr; cfg.numAttrs = 1;
   if (cudaLaunchKernelEx(&cfg, dkv::kernel, m[0], m[1], m[2], m[3], p, split) != cudaSuccess) return -11;
-  dqk::kernel<<<dim3(Hq, tiles), dqk::NUM_THREADS, dqk::SMEM_BYTES, stream>>>(m[0], m[1], m[2], m[3], p);
+  dqk::kernel<<<Hq * tiles, dqk::NUM_THREADS, dqk::SMEM_BYTES, stream>>>(m[0], m[1], m[2], m[3], p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

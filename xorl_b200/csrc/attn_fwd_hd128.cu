@@ -56,15 +56,17 @@ struct __align__(8) Barriers {
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
        const __grid_constant__ CUtensorMap tmap_v, const Params p) {
-  // the last (under a causal mask the longest) tiles of a sequence come first, those of all heads together
+  // the last (under a causal mask the longest) tiles of a sequence come first, those of all heads together;
+  // one grid dimension, the other two end at 65,535
+  const int head = (int)(blockIdx.x % (unsigned)p.Hq), tile = (int)(blockIdx.x / (unsigned)p.Hq);
   int seq = -1, qt = 0, seq_start = 0, seq_len = 0;
   {
     int acc = 0;
     for (int b = 0; b < p.num_seqs; ++b) {
       const int s0 = p.cu_seqlens[b], s1 = p.cu_seqlens[b + 1];
       const int nt = (s1 - s0 + p.tile_rows - 1) / p.tile_rows;
-      if ((int)blockIdx.y < acc + nt) {
-        seq = b; qt = nt - 1 - ((int)blockIdx.y - acc); seq_start = s0; seq_len = s1 - s0;
+      if (tile < acc + nt) {
+        seq = b; qt = nt - 1 - (tile - acc); seq_start = s0; seq_len = s1 - s0;
         break;
       }
       acc += nt;
@@ -73,7 +75,6 @@ kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUten
   if (seq < 0) return;
   const int k_start = p.k_starts ? p.k_starts[seq] : seq_start;
   if (k_start < 0) return;                       // this query block takes no part in the call
-  const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hkv);
   const int q0 = qt * p.tile_rows;               // position of the first row inside the sequence
   // first key tile that any row of the first query tile sees under a sliding window
@@ -366,6 +367,7 @@ int xb_attn_fwd_hd128(const void* q, const void* k, const void* v, void* out, fl
   // tiles)
   const int bound = max_tiles > 0 ? max_tiles : (T + BT - 1) / BT;
   const int tiles = (pairs ? (bound + 1) / 2 : bound) + num_seqs;
-  kernel<<<dim3(Hq, tiles), NUM_THREADS, SMEM_BYTES, stream>>>(m[0], m[1], m[2], p);
+  if ((long long)Hq * tiles > 0x7fffffffll) return -1;
+  kernel<<<Hq * tiles, NUM_THREADS, SMEM_BYTES, stream>>>(m[0], m[1], m[2], p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
