@@ -456,6 +456,71 @@ def test_hd64_documents_do_not_see_each_others_infinities(lens, causal, value):
         assert not got[1][n:].any()                           # rows of no document have no gradient
 
 
+def _shifted(t):
+    """The same values behind an address that only the type's own alignment holds for."""
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    return flat[1:].view_as(t).copy_(t)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_qk_norm_rope_attention_on_shifted_buffers(D):
+    """Rotation tables (both widths), and for 64-wide heads activations and output gradients, at odd offsets."""
+    from xorl_b200.ops import attention as A
+    torch.manual_seed(3)
+    lens, Hq, Hkv = [100, 61], 4, 2
+    T, cu = sum(lens), _make_cu(lens)
+    base = torch.randn(T, (Hq + 2 * Hkv) * D, device=DEV, dtype=torch.bfloat16)
+    ws = [(1 + 0.1 * torch.randn(D, device=DEV)).bfloat16().requires_grad_() for _ in range(2)]
+    ang = torch.rand(T, D // 2, device=DEV) * 6
+    go = torch.randn(T, Hq * D, device=DEV, dtype=torch.bfloat16)
+
+    def run(x, cos, sin, g):
+        x.requires_grad_()
+        y = A.qk_norm_rope_attention(x, *ws, cos, sin, cu, Hq, Hkv, D)
+        return [y.detach(), *torch.autograd.grad(y, [x, *ws], g)]
+
+    cos, sin = ang.cos(), ang.sin()
+    clean = run(base.clone(), cos, sin, go)
+    for a, b in zip(run(base.clone(), _shifted(cos), _shifted(sin), go), clean):
+        assert torch.equal(a, b)
+    if D == 64:
+        for a, b in zip(run(base.clone(), cos, sin, _shifted(go)), clean):
+            assert torch.equal(a, b)
+        got = run(_shifted(base), cos, sin, go)               # served by the reference
+        for a, b in zip(got, clean):
+            assert (a.float() - b.float()).norm() < 2 ** -7 * b.float().norm()
+
+
+def test_hd64_attention_outside_the_kernels_range():
+    """A width that does not fit the heads stays an error; gradients of the tables, and of the gradient, exist."""
+    from xorl_b200.ops import attention as A
+    torch.manual_seed(4)
+    lens, Hq, Hkv, D = [40, 25], 4, 2, 64
+    T, cu = sum(lens), _make_cu(lens)
+    x = torch.randn(T, (Hq + 2 * Hkv) * D, device=DEV, dtype=torch.bfloat16)
+    ang = torch.rand(T, D // 2, device=DEV) * 6
+    cos, sin = ang.cos(), ang.sin()
+    with pytest.raises(RuntimeError):
+        A.qk_norm_rope_attention(x[:, :-D].contiguous(), None, None, cos, sin, cu, Hq, Hkv, D)
+    A.qk_norm_rope_attention(x, None, None, cos.requires_grad_(), sin, cu, Hq, Hkv, D).float().sum().backward()
+    assert cos.grad is not None and cos.grad.abs().sum() > 0
+    cos = cos.detach()
+
+    def second(fn):
+        leaf = x.clone().requires_grad_()
+        y = fn(leaf)
+        (g,) = torch.autograd.grad(y, leaf, torch.ones_like(y), create_graph=True)
+        return torch.autograd.grad(g.float().pow(2).sum(), leaf)[0].float()
+
+    before = A.launch_count()
+    got = second(lambda t: A.qk_norm_rope_attention(t, None, None, cos, sin, cu, Hq, Hkv, D))
+    assert A.launch_count() > before
+    ref = second(lambda t: A.qk_norm_rope_attention_reference(t, None, None, cos, sin, cu, Hq, Hkv, D, 1e-6, True,
+                                                              D ** -0.5))
+    # first and second derivative are the reference's on both sides
+    assert torch.equal(got, ref)
+
+
 def test_status_words_clean():
     from xorl_b200.ops import _lib
     assert _lib.read_status()[0] == 0

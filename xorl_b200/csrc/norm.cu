@@ -446,8 +446,11 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout_bf16,
       }
     }
     float c[PER], sn[PER];
-    load_f32<PER>(cosb + (size_t)t * HALF + lane * PER, c);
-    load_f32<PER>(sinb + (size_t)t * HALF + lane * PER, sn);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {             // the tables are the caller's: no alignment beyond their type's
+      c[i] = __ldg(cosb + (size_t)t * HALF + lane * PER + i);
+      sn[i] = __ldg(sinb + (size_t)t * HALF + lane * PER + i);
+    }
 #pragma unroll
     for (int g = 0; g < QKR_HPW; ++g) {
       const int h = h0 + g;

@@ -186,19 +186,23 @@ def _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv) -> bool:
     """What the head-dim-64 kernels take; everything else of that width runs in the reference (fp32
     matmuls per document; a training step of 2 such layers with 16 heads on 2045 tokens took 11.9 ms there and
     takes 4.2 ms here, 0.13 ms of it per layer in the three attention kernels).
-    The reference also serves function transforms and forward-mode derivatives."""
-    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape[0] > 0 and Hq % Hkv == 0):
+    The reference also serves function transforms and forward-mode derivatives, gradients of the rotation tables, and
+    rows that TMA cannot address."""
+    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.shape[0] > 0 and Hq % Hkv == 0
+            and qkv.shape[1] == (Hq + 2 * Hkv) * 64):
         return False
     for w in (wq, wk):
         if (w is None) != (wq is None) or (w is not None and not (w.dtype == torch.bfloat16 and w.is_contiguous()
                                                                  and w.numel() == 64 and w.is_cuda)):
             return False
     for t in (cos, sin):
-        if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.shape == (qkv.shape[0], 32)):
+        if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.shape == (qkv.shape[0], 32)
+                and not t.requires_grad):
             return False
     return (cu_seqlens.is_cuda and cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous()
             and cu_seqlens.numel() > 1 and not torch._C._are_functorch_transforms_active()
-            and torch.autograd.forward_ad._current_level < 0)
+            and torch.autograd.forward_ad._current_level < 0
+            and (qkv.data_ptr() % 16 == 0 or not qkv.is_contiguous()))        # else copied, and aligned then
 
 
 def _qk_weight_grads(wq, wk, D: int, T: int, device):
@@ -312,6 +316,8 @@ class _QKNormRopeAttn(torch.autograd.Function):
         dout = dout.reshape(T, Hq, D)
         if not dout.is_contiguous():
             dout = dout.contiguous()
+        if D == 64 and dout.data_ptr() % 16:
+            dout = dout.clone()
         q = qk[:, :Hq * D].view(T, Hq, D)
         k = qk[:, Hq * D:].view(T, Hkv, D)
         v = qkv[:, (Hq + Hkv) * D:].view(T, Hkv, D)
