@@ -9,7 +9,7 @@
 // descriptors over the TMA-written tiles.  dQ is produced by attn_bwd_dq.cu.
 //
 // The step is software-pipelined over two buffers of everything that crosses between the tensor
-// core and the row threads: S / dP in TMEM and P / dS in shared memory.  The MMA thread issues
+// core and the row threads: S / dP in TMEM (P / dS in shared memory have one, see below).  The MMA thread issues
 // S, dP of step t+1 before it waits for P, dS of step t, so the tensor core multiplies while the
 // row threads exponentiate, and the dV / dK MMAs of step t overlap the row work of step t+1.
 // Eight row warps (two threads per query row, 32 key columns each) put two warps on every
@@ -33,22 +33,21 @@ constexpr int Q_CHUNK_BYTES = BQ * 128;
 constexpr int PS_BYTES = BQ * BKV * 2;        // 16 KB : [128 q rows][64 kv = 128 B]
 
 constexpr int D = 64;
-// P and dS are sums of two bf16 tiles (see attn_fwd.cu), and dO^T P and Q^T dS come from one product
+// P and dS are sums of three bf16 tiles (see attn_fwd.cu), and dO^T P and Q^T dS come from one product
 // [dO | Q]^T [P | dS] of 128 x 128: its diagonal blocks are dV^T and dK^T.  A product of M = 64 would run the
 // tensor core at half rate anyway, so the off-diagonal blocks are free and one MMA of N = 128 (65 cycles)
-// replaces two of N = 64 (50 cycles each).  dO and Q of a stage, and P and dS of a buffer, lie next to each
-// other as the two 64-wide chunks of one operand.
+// replaces two of N = 64 (50 cycles each).  dO and Q of a stage, and the same part of P and dS, lie next to each
+// other as the two 64-wide chunks of one operand.  The parts of one step take 96 KB, so there is one buffer of
+// them: the row threads exponentiate step t + 1 while the products of step t run, and write when these are done.
 constexpr int SMEM_K = 0;
 constexpr int SMEM_V = SMEM_K + KV_CHUNK_BYTES;
 constexpr int SMEM_RING = SMEM_V + KV_CHUNK_BYTES;                    // 2 stages of dO and Q
-constexpr int SMEM_PS = SMEM_RING + 4 * Q_CHUNK_BYTES;                // 2 buffers of P, dS and their remainders
-constexpr int SMEM_BAR = SMEM_PS + 8 * PS_BYTES;
+constexpr int SMEM_PS = SMEM_RING + 4 * Q_CHUNK_BYTES;                // P and dS, three parts
+constexpr int SMEM_BAR = SMEM_PS + 6 * PS_BYTES;
 constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
-constexpr int REST = 2 * PS_BYTES;                                    // from a high part to its remainder
+constexpr int PART = 2 * PS_BYTES;                                    // from a part to the next
 __device__ constexpr int at_do(int s) { return SMEM_RING + 2 * s * Q_CHUNK_BYTES; }
 __device__ constexpr int at_q(int s) { return at_do(s) + Q_CHUNK_BYTES; }
-__device__ constexpr int at_p(int b) { return SMEM_PS + 4 * b * PS_BYTES; }
-__device__ constexpr int at_ds(int b) { return at_p(b) + PS_BYTES; }
 
 struct Params {
   const float* lse;     // [Hq, T]
@@ -68,7 +67,7 @@ struct __align__(8) Barriers {
   uint64_t kv_full;
   uint64_t q_full[2], q_empty[2];
   uint64_t sdp_full[2], sdp_empty[2];   // S and dP ready in TMEM / read out by the row threads
-  uint64_t pds_full[2], pds_free[2];    // P and dS written to shared memory / consumed by the MMAs
+  uint64_t pds_full, pds_free;          // P and dS written to shared memory / consumed by the MMAs
   uint64_t all_done;
   uint32_t tmem_base;
   int abort_flag;
@@ -116,9 +115,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       mbar_init(&bars->q_empty[s], 1);
       mbar_init(&bars->sdp_full[s], 1);
       mbar_init(&bars->sdp_empty[s], ROW_THREADS);
-      mbar_init(&bars->pds_full[s], ROW_THREADS);
-      mbar_init(&bars->pds_free[s], 1);
     }
+    mbar_init(&bars->pds_full, ROW_THREADS);
+    mbar_init(&bars->pds_free, 1);
     mbar_init(&bars->all_done, 1);
     bars->abort_flag = 0;
     mbar_fence_init();
@@ -207,23 +206,25 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         if (t + 1 < n_steps) {
           if (!issue_sdp(t + 1)) { ok = false; break; }
         }
-        if (!mbar_wait(&bars->pds_full[s], (t >> 1) & 1, abort_flag, p.status, XB_K_ATTN_BWD, 840 + s)) {
+        if (!mbar_wait(&bars->pds_full, t & 1, abort_flag, p.status, XB_K_ATTN_BWD, 840)) {
           ok = false;
           break;
         }
         tc_fence_after();
         const uint32_t sdo = xb_smem_u32(smem + at_do(s));
-        const uint32_t spp = xb_smem_u32(smem + at_p(s));
+        const uint32_t spp = xb_smem_u32(smem + SMEM_PS);
         // dV^T += dO^T P ; dK^T += Q^T dS   (reduction over the 128 query rows, 16 per MMA)
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k) {
           tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
                         xb_smem_desc(mn_ps, spp + k * 2048), idesc_t, (t > 0 || k > 0) ? 1u : 0u);
           tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
-                        xb_smem_desc(mn_ps, spp + REST + k * 2048), idesc_t, 1u);
+                        xb_smem_desc(mn_ps, spp + PART + k * 2048), idesc_t, 1u);
+          tc_mma_f16_ss(tmem_base + COL_DV, xb_smem_desc(mn_q, sdo + k * 2048),
+                        xb_smem_desc(mn_ps, spp + 2 * PART + k * 2048), idesc_t, 1u);
         }
         tc_commit(&bars->q_empty[s]);
-        tc_commit(&bars->pds_free[s]);
+        tc_commit(&bars->pds_free);
       }
       if (ok) tc_commit(&bars->all_done);
     }
@@ -302,43 +303,29 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           if (!row_valid) xb_zero_row128(smem + (half ? at_do(s) : at_q(s)) + r * 128);
         }
       }
-      // the dV / dK MMAs of step t-2 read this P / dS buffer: wait until they are done
-      if (!__all_sync(0xffffffffu, mbar_wait(&bars->pds_free[s], ph ^ 1, abort_flag, p.status, XB_K_ATTN_BWD, 910 + s))) {
+      // the dV / dK MMAs of step t-1 read the P / dS buffer: wait until they are done
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->pds_free, (t & 1) ^ 1, abort_flag, p.status, XB_K_ATTN_BWD, 910))) {
         ok = false;
         break;
       }
       // P and dS rows (bf16) -> shared memory, [128 rows][128 B] with the 128B swizzle
-      uint8_t* sp = smem + at_p(s) + r * 128;
-      uint8_t* sd = smem + at_ds(s) + r * 128;
+      uint8_t* sp = smem + SMEM_PS + r * 128;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint4 v, w;
-        v.x = pack_bf16x2(pv[c * 8 + 0], pv[c * 8 + 1]);
-        v.y = pack_bf16x2(pv[c * 8 + 2], pv[c * 8 + 3]);
-        v.z = pack_bf16x2(pv[c * 8 + 4], pv[c * 8 + 5]);
-        v.w = pack_bf16x2(pv[c * 8 + 6], pv[c * 8 + 7]);
-        w.x = pack_bf16x2(ds[c * 8 + 0], ds[c * 8 + 1]);
-        w.y = pack_bf16x2(ds[c * 8 + 2], ds[c * 8 + 3]);
-        w.z = pack_bf16x2(ds[c * 8 + 4], ds[c * 8 + 5]);
-        w.w = pack_bf16x2(ds[c * 8 + 6], ds[c * 8 + 7]);
         const int slot = (half * 4 + c) ^ (r & 7);
-        *reinterpret_cast<uint4*>(sp + slot * 16) = v;
-        *reinterpret_cast<uint4*>(sd + slot * 16) = w;
-        uint4 v2, w2;
-        v2.x = pack_bf16x2_rest(pv[c * 8 + 0], pv[c * 8 + 1], v.x);
-        v2.y = pack_bf16x2_rest(pv[c * 8 + 2], pv[c * 8 + 3], v.y);
-        v2.z = pack_bf16x2_rest(pv[c * 8 + 4], pv[c * 8 + 5], v.z);
-        v2.w = pack_bf16x2_rest(pv[c * 8 + 6], pv[c * 8 + 7], v.w);
-        w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
-        w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
-        w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
-        w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
-        *reinterpret_cast<uint4*>(sp + REST + slot * 16) = v2;
-        *reinterpret_cast<uint4*>(sd + REST + slot * 16) = w2;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {                // P, dS
+          uint4 hi, mid, lo;
+          split3_bf16x8((m ? ds : pv) + c * 8, hi, mid, lo);
+          uint8_t* dst = sp + m * PS_BYTES + slot * 16;
+          *reinterpret_cast<uint4*>(dst) = hi;
+          *reinterpret_cast<uint4*>(dst + PART) = mid;
+          *reinterpret_cast<uint4*>(dst + 2 * PART) = lo;
+        }
       }
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(&bars->pds_full[s]);
+      mbar_arrive(&bars->pds_full);
     }
     if (ok && n_steps > 0) ok = mbar_wait(&bars->all_done, 0, abort_flag, p.status, XB_K_ATTN_BWD, 920);
     ok = __all_sync(0xffffffffu, ok);

@@ -4,8 +4,8 @@
 // One CTA owns a 128-row query tile of one query head and walks the 64-row key/value tiles it can
 // see.  Per step three tcgen05 GEMM groups:
 //     S  = Q K^T   (128 x 64, K = d)      dP = dO V^T   (128 x 64, K = d)
-//     dQ += dS K   (128 x 64, K = 64 kv rows)           dS = P o (dP - delta) * scale
-// dQ stays in TMEM for the CTA's lifetime and is written once, with plain stores: every (row,
+//     dQ += dS K   (128 x 64, K = 64 kv rows)           dS = P o (dP - delta)
+// dQ stays in TMEM for the CTA's lifetime and is written once, times the scale, with plain stores: every (row,
 // head) of dQ belongs to exactly one CTA.  S / dP are double-buffered in TMEM and dS in shared
 // memory, so the MMAs of step j+1 run while the row threads turn step j into dS.
 // Together with the dK / dV kernel this needs no atomics; the price is a second evaluation of S and dP.
@@ -30,12 +30,12 @@ constexpr int Q_CHUNK_BYTES = BQ * 128;
 constexpr int DS_BYTES = BQ * BKV * 2;         // 16 KB : [128 q rows][64 kv = 128 B]
 
 constexpr int D = 64;
-// dS is the sum of two bf16 tiles (see attn_fwd.cu)
+// dS is the sum of three bf16 tiles (see attn_fwd.cu)
 constexpr int SMEM_Q = 0;
 constexpr int SMEM_DO = SMEM_Q + Q_CHUNK_BYTES;
 constexpr int SMEM_KV = SMEM_DO + Q_CHUNK_BYTES;                  // NS x (K tile, V tile)
-constexpr int SMEM_DS = SMEM_KV + NS * 2 * KV_CHUNK_BYTES;        // 2 buffers of high part and remainder
-constexpr int DS_BUF = 2 * DS_BYTES;
+constexpr int SMEM_DS = SMEM_KV + NS * 2 * KV_CHUNK_BYTES;        // 2 buffers of the three parts
+constexpr int DS_BUF = 3 * DS_BYTES;
 constexpr int SMEM_BAR = SMEM_DS + 2 * DS_BUF;
 constexpr int SMEM_BYTES = SMEM_BAR + 256 + 1024;
 
@@ -212,6 +212,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                         xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, (j > 0 || k > 0) ? 1u : 0u);
           tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + DS_BYTES + k * 32),
                         xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, 1u);
+          tc_mma_f16_ss(tmem_base + COL_DQ, xb_smem_desc(kmaj, sds + 2 * DS_BYTES + k * 32),
+                        xb_smem_desc(mn_kv, sk + k * 2048), idesc_q, 1u);
         }
         tc_commit(&bars->kv_empty[s]);   // K_j (and V_j, read earlier) no longer needed
         tc_commit(&bars->ds_free[b]);
@@ -289,18 +291,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int c16 = half * 4 + c;
-        uint4 w;
-        w.x = pack_bf16x2(ds[c * 8 + 0], ds[c * 8 + 1]);
-        w.y = pack_bf16x2(ds[c * 8 + 2], ds[c * 8 + 3]);
-        w.z = pack_bf16x2(ds[c * 8 + 4], ds[c * 8 + 5]);
-        w.w = pack_bf16x2(ds[c * 8 + 6], ds[c * 8 + 7]);
-        *reinterpret_cast<uint4*>(sd + ((c16 ^ (r & 7)) * 16)) = w;
-        uint4 w2;
-        w2.x = pack_bf16x2_rest(ds[c * 8 + 0], ds[c * 8 + 1], w.x);
-        w2.y = pack_bf16x2_rest(ds[c * 8 + 2], ds[c * 8 + 3], w.y);
-        w2.z = pack_bf16x2_rest(ds[c * 8 + 4], ds[c * 8 + 5], w.z);
-        w2.w = pack_bf16x2_rest(ds[c * 8 + 6], ds[c * 8 + 7], w.w);
-        *reinterpret_cast<uint4*>(sd + DS_BYTES + ((c16 ^ (r & 7)) * 16)) = w2;
+        uint4 hi, mid, lo;
+        split3_bf16x8(ds + c * 8, hi, mid, lo);
+        uint8_t* dst = sd + ((c16 ^ (r & 7)) * 16);
+        *reinterpret_cast<uint4*>(dst) = hi;
+        *reinterpret_cast<uint4*>(dst + DS_BYTES) = mid;
+        *reinterpret_cast<uint4*>(dst + 2 * DS_BYTES) = lo;
       }
       fence_proxy_async_smem();
       tc_fence_before();

@@ -369,15 +369,26 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float2 unpack_bf16x2(uint32_t u);
-// what rounding (lo, hi) to the packed pair `rounded` left over, as a bf16 pair
-__device__ __forceinline__ uint32_t pack_bf16x2_rest(float lo, float hi, uint32_t rounded) {
-  const float2 f = unpack_bf16x2(rounded);
-  return pack_bf16x2(lo - f.x, hi - f.y);
-}
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(v);
+}
+// Eight fp32 values as the sums of three bf16 values each: a significand of 24 bits in parts of eight (what
+// underflows bf16's range is lost, as it is in fp32).
+__device__ __forceinline__ void split3_bf16x8(const float* f, uint4& hi, uint4& mid, uint4& lo) {
+  uint32_t h[4], m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    h[i] = pack_bf16x2(f[2 * i], f[2 * i + 1]);
+    const float2 a = unpack_bf16x2(h[i]);
+    const float r0 = f[2 * i] - a.x, r1 = f[2 * i + 1] - a.y;
+    m[i] = pack_bf16x2(r0, r1);
+    const float2 b = unpack_bf16x2(m[i]);
+    l[i] = pack_bf16x2(r0 - b.x, r1 - b.y);
+  }
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  mid = make_uint4(m[0], m[1], m[2], m[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
