@@ -522,6 +522,17 @@ def test_hd64_attention_outside_the_kernels_range():
     assert torch.equal(got, ref)
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_hd64_attention_with_a_scale_that_is_not_positive(scale):
+    from xorl_b200.ops import attention as A
+    torch.manual_seed(7)
+    cu, D = _make_cu([90, 70]), 64
+    x = torch.randn(160, 8 * D, device=DEV, dtype=torch.bfloat16)
+    cos, sin = torch.ones(160, D // 2, device=DEV), torch.zeros(160, D // 2, device=DEV)
+    got = A.qk_norm_rope_attention(x, None, None, cos, sin, cu, 4, 2, D, scale=scale)
+    assert torch.equal(got, A.qk_norm_rope_attention_reference(x, None, None, cos, sin, cu, 4, 2, D, 1e-6, True, scale))
+
+
 def test_status_words_clean():
     from xorl_b200.ops import _lib
     assert _lib.read_status()[0] == 0

@@ -1,4 +1,5 @@
-"""Variable-length flash attention (``csrc/attn_fwd.cu`` / ``csrc/attn_bwd.cu``) and the fused
+"""Variable-length flash attention (``csrc/attn_fwd_hd128.cu`` / ``csrc/attn_bwd_hd128.cu``; 64-wide heads
+of the fused block: ``csrc/attn_fwd.cu``, ``csrc/attn_bwd_dkv.cu``, ``csrc/attn_bwd_dq.cu``) and the fused
 qk-RMSNorm + RoPE + attention block used by the decoder layers.
 
 Layout is the packed one of the reference's varlen path
@@ -182,14 +183,14 @@ def _kernel_ok(t: torch.Tensor, D: int) -> bool:
     return t.is_cuda and t.dtype == torch.bfloat16 and D == 128
 
 
-def _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv) -> bool:
+def _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv, scale) -> bool:
     """What the head-dim-64 kernels take; everything else of that width runs in the reference (fp32
     matmuls per document; a training step of 2 such layers with 16 heads on 2045 tokens took 11.9 ms there and
-    takes 4.2 ms here, 0.13 ms of it per layer in the three attention kernels).
+    takes 2.9 ms here, 0.18 ms of it per layer in the attention kernels).
     The reference also serves function transforms and forward-mode derivatives, gradients of the rotation tables, and
     rows that TMA cannot address."""
     if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.shape[0] > 0 and Hq % Hkv == 0
-            and qkv.shape[1] == (Hq + 2 * Hkv) * 64):
+            and qkv.shape[1] == (Hq + 2 * Hkv) * 64 and scale > 0):      # the kernels scale a row's largest score
         return False
     for w in (wq, wk):
         if (w is None) != (wq is None) or (w is not None and not (w.dtype == torch.bfloat16 and w.is_contiguous()
@@ -418,8 +419,8 @@ def qk_norm_rope_attention(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps=1e
     cos/sin: fp32 [T, D/2] gathered at each token's position.  Returns [T, Hq*D].
     """
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
-    if _kernel_ok(qkv, D) or (D == 64 and _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv)):
+    if _kernel_ok(qkv, D) or (D == 64 and _fused_hd64_ok(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv, scale)):
         return _lib.apply(_QKNormRopeAttn, qkv.contiguous(), wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps, causal,
-                                     scale)
+                          scale)
     return qk_norm_rope_attention_reference(qkv, wq, wk, cos, sin, cu_seqlens, Hq, Hkv, D, eps,
                                             causal, scale)
