@@ -544,17 +544,6 @@ def _permute_kernels_ok(x: torch.Tensor) -> bool:
             and os.environ.get("XORL_B200_MOE_KERNELS", "1") == "1")
 
 
-def _gather_rows(inp, src_row, rows, scale=None):
-    global _launches
-    out = torch.empty((rows, inp.shape[1]), device=inp.device, dtype=inp.dtype)
-    inp = inp.contiguous()
-    _lib.check(_lib.cuda_lib().xb_moe_gather_rows(out.data_ptr(), out.stride(0), inp.data_ptr(), inp.stride(0),
-                                                  src_row.data_ptr(), _lib.ptr(scale), rows, inp.shape[1],
-                                                  _lib.stream_ptr()), "xb_moe_gather_rows")
-    _launches += 1
-    return out
-
-
 def _gather_sum(inp, idx, w):
     global _launches
     T, k = idx.shape
@@ -631,13 +620,6 @@ def canonical_combine(y_slots: torch.Tensor, weights: torch.Tensor) -> torch.Ten
             nxt.append(parts[-1])
         parts = nxt
     return parts[0].to(y_slots.dtype)
-
-
-def token_of_row(dest: torch.Tensor, rows: int, k: int) -> torch.Tensor:
-    """Inverse of ``dest`` [T*k]: token index stored in every buffer row, -1 for padding rows."""
-    tok = torch.full((rows,), -1, device=dest.device, dtype=torch.int32)
-    tok[dest] = (torch.arange(dest.numel(), device=dest.device) // k).to(torch.int32)
-    return tok
 
 
 def local_moe_forward(x: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor, experts,

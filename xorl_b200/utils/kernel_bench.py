@@ -345,20 +345,22 @@ def bench_qk_norm_rope(a) -> Dict:
 
 
 def bench_permute(a) -> Dict:
-    """MoE row gather (token -> expert-sorted buffer) and weighted combine (k rows -> token)."""
+    """MoE plan (expert ids -> buffer rows), row gather (token -> expert-sorted buffer) and weighted combine (k rows
+    -> token)."""
     from ..ops import moe as moe_ops
     T, k, H, E = a.tokens, 8, a.hidden, a.experts
     x = torch.randn(T, H, device="cuda").bfloat16()
     idx = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(64)]).repeat(T // 64 + 1, 1)[:T]
-    dest, seg, _ = moe_ops.aligned_sort_indices(idx.reshape(-1), E)
     rows = moe_ops.buffer_rows(T * k, E)
-    tok = moe_ops.token_of_row(dest, rows, k)
-    w = torch.rand(T, k, device="cuda")
-    ms_g = _time(lambda: moe_ops._gather_rows(x, tok, rows), a.warmup, a.iters, a.flush)
-    buf = moe_ops._gather_rows(x, tok, rows)
+    ms_p = _time(lambda: moe_ops.sort_plan(idx.reshape(-1), E, rows), a.warmup, a.iters, a.flush)
+    dest, _, slot = moe_ops.sort_plan(idx.reshape(-1), E, rows)
     d2 = dest.view(T, k)
-    ms_c = _time(lambda: moe_ops._gather_sum(buf, d2, w), a.warmup, a.iters, a.flush)
-    return {"kernel": "moe_permute", "tokens": T, "k": k, "hidden": H, "gather_ms": ms_g,
+    w = torch.rand(T, k, device="cuda")
+    with torch.no_grad():
+        ms_g = _time(lambda: moe_ops._Permute.apply(x, d2, slot), a.warmup, a.iters, a.flush)
+        buf = moe_ops._Permute.apply(x, d2, slot)
+        ms_c = _time(lambda: moe_ops._Combine.apply(buf, w, d2, slot), a.warmup, a.iters, a.flush)
+    return {"kernel": "moe_permute", "tokens": T, "k": k, "hidden": H, "plan_ms": ms_p, "gather_ms": ms_g,
             "gather_gbs": (T * k * H * 2 * 2) / ms_g / 1e6, "combine_ms": ms_c,
             "combine_gbs": (T * k * H * 2 + T * H * 2) / ms_c / 1e6}
 
