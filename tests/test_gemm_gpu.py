@@ -95,3 +95,23 @@ def test_gemm_sum_of_two_products(M, N, K, K2, b_mn):
     bound = mag * ((K + K2) * 2.0 ** -24) + (ref.abs() + (x.double() @ op(w)).abs()) * 2.0 ** -8
     assert ((gemm_sum(x, w, x2, w2, b_mn).double() - ref).abs() <= bound + 1e-6).all()
     assert all(v == 0 for v in _lib.read_status()[:4])
+
+
+@pytest.mark.parametrize("rows", [(1024, 8), (8, 1024), (1024, 64, 1024, 8)])
+def test_weight_used_at_several_lengths_sums_its_gradients(rows):
+    """An engine's fp32 buffer with products on the side stream (2^31 multiply-adds and more) and on the main one.
+    fp32 sums over all rows."""
+    from xorl_b200.ops import gemm, grad_sink
+    torch.manual_seed(0)
+    N, K = 2048, 2048
+    w = torch.nn.Parameter((torch.randn(N, K, device="cuda") * 0.02).bfloat16())
+    xs = [torch.randn(r, K, device="cuda").bfloat16() for r in rows]
+    dys = [torch.randn(r, N, device="cuda").bfloat16() for r in rows]
+    ref = sum(d.double().t() @ x.double() for d, x in zip(dys, xs))
+    bound = sum(d.double().abs().t() @ x.double().abs() for d, x in zip(dys, xs)) * (sum(rows) * 2.0 ** -24)
+    for _ in range(10):
+        w._xb_grad_buf, w._xb_grad_fresh = torch.full((N, K), float("nan"), device="cuda"), True
+        for x, dy in zip(xs, dys):
+            assert gemm.weight_grad(dy, x, w) is None
+        grad_sink.join_wgrad_stream()
+        assert ((w._xb_grad_buf.double() - ref).abs() <= bound + 1e-6).all()

@@ -332,15 +332,85 @@ def test_attention_128_against_the_single_backward_kernel(lens, Hq, Hkv, causal,
         refs = [ref.detach()] + [t.grad for t in ins]
     else:
         prev = A.set_backward_mode("fused")
-        dv2 = torch.empty_like(v)
-        dq2, dk2 = A._attn_bwd(q, k, v, out, go, lse, cu, causal, D ** -0.5, dv2, window)
-        A.set_backward_mode(prev)
-        refs = [None, dq2, dk2, dv2]
+        try:
+            dv2 = torch.empty_like(v)
+            dq2, dk2 = A._attn_bwd(q, k, v, out, go, lse, cu, causal, D ** -0.5, dv2, window)
+        finally:
+            A.set_backward_mode(prev)
+        refs = [A.attention_reference(q.float(), k.float(), v.float(), cu, causal=causal), dq2, dk2, dv2]
     for name, g, r in zip(("out", "dq", "dk", "dv"), got, refs):
-        if r is not None:
-            err = (g.float() - r.float()).norm().item() / max(r.float().norm().item(), 1e-3 * go.float().norm().item())
-            assert err < 2 ** -7, (name, err)
+        err = (g.float() - r.float()).norm().item() / max(r.float().norm().item(), 1e-3 * go.float().norm().item())
+        assert err < 2 ** -7, (name, err)
     assert _lib.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("lens,pad,Hq,Hkv", [([128, 300], 0, 4, 2), ([77, 1, 513], 40, 8, 1), ([640], 128, 2, 2)])
+def test_block_attention_against_key_blocks(lens, pad, Hq, Hkv):
+    """What ring attention asks of the 128-wide kernels: keys that start elsewhere in a longer tensor, blocks that take
+    no part, and dq added to in a second call.  Float32 on the CPU is the oracle; P and dS are bf16, 2^-7 of the norm."""
+    from xorl_b200.parallel.sequence_parallel import block_attention, block_attention_bwd
+    torch.manual_seed(5)
+    D, T, B = 128, sum(lens), len(lens)
+    cu = _make_cu(lens)
+    Tk = 2 * T + pad                                          # two key sets behind `pad` rows that nobody sees
+    starts = torch.tensor([0] + lens[:-1]).cumsum(0).to(torch.int32)
+    own, other = (starts + pad).to(DEV), (starts + pad + T).to(DEV)
+    if B > 1:
+        other[0] = -1
+    q, go = (torch.randn(T, Hq, D, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(Tk, Hkv, D, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    scale = D ** -0.5
+    parts = {dev: [block_attention(*(t.to(dev) if dev == DEV else t.cpu().float() for t in (q, k, v)),
+                                   cu.to(dev), ks.to(dev), causal, scale) for ks, causal in ((own, True), (other, False))]
+             for dev in (DEV, "cpu")}
+    close = lambda name, a, b: (a.cpu().float() - b.float()).norm() <= 2 ** -7 * b.float().norm() or pytest.fail(name)
+    for (o, l), (ro, rl) in zip(parts[DEV], parts["cpu"]):
+        close("out", o, ro)
+        seen = rl.isfinite()
+        assert torch.equal(l.cpu().isfinite(), seen) and (l.cpu() - rl)[seen].abs().max() < 1e-2
+    (o1, l1), (o2, l2) = parts["cpu"]
+    lse = torch.logaddexp(l1, l2)
+    mix = lambda o, l: o.float() * torch.exp(l - lse).transpose(0, 1).unsqueeze(-1)
+    out = (mix(o1, l1) + mix(o2, l2)).bfloat16()
+    got = {}
+    for dev in (DEV, "cpu"):
+        cast = (lambda t: t.to(dev)) if dev == DEV else (lambda t: t.cpu().float())
+        delta = torch.full((Hq, T), float("nan"), device=dev)
+        dq = torch.full((T, Hq, D), float("nan"), device=dev)
+        got[dev] = []
+        for i, (ks, causal) in enumerate(((own, True), (other, False))):
+            got[dev] += block_attention_bwd(cast(q), cast(k), cast(v), cast(out), cast(go), lse.to(dev), delta, dq,
+                                            cu.to(dev), ks.to(dev), causal, scale, i == 0)
+        got[dev].append(dq)
+    for name, a, b in zip(("dk", "dv", "dk other", "dv other", "dq"), got[DEV], got["cpu"]):
+        close(name, a, b)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_gradient_rows_outside_every_document_are_zero(D, monkeypatch):
+    """Documents that begin behind the first token and end before the last; every allocation holds NaN before."""
+    from xorl_b200.ops import attention as A
+    torch.manual_seed(6)
+    T, Hq, Hkv = 400, 4, 2
+    cu = torch.tensor([30, 190, 371], device=DEV, dtype=torch.int32)
+    q, k, v = (torch.randn(T, h, D, device=DEV, dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    go = torch.randn(T, Hq, D, device=DEV, dtype=torch.bfloat16)
+    dv = torch.full_like(v, float("nan"))
+    monkeypatch.setattr(torch, "empty", lambda *a, **kw: torch.full(*a, float("nan"), **kw))
+    if D == 64:
+        out, lse, f32 = A._attn_fwd_hd64(q, k, v, cu, True, D ** -0.5, True)
+        dq, dk = A._attn_bwd_hd64(q, k, v, f32, go, lse, cu, True, D ** -0.5, dv)
+    else:
+        out, lse = A._attn_fwd(q, k, v, cu, True, D ** -0.5)
+        dq, dk = A._attn_bwd(q, k, v, out, go, lse, cu, True, D ** -0.5, dv)
+    monkeypatch.undo()
+    ins = [t[30:371].float().requires_grad_() for t in (q, k, v)]
+    ref = A.attention_reference(*ins, cu - 30)
+    ref.backward(go[30:371].float())
+    for a, r in zip((out, dq, dk, dv), [ref.detach()] + [t.grad for t in ins]):
+        assert (a[30:371].float() - r).norm() < 2 ** -7 * r.norm()
+    for t in (dq, dk, dv) if D == 64 else (dq,):
+        assert not t[:30].any() and not t[371:].any()
 
 
 def test_attention_128_takes_more_tiles_than_a_grid_is_high():
