@@ -107,3 +107,36 @@ def test_anyprecision_adamw_with_moments_in_host_memory():
     for n, t in out[0].items():
         assert torch.equal(t, out[1][n]), n
     reset_parallel_state()
+
+
+@pytest.mark.parametrize("recompute", [False, True])
+def test_router_without_numbers_stops_the_step(recompute):
+    """Expert ids are looked at once per pass: the step and the forward pass raise, and both work again afterwards."""
+    from xorl_b200.models import ModelConfig
+    from xorl_b200.models.decoder import DecoderLM
+    from xorl_b200.parallel.state import init_parallel_state, reset_parallel_state
+    from xorl_b200.parallel.zero import Zero3Engine
+    reset_parallel_state()
+    ps = init_parallel_state(device_type="cuda")
+    cfg = ModelConfig.from_dict(dict(model_type="qwen3_moe", vocab_size=256, hidden_size=128, num_hidden_layers=3,
+                                     num_attention_heads=2, num_key_value_heads=1, head_dim=128, intermediate_size=128,
+                                     num_experts=8, num_experts_per_tok=2, moe_intermediate_size=128,
+                                     router_aux_loss_coef=1e-3))
+    model = DecoderLM(cfg, device="meta")
+    model.aux_loss_enabled = True
+    eng = Zero3Engine(model, ps, compute_dtype=torch.bfloat16, device=torch.device("cuda", 0), recompute=recompute)
+    ids = torch.randint(0, 256, (1, 200), device="cuda")
+    labels = torch.randint(0, 256, (1, 200), device="cuda")
+    clean = eng.forward_backward(ids, labels, grad_scale=1 / 200), eng.forward_only(ids)
+    eng.finish_grad_sync()
+    gate = next(p for n, p in model.named_parameters() if "layers.1." in n and "gate." in n)
+    kept = gate.data[3, 5].clone()
+    gate.data[3, 5] = float("nan")
+    with pytest.raises(RuntimeError, match="expert ids"):
+        eng.forward_backward(ids, labels, grad_scale=1 / 200)
+    with pytest.raises(RuntimeError, match="expert ids"):
+        eng.forward_only(ids)
+    gate.data[3, 5] = kept
+    again = eng.forward_backward(ids, labels, grad_scale=1 / 200), eng.forward_only(ids)
+    assert torch.equal(again[0], clean[0]) and torch.equal(again[1], clean[1])
+    reset_parallel_state()

@@ -203,7 +203,8 @@ class MoEBlock(nn.Module):
             out = ep_ops.ep_moe_forward(xe, weights, indices, self.experts, self.cfg.num_experts, ctx)
         else:
             out = moe_ops.local_moe_forward(xe, weights, indices, self.experts, self.cfg.num_experts,
-                                            canonical=bool(ctx.aux.get("canonical_moe", False)))
+                                            canonical=bool(ctx.aux.get("canonical_moe", False)),
+                                            checks=ctx.aux.get("placed_checks"))
         out = self.post_experts(out)
         if self.shared_expert is not None:
             sh = self.shared_expert(x)

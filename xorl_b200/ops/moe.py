@@ -310,32 +310,39 @@ def sort_plan(expert_ids: torch.Tensor, num_experts: int, rows: int, placed: Opt
     return dest, seg, slot_of_row
 
 
-class _PlacedCheck:
+class PlacedChecks:
     """Raises when a plan could not place every slot (an id that is no expert: a bad replay record, or the
-    router's choice among logits that are not numbers).  The count travels to the host behind the plan and is read
-    once the expert MLP has been launched: the host waits for the plan only, with the GPU busy.  A stream under
-    capture cannot be waited for; the rows of such tokens are NaN there as anywhere."""
+    router's choice among logits that are not numbers).  ``send`` copies the counts of the plans so far to the host
+    behind the work in the stream, ``raise_if_short`` waits for that copy: with a layer's or a pass's work launched
+    in between the GPU stays busy.  A stream under capture cannot be waited for; the rows of such tokens are NaN
+    there as anywhere."""
 
-    def __init__(self, device):
-        self.count = torch.empty(1, device=device, dtype=torch.int32)
-        self.event = None
+    def __init__(self):
+        self.counts, self.expected, self.event = [], [], None
+
+    def count(self, device, slots: int, num_experts: int) -> torch.Tensor:
+        """Where the next plan writes how many of its ``slots`` it has placed."""
+        self.counts.append(torch.empty(1, device=device, dtype=torch.int32))
+        self.expected.append((slots, num_experts))
+        return self.counts[-1]
 
     def send(self) -> None:
-        if torch.cuda.is_current_stream_capturing():
+        if not self.counts or torch.cuda.is_current_stream_capturing():
             return
-        self.host = torch.empty(1, dtype=torch.int32, pin_memory=True)
-        self.host.copy_(self.count, non_blocking=True)
+        counts = torch.cat(self.counts) if len(self.counts) > 1 else self.counts[0]
+        self.host = torch.empty(len(self.counts), dtype=torch.int32, pin_memory=True)
+        self.host.copy_(counts, non_blocking=True)
         self.event = torch.cuda.Event()
         self.event.record(_lib.current_stream())
 
-    def raise_if_short(self, slots: int, num_experts: int) -> None:
+    def raise_if_short(self) -> None:
         if self.event is None:
             return
         self.event.synchronize()
-        missing = slots - self.host.item()
-        if missing:
-            raise RuntimeError(f"{missing} of {slots} expert ids lie outside [0, {num_experts}): "
-                               "router logits that are not numbers, or bad recorded choices")
+        for n, (slots, num_experts) in zip(self.host.tolist(), self.expected):
+            if n != slots:
+                raise RuntimeError(f"{slots - n} of {slots} expert ids lie outside [0, {num_experts}): "
+                                   "router logits that are not numbers, or bad recorded choices")
 
 
 def buffer_rows(num_slots: int, num_experts: int, align: int = SEG_ALIGN) -> int:
@@ -623,23 +630,28 @@ def canonical_combine(y_slots: torch.Tensor, weights: torch.Tensor) -> torch.Ten
 
 
 def local_moe_forward(x: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor, experts,
-                      num_experts: int, canonical: bool = False) -> torch.Tensor:
+                      num_experts: int, canonical: bool = False, checks=None) -> torch.Tensor:
     """All experts local: gather tokens into expert-sorted aligned segments, run the grouped MLP,
-    combine the k expert outputs of every token with its routing weights (fp32 accumulation)."""
+    combine the k expert outputs of every token with its routing weights (fp32 accumulation).  An id that is no
+    expert raises here, or where the caller looks at the ``PlacedChecks`` that it hands in; False: ids that have
+    been looked at before."""
     T, H = x.shape
     k = indices.shape[1]
     rows = buffer_rows(T * k, num_experts)
     flat = indices.reshape(-1)
     if (_permute_kernels_ok(x) and not canonical and flat.dtype == torch.int64 and num_experts <= PLAN_MAX_EXPERTS
             and rows < 2 ** 31):
-        check = _PlacedCheck(x.device)
-        dest, seg, slot_of_row = sort_plan(flat.contiguous(), num_experts, rows, check.count)
-        check.send()
+        mine = PlacedChecks() if checks is None else checks
+        count = mine.count(x.device, T * k, num_experts) if mine is not False else None
+        dest, seg, slot_of_row = sort_plan(flat.contiguous(), num_experts, rows, count)
+        if checks is None:
+            mine.send()
         dest2 = dest.view(T, k)
         buf = _Permute.apply(x, dest2, slot_of_row)
         y = expert_mlp_aligned(buf, seg, experts.gate_up_proj, experts.down_proj, **experts_mlp_kwargs(experts))
         out = _Combine.apply(y, weights, dest2, slot_of_row)
-        check.raise_if_short(T * k, num_experts)
+        if checks is None:
+            mine.raise_if_short()
         return out
     dest, seg, _ = aligned_sort_indices(flat, num_experts)
     token_of_slot = torch.arange(T, device=x.device).repeat_interleave(k)

@@ -31,6 +31,7 @@ from torch import nn
 
 from ..ops import _lib
 from ..ops import optim as optim_ops
+from ..ops.moe import PlacedChecks
 from .state import ParallelState, get_parallel_state
 
 ALIGN = 64  # elements; keeps every parameter and every shard 128-byte aligned in bf16
@@ -760,6 +761,8 @@ class Zero3Engine:
         what ``chunk_backward`` needs (unit inputs when recomputing, autograd graphs otherwise)."""
         nl = len(layers)
         saved: List = []
+        # expert ids are looked at by chunk_backward: a host wait per pass instead of one per layer
+        checks = ctx.aux["placed_checks"] = PlacedChecks()
         if nl:
             self.gather(layers[0])
         for i, unit in enumerate(layers):
@@ -782,6 +785,9 @@ class Zero3Engine:
                 self._take_expert_load(ctx, getattr(layer, "layer_idx", i))
             if self.reshard and self.recompute and not (keep_last_gathered and i == nl - 1):
                 self.release(unit)
+        checks.send()
+        ctx.aux["placed_checks"] = None
+        ctx.aux.setdefault("placed_pending", []).append(checks)
         return acts, saved
 
     def chunk_backward(self, layers: List[ZeroUnit], saved: List, dacts, ctx, defer_reduce: bool = False):
@@ -789,6 +795,9 @@ class Zero3Engine:
         ``pending`` lists the units whose gradient reduction was deferred (``defer_reduce``)."""
         nl = len(layers)
         pending: List = []
+        for checks in ctx.aux.pop("placed_pending", ()):
+            checks.raise_if_short()
+        ctx.aux["placed_checks"] = False          # the choices are those of the first pass
         for i in range(nl - 1, -1, -1):
             unit = layers[i]
             self.gather(unit)
@@ -953,6 +962,7 @@ class Zero3Engine:
         self.gather(root)
         self.wait_gather(root)
         ctx = model.make_context(input_ids, position_ids, cu_seqlens, training=False)
+        checks = ctx.aux["placed_checks"] = PlacedChecks()
         acts = model.forward_embed(input_ids, ctx)
         for i, unit in enumerate(layers):
             self.gather(unit)
@@ -962,9 +972,11 @@ class Zero3Engine:
             acts = unit.modules[0](*acts, ctx)
             if self.reshard:
                 self.release(unit)
+        checks.send()
         hidden = model.forward_head(*acts, ctx)
         if self.reshard:
             self.release(root)
+        checks.raise_if_short()
         return hidden
 
     # ---------------------------------------------------------------------------------------
