@@ -134,6 +134,8 @@ class TrainingArguments:
     moe_global_load_balancing: bool = False
     ce_mode: Optional[str] = None
     ce_num_chunks: int = 8
+    # gradients of logits that the lm-head loss may hold, in MiB.  Unset: 1280 where a chunk has 1024 tokens or more,
+    # one chunk (2 x tokens x vocabulary bytes) below; 0: always one chunk
     ce_kept_logits_mb: Optional[int] = None
     micro_batch_size: int = 1
     gradient_accumulation_steps: int = 1

@@ -491,7 +491,8 @@ int xb_attn_dq_hd64(const void* q, const void* k, const void* v, const void* dou
                     cudaStream_t stream);
 
 // Inputs as in xb_attn_fwd plus out / dout [T, Hq, 128] and lse [Hq, T].
-// Scratch: delta fp32 [Hq * T]; dq_accum fp32 [T * Hq * 128] (this call zeroes it).
+// Scratch: delta fp32 [Hq * T]; dq_accum fp32 [T * Hq * 128], which need not be zeroed (flags bit 0: this call adds
+// to it).
 // Outputs: dq_accum (fp32 dQ), dk fp32 [T, Hkv, 128], dv bf16 [T, Hkv, 128] (token stride lddv).
 XB_API int xb_attn_bwd_ex(const void* q, const void* k, const void* v, const void* out,
                           const void* dout, const float* lse, float* delta, float* dq_accum,

@@ -2,8 +2,8 @@
 // the kernels of moe_permute.cu.  All of it is small (a few MB at most), so what counts is the number of
 // launches and that nothing waits for the host: as sorts, scans, scatters and elementwise operations it was
 // about 70 launches per layer and pass with one host wait for the counts.  65,536 slots over 16 experts are
-// planned in 2.3 + 6.4 us (radix sort, bincount and index arithmetic: 110 us); a training step of two layers with
-// 16 experts and 4096 tokens went from 14.0 to 11.6 ms, one of the small preset from 7.3 to 5.5 ms.
+// planned in 2.3 + 6.4 us (radix sort, bincount and index arithmetic: 110 us).  An id that is no expert gets no row;
+// the host learns of it from the number of placed slots, once per pass (ops/moe.py:PlacedChecks).
 //
 //   xb_moe_plan          expert ids -> row of every slot in the expert-sorted, 128-row-aligned buffer,
 //                        segment table, inverse map and number of placed slots; stable, no host
